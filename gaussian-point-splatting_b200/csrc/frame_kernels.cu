@@ -33,6 +33,11 @@ constexpr uint32_t kScanTile = kScanThreads * kScanItems * kScanRoundsMax;  // l
 constexpr uint32_t kScanTileSmall = kScanThreads * kScanItems;             // 4096
 constexpr uint32_t kScanBigScene = 32u << 20;
 
+// First statement of every kernel that launch_k starts: such a kernel may be scheduled while the
+// previous kernel of its stream drains, so it reads and writes nothing before that kernel's
+// memory is complete.
+__device__ __forceinline__ void previous_kernel_done() { cudaGridDependencySynchronize(); }
+
 // ---------------------------------------------------------------------------------
 // Hi-Z query (depth_mip_chain.cuh:172-215, the non-tree variant the reference compiles)
 // ---------------------------------------------------------------------------------
@@ -118,6 +123,7 @@ __device__ __forceinline__ bool aabb_project_bounds(vec3 bmin, vec3 bmax, const 
 }
 
 __global__ void __launch_bounds__(256) block_cull_kernel(BlockView b, FrameConst fc, HizView hiz) {
+    previous_kernel_done();
     const uint32_t idx = blockIdx.x * blockDim.x + threadIdx.x;
     if (idx == 0 && b.chunk_count) *b.chunk_count = 0u;
     const uint32_t word = (idx & ~31u) >> 5;
@@ -146,6 +152,7 @@ __global__ void __launch_bounds__(256) block_cull_kernel(BlockView b, FrameConst
 __global__ void __launch_bounds__(256) visible_chunks_kernel(BlockView b, uint32_t n, uint32_t* __restrict__ list,
                                                              uint32_t* mask_cur, uint32_t* mask_b,
                                                              const uint32_t* __restrict__ mask_iter) {
+    previous_kernel_done();
     if (mask_iter && (*mask_iter & 1u)) mask_cur = mask_b;  // with mask_iter, mask_cur arrives as mask A
     const uint32_t chunks = (n + 31u) >> 5;
     const uint32_t lane = threadIdx.x & 31u;
@@ -305,6 +312,7 @@ __device__ __forceinline__ bool preprocess_one(const PreprocessArgs& a, const Sc
 // per 256 Gaussians.
 template <class Scene, bool kImmediate>
 __global__ void __launch_bounds__(256) preprocess_kernel(PreprocessArgs a, Scene scene) {
+    previous_kernel_done();
     uint32_t* mask_cur = a.mask_cur;
     const uint32_t* mask_prev = a.mask_prev;
     if (a.mask_iter) {
@@ -457,6 +465,7 @@ __device__ __forceinline__ void block_scan_pair(uint32_t s, uint32_t p, uint32_t
 // Pass 1 of the scan: every tile's survivor and point totals, fully parallel.
 template <int kScanRounds>
 __global__ void __launch_bounds__(kScanThreads) scan_reduce_kernel(ScanArgs a) {
+    previous_kernel_done();
     const uint32_t* mask = a.mask;  // (a select, not a runtime index into the parameter array)
     if (a.mask_iter) mask = (*a.mask_iter & 1u) ? a.mask_pair[1] : a.mask_pair[0];
     const uint32_t tile = blockIdx.x;
@@ -545,6 +554,7 @@ __device__ __forceinline__ void scan_words_inplace(unsigned long long* words_g, 
 // pass counters (points mod 2^32, like the reference's u32 offsets); block 1, when the pass is
 // screen-binned, does the same for the bin histogram.
 __global__ void __launch_bounds__(kTileScanThreads) scan_tiles_kernel(ScanArgs a, uint32_t num_tiles) {
+    previous_kernel_done();
     uint32_t carry_s, carry_p;
     if (blockIdx.x == 1) {
         uint32_t most = 0;
@@ -572,6 +582,7 @@ __global__ void __launch_bounds__(kTileScanThreads) scan_tiles_kernel(ScanArgs a
 // ids and first points.
 template <int kScanRounds>
 __global__ void __launch_bounds__(kScanThreads) scan_write_kernel(ScanArgs a) {
+    previous_kernel_done();
     const uint32_t* mask = a.mask;  // (a select, not a runtime index into the parameter array)
     if (a.mask_iter) mask = (*a.mask_iter & 1u) ? a.mask_pair[1] : a.mask_pair[0];
     const uint32_t tile = blockIdx.x;
@@ -621,6 +632,7 @@ __device__ __forceinline__ void own_tiles(uint32_t* __restrict__ tile_first_rank
 
 template <int kScanRounds>
 __global__ void __launch_bounds__(kScanThreads) scan_write_fused_kernel(ScanArgs a) {
+    previous_kernel_done();
     const uint32_t tile = blockIdx.x;
     // a tile without survivors (its exclusive survivor prefix equals the next tile's) has
     // nothing to write: culled regions of the scene cost two loads, not a pass over their masks
@@ -688,6 +700,7 @@ __global__ void __launch_bounds__(256) tile_owner_kernel(const uint32_t* __restr
                                                          uint32_t* __restrict__ tile_first_rank,
                                                          const PassCounters* __restrict__ counters,
                                                          uint32_t tile_points, uint32_t* __restrict__ mask_iter) {
+    previous_kernel_done();
     const uint32_t points = counters->points;
     const uint32_t survivors = counters->survivors;
     if (mask_iter && points > 0 && blockIdx.x == 0 && threadIdx.x == 0) *mask_iter += 1u;
@@ -1104,6 +1117,7 @@ template <int K>
 #endif
 // (K = 8 keeps two passes of eight samples in flight: more registers, fewer resident blocks)
 __global__ void __launch_bounds__(kSplatTile, kSplatRounds > 1 ? (K >= 8 ? 2 : GPS_SPLAT_MIN_BLOCKS) : 1) splat_kernel(SplatArgs a) {
+    previous_kernel_done();
     __shared__ uint32_t s_start[kSplatWindow];
     __shared__ uint32_t s_spread[kTileSize];
     if (GPS_SPLAT_MORTON_LUT && threadIdx.x < kTileSize) s_spread[threadIdx.x] = morton_spread(threadIdx.x);
@@ -1190,6 +1204,7 @@ __global__ void __launch_bounds__(kSplatTile, kSplatRounds > 1 ? (K >= 8 ? 2 : G
 // Clear and resolve (gaussian_point_splatting.cu:484-548, 580-585)
 // ---------------------------------------------------------------------------------
 __global__ void clear_kernel(ulonglong2* __restrict__ buf, uint64_t pairs, unsigned long long value) {
+    previous_kernel_done();
     const ulonglong2 v = make_ulonglong2(value, value);
     for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < pairs; i += (uint64_t)gridDim.x * blockDim.x)
         buf[i] = v;
@@ -1246,9 +1261,21 @@ __device__ __forceinline__ void resolve_pixel(const ResolveArgs& a, int x, int y
     a.depth[idx] = depth;
 }
 
+// The frame's counters written to pinned host memory by the first block of the final resolve: a
+// copy in the stream after it would hold up the kernels behind it by some microseconds.
+__device__ __forceinline__ void report_counters(const ResolveArgs& a) {
+    constexpr uint32_t kWords = sizeof(PassCounters) / 4u;
+    if (!a.report_to || (blockIdx.x | blockIdx.y) != 0u || threadIdx.y != 0u || threadIdx.x >= 2u * kWords) return;
+    const bool ran = (int)(threadIdx.x / kWords) < a.report_passes;
+    reinterpret_cast<volatile uint32_t*>(a.report_to)[threadIdx.x] =
+        ran ? reinterpret_cast<const uint32_t*>(a.report_from)[threadIdx.x] : 0u;
+}
+
 // Row-major pixels (any supersampling factor).
 template <bool kDepthOnly>
 __global__ void __launch_bounds__(256) resolve_kernel(ResolveArgs a) {
+    previous_kernel_done();
+    report_counters(a);
     const int x = blockIdx.x * blockDim.x + threadIdx.x;
     const int y = blockIdx.y * blockDim.y + threadIdx.y;
     if (x >= a.width || y >= a.height) return;
@@ -1270,6 +1297,8 @@ __device__ __forceinline__ uint32_t morton_compact(uint32_t a) {
 
 template <bool kDepthOnly>
 __global__ void __launch_bounds__(256) resolve_morton_kernel(ResolveArgs a, int ss_log2) {
+    previous_kernel_done();
+    report_counters(a);
     const uint32_t tile_px = (uint32_t)kTileSize >> ss_log2;
     const uint32_t per_tile_log2 = 2u * (uint32_t)(kTileBits - ss_log2);
     const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1298,6 +1327,8 @@ constexpr int kResolveStageBytes = 48 * 1024;
 
 template <bool kDepthOnly>
 __global__ void __launch_bounds__(256) resolve_staged_kernel(ResolveArgs a, int ss_log2, int run_log2) {
+    previous_kernel_done();
+    report_counters(a);
     extern __shared__ uint64_t stage[];
     const uint32_t run = 1u << run_log2;                            // entries per pixel
     // blocks take the buffer from its end: the splat walks screen bins (buffer tiles) in
@@ -1346,6 +1377,7 @@ __device__ __forceinline__ float hiz_op(bool use_min, float a, float b) { return
 
 __global__ void __launch_bounds__(kHizThreads * kHizThreads) hiz_build_kernel(HizView c, const float* __restrict__ src,
                                                                                int min_levels) {
+    previous_kernel_done();
     __shared__ float sm[kHizThreads * kHizThreads];
     __shared__ int s_last;
     const int L = c.levels - 1;
@@ -1643,6 +1675,7 @@ __global__ void taa_kernel(uint8_t* __restrict__ image, float* __restrict__ out_
                            const float* __restrict__ prev_color, const float* __restrict__ cur_depth,
                            const float* __restrict__ prev_depth, mat4 reproj, float blend, int width, int height,
                            int frame_number) {
+    previous_kernel_done();
     // 32 x 8 pixel blocks: a block's 3 x 3 neighbourhood reads stay within 10 rows of L1
     // (TAA 0.042 -> 0.038 ms at 1080p)
     const int x = blockIdx.x * 32 + (int)(threadIdx.x & 31u);
@@ -1702,6 +1735,7 @@ __global__ void taa_kernel(uint8_t* __restrict__ image, float* __restrict__ out_
 
 __global__ void progressive_kernel(uint8_t* __restrict__ image, float* __restrict__ cur, float* __restrict__ accum,
                                    int width, int height, int frames) {
+    previous_kernel_done();
     int idx = blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= width * height) return;
     vec3 color = ld3(cur, idx);
@@ -1727,9 +1761,28 @@ int g_num_sms = 0;
 // launchers
 // ---------------------------------------------------------------------------------
 namespace {
+// Every frame kernel is launched as a programmatic dependent of the one before it in its stream:
+// the launch is set up while that kernel runs, and its blocks start as soon as the last block of
+// that kernel has left the GPU instead of after its completion has been reported back.  No kernel
+// signals earlier (griddepcontrol.launch_dependents): blocks of the next kernel that wait beside
+// a persistent grid's tail land unevenly on the SMs, and frames got slower (16M town: 2.79
+// against 2.38 ms).  A frame is 6 to 18 launches, most of them a few microseconds long on small
+// views.  Measured with the frame's counters handed over by the final resolve, against plain
+// launches and a copy: 20k cube at 160x90 45.5 -> 22.0 us a frame, 60k town at 320x180 130 -> 89,
+// 1M cube at 640x360 177 -> 154, 4M town at 1080p 1121 -> 1076.
 template <typename... KArgs, typename... Args>
 void launch_k(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args... args) {
-    kernel<<<grid, block, smem, stream>>>(args...);
+    cudaLaunchAttribute dependent{};
+    dependent.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    dependent.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cfg.attrs = &dependent;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, kernel, KArgs(args)...);
 }
 }  // namespace
 

@@ -208,6 +208,11 @@ struct ResolveArgs {
     uint64_t entries;
     float near_plane, far_plane;
     uint64_t initial_value;
+    // The final resolve also hands the frame's counters to the host: those of its first
+    // `report_passes` passes, zeros for the others (null report_to: not this launch).
+    const PassCounters* report_from;
+    PassCounters* report_to;  // [2], pinned host memory
+    int report_passes;
 };
 
 // launchers (all asynchronous on `stream`)

@@ -984,9 +984,10 @@ gps_status render_frame_impl(gps_renderer* r, const gps_camera* cam, float* d_im
             render_pass(r, fc, cam->frame, false, st);
             r->second_pass_last = true;
         }
-    } else {
-        cudaMemsetAsync(r->counters.get() + 1, 0, sizeof(PassCounters), st);
     }
+    ra.report_from = r->counters.get();
+    ra.report_to = r->host_counters;
+    ra.report_passes = r->n == 0 ? 0 : r->s.enable_occlusion_culling ? 2 : 1;
     r->timer.mark(kStResolve, st);
     launch_resolve(ra, false, st);
     count_launch(r, kStResolve);
@@ -996,7 +997,6 @@ gps_status render_frame_impl(gps_renderer* r, const gps_camera* cam, float* d_im
         count_launch(r, kStHiz);
     }
     r->timer.mark(-1, st);
-    cudaMemcpyAsync(r->host_counters, r->counters.get(), sizeof(PassCounters) * 2, cudaMemcpyDeviceToHost, st);
     cudaEventRecord(r->done, st);
     r->have_frame = true;
     cudaError_t e = cudaGetLastError();
