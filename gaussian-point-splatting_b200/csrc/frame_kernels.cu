@@ -1210,29 +1210,12 @@ __global__ void clear_kernel(ulonglong2* __restrict__ buf, uint64_t pairs, unsig
         buf[i] = v;
 }
 
-// Where resolve_pixel reads entry i of the splat buffer from.
-struct GlobalEntries {
-    const uint64_t* buffer;
-    __device__ __forceinline__ uint64_t operator()(int i) const {
-        return __ldg(reinterpret_cast<const unsigned long long*>(buffer) + i);
-    }
-};
-struct StagedEntries {  // a contiguous run of the buffer copied to shared memory, one pad
-    const uint64_t* stage;  // word after every pixel's samples (stride = run + 1)
-    int first;
-    int run_log2;
-    __device__ __forceinline__ uint64_t operator()(int i) const {
-        const int w = i - first;
-        return stage[w + (w >> run_log2)];
-    }
-};
-
 // One output pixel: the mean colour of its SS x SS x spp samples and their nearest NDC depth,
 // in the reference's loop order.  The depth arithmetic is kept in exactly this form (and
 // loop shape) because the reference's result depends on how the compiler evaluates it under
 // fast math; the parity tests check it bit for bit.
-template <bool kDepthOnly, class Src>
-__device__ __forceinline__ void resolve_pixel(const ResolveArgs& a, int x, int y, Src src) {
+template <bool kDepthOnly>
+__device__ __forceinline__ float resolve_pixel(const ResolveArgs& a, int x, int y) {
     const uint32_t idx = (uint32_t)(y * a.width + x);
     const int bx = x * a.ss, by = y * a.ss;
     const int up_w = a.width * a.ss, up_h = a.height * a.ss;
@@ -1243,7 +1226,7 @@ __device__ __forceinline__ void resolve_pixel(const ResolveArgs& a, int x, int y
             for (int p = 0; p < a.num_passes; ++p) {
                 int i = splat_index(bx + dx, by + dy, p, a.num_passes, up_w, up_h);
                 if ((uint64_t)(int64_t)i >= a.entries) continue;
-                uint64_t val = src(i);
+                uint64_t val = __ldg(reinterpret_cast<const unsigned long long*>(a.buffer) + i);
                 float view_depth = view_depth_from_key((val >> 36ull) & kDepthMax, a.near_plane, a.far_plane);
                 float z_ndc = view_to_projected_depth(view_depth, a.near_plane, a.far_plane);
                 depth = gmin(depth, z_ndc);
@@ -1258,7 +1241,7 @@ __device__ __forceinline__ void resolve_pixel(const ResolveArgs& a, int x, int y
         a.color[3 * idx + 1] = color.y * inv_passes;
         a.color[3 * idx + 2] = color.z * inv_passes;
     }
-    a.depth[idx] = depth;
+    return depth;
 }
 
 // The frame's counters written to pinned host memory by the first block of the final resolve: a
@@ -1271,6 +1254,44 @@ __device__ __forceinline__ void report_counters(const ResolveArgs& a) {
         ran ? reinterpret_cast<const uint32_t*>(a.report_from)[threadIdx.x] : 0u;
 }
 
+__device__ __forceinline__ float hiz_op(bool use_min, float a, float b) { return use_min ? fminf(a, b) : fmaxf(a, b); }
+__device__ __forceinline__ float hiz_identity(bool use_min) { return use_min ? INFINITY : -INFINITY; }
+
+// The four finest Hi-Z levels (full size, 1/2, 1/4, 1/8), written by the resolve that has the
+// depths in registers: thread m of a group of 64 holds the pixel with in-group Morton code m, so a
+// texel's children are neighbouring lanes.  Level j from the finest reduces with min while
+// j <= min_levels, else with max; texels past the image's edge don't exist and take no part.
+// Called by all threads of the block (whole groups of 64); `exchange` holds a word per warp.
+// Before, one launch read the depth image back and built the whole chain: with the minimum taken
+// over keys below, two resolves and two builds went from 199 to 146 us a frame (4M town, 1080p,
+// 4 spp) and from 441 to 306 (1M town, 4K, 2 spp); a frame of the 60k town at 320x180 89 -> 80.
+__device__ __forceinline__ void hiz_fine_levels(const HizView& c, float depth, int x, int y, int min_levels,
+                                                float* exchange) {
+    const int L = c.levels - 1;  // the caller checked L >= 3
+    const uint32_t m = threadIdx.x & 63u;
+    bool exists = x < c.level_w[L] && y < c.level_h[L];
+    if (exists) c.mip[c.level_off[L] + (uint64_t)y * c.level_w[L] + x] = depth;
+    float v = depth;
+#pragma unroll
+    for (int j = 1; j <= 3; ++j) {
+        const bool use_min = j <= min_levels;
+        const int l = L - j;
+        if (!exists) v = hiz_identity(use_min);
+        v = hiz_op(use_min, v, __shfl_xor_sync(0xffffffffu, v, 1 << (2 * j - 2)));
+        if (j < 3) {
+            v = hiz_op(use_min, v, __shfl_xor_sync(0xffffffffu, v, 2 << (2 * j - 2)));
+        } else {  // the group's other half is the other warp
+            if ((threadIdx.x & 31u) == 0u) exchange[threadIdx.x >> 5] = v;
+            __syncthreads();
+            v = hiz_op(use_min, v, exchange[(threadIdx.x >> 5) ^ 1u]);
+        }
+        x >>= 1;
+        y >>= 1;
+        exists = x < c.level_w[l] && y < c.level_h[l];
+        if (exists && (m & ((1u << (2 * j)) - 1u)) == 0u) c.mip[c.level_off[l] + (uint64_t)y * c.level_w[l] + x] = v;
+    }
+}
+
 // Row-major pixels (any supersampling factor).
 template <bool kDepthOnly>
 __global__ void __launch_bounds__(256) resolve_kernel(ResolveArgs a) {
@@ -1279,7 +1300,7 @@ __global__ void __launch_bounds__(256) resolve_kernel(ResolveArgs a) {
     const int x = blockIdx.x * blockDim.x + threadIdx.x;
     const int y = blockIdx.y * blockDim.y + threadIdx.y;
     if (x >= a.width || y >= a.height) return;
-    resolve_pixel<kDepthOnly>(a, x, y, GlobalEntries{a.buffer});
+    a.depth[y * a.width + x] = resolve_pixel<kDepthOnly>(a, x, y);
 }
 
 // Power-of-two supersampling: the pixels of each 64x64 splat tile in Morton order.  An
@@ -1295,75 +1316,131 @@ __device__ __forceinline__ uint32_t morton_compact(uint32_t a) {
     return a;
 }
 
-template <bool kDepthOnly>
-__global__ void __launch_bounds__(256) resolve_morton_kernel(ResolveArgs a, int ss_log2) {
-    previous_kernel_done();
-    report_counters(a);
+// Pixel of thread g in Morton-tile order.
+__device__ __forceinline__ void morton_pixel(const ResolveArgs& a, uint32_t g, int ss_log2, int& x, int& y) {
     const uint32_t tile_px = (uint32_t)kTileSize >> ss_log2;
     const uint32_t per_tile_log2 = 2u * (uint32_t)(kTileBits - ss_log2);
-    const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
     const uint32_t tile = g >> per_tile_log2;
     const uint32_t m = g & ((1u << per_tile_log2) - 1u);
     const uint32_t tiles_per_row = (uint32_t)((a.width * a.ss + kTileSize - 1) >> kTileBits);
-    const int x = (int)((tile % tiles_per_row) * tile_px + morton_compact(m));
-    const int y = (int)((tile / tiles_per_row) * tile_px + morton_compact(m >> 1));
-    if (x >= a.width || y >= a.height) return;
-    resolve_pixel<kDepthOnly>(a, x, y, GlobalEntries{a.buffer});
+    x = (int)((tile % tiles_per_row) * tile_px + morton_compact(m));
+    y = (int)((tile / tiles_per_row) * tile_px + morton_compact(m >> 1));
+}
+
+// With `hiz` (a.hiz_levels) the fine Hi-Z levels come with it, and a depth-only launch then
+// leaves the depth image itself to the final resolve.
+template <bool kDepthOnly>
+__global__ void __launch_bounds__(256) resolve_morton_kernel(ResolveArgs a, HizView hiz, int ss_log2) {
+    previous_kernel_done();
+    report_counters(a);
+    __shared__ float exchange[8];
+    int x, y;
+    morton_pixel(a, blockIdx.x * blockDim.x + threadIdx.x, ss_log2, x, y);
+    const bool inside = x < a.width && y < a.height;
+    float depth = 0.0f;
+    if (inside) depth = resolve_pixel<kDepthOnly>(a, x, y);
+    if (inside && !(kDepthOnly && a.hiz_fused)) a.depth[y * a.width + x] = depth;
+    if (a.hiz_fused) hiz_fine_levels(hiz, depth, x, y, a.hiz_min_levels, exchange);
 }
 
 // Staged variant: a block's pixels are consecutive in Morton-tile order, so their samples are
-// one contiguous run of the buffer (px_per_block x SS*SS*spp entries, at most 48 KB).  The
-// block copies the run to shared memory with coalesced 16-byte loads, all in flight at once,
-// then each thread resolves its pixel from shared memory with the same per-pixel code.  A pad
-// word after each pixel's samples keeps the threads of a warp, which read samples a whole
-// pixel run apart, on different banks.  Used when SS*SS*spp is a power of two >= 2.
+// one contiguous run of the buffer (px_per_block x SS*SS*spp entries, at most 48 KB), which the
+// block reads with coalesced 16-byte loads.  Used when SS*SS*spp is a power of two >= 2.
+//   depth only: of every entry pair the smaller high word goes to shared memory; a pixel's depth
+//     is that of its smallest key.  The conversion to NDC does not decrease with the key (every
+//     step of it rounds monotonically for 0 < near < far; checked over all 2^28 keys for 40 pairs
+//     of planes between 1e-6 and 1e9, and launch_resolve keeps to that range), so the smallest key's depth is the smallest depth, bit for bit.
+//   final: the run itself goes to shared memory, two pad words after each pixel's samples to keep
+//     a warp's 16-byte reads on different banks; the 12-bit channels become floats by their bits
+//     under 2^23 (exact), which keeps them off the conversion unit.
 constexpr int kResolveStageBytes = 48 * 1024;
-#ifndef GPS_RESOLVE_REVERSED
-#define GPS_RESOLVE_REVERSED 1
-#endif
-#ifndef GPS_RESOLVE_PIXELS
-#define GPS_RESOLVE_PIXELS 64
-#endif
+constexpr uint32_t kResolvePixels = 64;  // per block; 64 measured 155 us for both, 32 196, 256 162
 
-template <bool kDepthOnly>
-__global__ void __launch_bounds__(256) resolve_staged_kernel(ResolveArgs a, int ss_log2, int run_log2) {
+__device__ __forceinline__ float channel12(uint32_t c) { return __uint_as_float(0x4B000000u | (c & 0xFFFu)) - 8388608.0f; }
+
+__device__ __forceinline__ float depth_of_key(uint32_t high_word, const ResolveArgs& a) {
+    const float view_depth = view_depth_from_key((uint64_t)(high_word >> 4), a.near_plane, a.far_plane);
+    return gmin(1e9f, view_to_projected_depth(view_depth, a.near_plane, a.far_plane));
+}
+
+template <bool kDepthOnly, int kSsLog2>
+__global__ void __launch_bounds__(kResolvePixels) resolve_staged_kernel(ResolveArgs a, HizView hiz, int run_log2) {
     previous_kernel_done();
     report_counters(a);
-    extern __shared__ uint64_t stage[];
-    const uint32_t run = 1u << run_log2;                            // entries per pixel
+    extern __shared__ __align__(16) uint64_t stage[];
+    __shared__ float exchange[2];
     // blocks take the buffer from its end: the splat walks screen bins (buffer tiles) in
     // ascending order, so the tiles it touched last are the ones still in L2
-    const uint32_t bid = GPS_RESOLVE_REVERSED ? gridDim.x - 1u - blockIdx.x : blockIdx.x;
-    const uint32_t g0 = bid * blockDim.x;
-    const uint64_t first = (uint64_t)g0 * run;
-    uint64_t last = first + (uint64_t)blockDim.x * run;
-    if (last > a.entries) last = a.entries;
-    const uint32_t chunks = (uint32_t)((last - first) / 2);        // first and last are even
-    const ulonglong2* src = reinterpret_cast<const ulonglong2*>(a.buffer + first);
-    for (uint32_t i = threadIdx.x; i < chunks; i += blockDim.x) {
-        const ulonglong2 q = __ldcs(src + i);
-        const uint32_t w = 2u * i;                                  // both words in one pixel run
-        const uint32_t d = w + (w >> run_log2);
-        stage[d] = q.x;
-        stage[d + 1] = q.y;
+    const uint32_t g0 = (gridDim.x - 1u - blockIdx.x) * blockDim.x;
+    const uint32_t pairs = blockDim.x << (run_log2 - 1);
+    const ulonglong2* src = reinterpret_cast<const ulonglong2*>(a.buffer + ((uint64_t)g0 << run_log2));
+    int x, y;
+    morton_pixel(a, g0 + threadIdx.x, kSsLog2, x, y);
+    const bool inside = x < a.width && y < a.height;
+    float depth;
+    if (kDepthOnly) {
+        uint32_t* high = reinterpret_cast<uint32_t*>(stage);
+        const int half_log2 = run_log2 - 1;                    // words per pixel, then one pad word
+#pragma unroll 4
+        for (uint32_t i = threadIdx.x; i < pairs; i += blockDim.x) {
+            const uint4 q = __ldcs(reinterpret_cast<const uint4*>(src) + i);
+            high[i + (i >> half_log2)] = min(q.y, q.w);
+        }
+        __syncthreads();
+        const uint32_t* mine = high + threadIdx.x * ((1u << half_log2) + 1u);
+        uint32_t nearest = 0xFFFFFFFFu;
+#pragma unroll 8
+        for (int k = 0; k < (1 << half_log2); ++k) nearest = min(nearest, mine[k]);
+        depth = depth_of_key(nearest, a);
+    } else {
+        ulonglong2* put = reinterpret_cast<ulonglong2*>(stage);
+#pragma unroll 4
+        for (uint32_t i = threadIdx.x; i < pairs; i += blockDim.x) put[i + (i >> (run_log2 - 1))] = __ldcs(src + i);
+        __syncthreads();
+        const uint64_t* mine = stage + threadIdx.x * ((1u << run_log2) + 2u);
+        vec3 color = make_v3(0.0f, 0.0f, 0.0f);
+        uint32_t nearest = 0xFFFFFFFFu;
+        auto add = [&](uint64_t val) {
+            const uint32_t lo = (uint32_t)val, hi = (uint32_t)(val >> 32);
+            nearest = min(nearest, hi);
+            color.x += channel12(__funnelshift_r(lo, hi, 24)) / 255.0f;
+            color.y += channel12(lo >> 12) / 255.0f;
+            color.z += channel12(lo) / 255.0f;
+        };
+#pragma unroll
+        for (int dx = 0; dx < (1 << kSsLog2); ++dx)
+#pragma unroll
+            for (int dy = 0; dy < (1 << kSsLog2); ++dy) {
+                const uint64_t* at = mine + morton_encode((uint32_t)dx, (uint32_t)dy) * (uint32_t)a.num_passes;
+                if (a.num_passes == 1) {
+                    add(*at);
+                } else {
+                    for (int p = 0; p < a.num_passes; p += 2) {
+                        const ulonglong2 q = *reinterpret_cast<const ulonglong2*>(at + p);
+                        add(q.x);
+                        add(q.y);
+                    }
+                }
+            }
+        depth = depth_of_key(nearest, a);
+        if (inside) {
+            const uint32_t idx = (uint32_t)(y * a.width + x);
+            const float inv_passes = 1.0f / (float)(a.num_passes * a.ss * a.ss);
+            a.color[3 * idx + 0] = color.x * inv_passes;
+            a.color[3 * idx + 1] = color.y * inv_passes;
+            a.color[3 * idx + 2] = color.z * inv_passes;
+        }
     }
-    __syncthreads();
-    const uint32_t tile_px = (uint32_t)kTileSize >> ss_log2;
-    const uint32_t per_tile_log2 = 2u * (uint32_t)(kTileBits - ss_log2);
-    const uint32_t g = g0 + threadIdx.x;
-    const uint32_t tile = g >> per_tile_log2;
-    const uint32_t m = g & ((1u << per_tile_log2) - 1u);
-    const uint32_t tiles_per_row = (uint32_t)((a.width * a.ss + kTileSize - 1) >> kTileBits);
-    const int x = (int)((tile % tiles_per_row) * tile_px + morton_compact(m));
-    const int y = (int)((tile / tiles_per_row) * tile_px + morton_compact(m >> 1));
-    if (x >= a.width || y >= a.height) return;
-    resolve_pixel<kDepthOnly>(a, x, y, StagedEntries{stage, (int)first, run_log2});
+    if (inside && !(kDepthOnly && a.hiz_fused)) a.depth[y * a.width + x] = depth;
+    if (a.hiz_fused) hiz_fine_levels(hiz, depth, x, y, a.hiz_min_levels, exchange);
 }
 
 // ---------------------------------------------------------------------------------
 // Hi-Z chain (depth_mip_chain.cu:7-67)
 // ---------------------------------------------------------------------------------
-// The whole chain in one launch.  A 16x16-thread block covers a 64x64 tile of the depth image:
+// The whole chain in one launch, for views whose resolve does not write the fine levels (a
+// supersampling factor that is no power of two, runs of 128 samples and more, images of up to
+// four pixels).  A 16x16-thread block covers a 64x64 tile of the depth image:
 // each thread copies its 4x4 texels into the finest level and reduces them in registers to
 // the next two levels (2x2, then 1), the block reduces its 16x16 results through four more
 // levels in shared memory, and the block that finishes last (a counter, no waiting) reduces
@@ -1373,13 +1450,56 @@ __global__ void __launch_bounds__(256) resolve_staged_kernel(ResolveArgs a, int 
 constexpr int kHizThreads = 16;                  // threads per block edge
 constexpr int kHizTile = 4 * kHizThreads;        // finest texels per block edge
 
-__device__ __forceinline__ float hiz_op(bool use_min, float a, float b) { return use_min ? fminf(a, b) : fmaxf(a, b); }
+// The levels above `have`, by the block that finishes last (a counter, no waiting), with 256
+// threads: a level of up to 1024 texels is reduced in shared memory, so that the last levels cost
+// a barrier each and not a round trip through L2 (1080p: five levels above 30 x 17).
+__device__ __forceinline__ void hiz_coarse_levels(const HizView& c, int have, int min_levels) {
+    constexpr int kIn = 1024;
+    __shared__ float level[2][kIn];
+    __shared__ int s_last;
+    if (have <= 0) return;                                       // the chain is complete
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) s_last = atomicAdd(c.done, 1u) == gridDim.x * gridDim.y - 1;
+    __syncthreads();
+    if (!s_last) return;
+    __threadfence();
+    const int L = c.levels - 1;
+    int cur = 0;
+    bool staged = false;
+    for (int l = have - 1; l >= 0; --l) {
+        const bool use_min = (L - l) <= min_levels;
+        const int wl = c.level_w[l], hl = c.level_h[l];
+        const int wf = c.level_w[l + 1], hf = c.level_h[l + 1];
+        const float* fine = c.mip + c.level_off[l + 1];
+        if (!staged && wf * hf <= kIn) {
+            for (int i = threadIdx.x; i < wf * hf; i += blockDim.x) level[cur][i] = __ldcg(fine + i);
+            __syncthreads();
+            staged = true;
+        }
+        for (int i = threadIdx.x; i < wl * hl; i += blockDim.x) {
+            const int x = i % wl, y = i / wl;
+            float acc = hiz_identity(use_min);
+            for (int dy = 0; dy < 2; ++dy)
+                for (int dx = 0; dx < 2; ++dx) {
+                    const int fx = 2 * x + dx, fy = 2 * y + dy;
+                    if (fx < wf && fy < hf)
+                        acc = hiz_op(use_min, acc, staged ? level[cur][fy * wf + fx] : __ldcg(fine + (uint64_t)fy * wf + fx));
+                }
+            c.mip[c.level_off[l] + (uint64_t)y * wl + x] = acc;
+            if (staged) level[cur ^ 1][i] = acc;
+        }
+        if (staged) cur ^= 1;
+        else __threadfence_block();
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) *c.done = 0u;
+}
 
 __global__ void __launch_bounds__(kHizThreads * kHizThreads) hiz_build_kernel(HizView c, const float* __restrict__ src,
                                                                                int min_levels) {
     previous_kernel_done();
     __shared__ float sm[kHizThreads * kHizThreads];
-    __shared__ int s_last;
     const int L = c.levels - 1;
     const int tx = threadIdx.x % kHizThreads, ty = threadIdx.x / kHizThreads;
     const int gx = blockIdx.x * kHizThreads + tx, gy = blockIdx.y * kHizThreads + ty;  // coords at level L-2
@@ -1455,32 +1575,40 @@ __global__ void __launch_bounds__(kHizThreads * kHizThreads) hiz_build_kernel(Hi
         __syncthreads();
     }
     const int done_levels = (L >= 2 ? 2 : L) + shared_levels;   // levels below L written so far
-    if (done_levels >= L) return;                                // the whole chain fits one block
-    __threadfence();
-    __syncthreads();
-    if (threadIdx.x == 0) s_last = atomicAdd(c.done, 1u) == gridDim.x * gridDim.y - 1;
-    __syncthreads();
-    if (!s_last) return;
-    __threadfence();
-    for (int l = L - done_levels - 1; l >= 0; --l) {
-        const bool use_min = (L - 1 - l) < min_levels;
-        const int wl = c.level_w[l], hl = c.level_h[l];
-        const int wf = c.level_w[l + 1], hf = c.level_h[l + 1];
-        const float* fine = c.mip + c.level_off[l + 1];
-        for (int i = threadIdx.x; i < wl * hl; i += blockDim.x) {
-            const int x = i % wl, y = i / wl;
-            float acc = use_min ? INFINITY : -INFINITY;
-            for (int dy = 0; dy < 2; ++dy)
-                for (int dx = 0; dx < 2; ++dx) {
-                    const int fx = 2 * x + dx, fy = 2 * y + dy;
-                    if (fx < wf && fy < hf) acc = hiz_op(use_min, acc, __ldcg(fine + (uint64_t)fy * wf + fx));
-                }
-            c.mip[c.level_off[l] + (uint64_t)y * wl + x] = acc;
-        }
-        __threadfence_block();
+    hiz_coarse_levels(c, L - done_levels, min_levels);
+}
+
+// The rest of the chain above the levels that the resolve wrote (hiz_fine_levels): a block reduces
+// 16 x 16 texels of the 1/8-size level through four more levels, the last block does the others.
+__global__ void __launch_bounds__(256) hiz_top_kernel(HizView c, int min_levels) {
+    previous_kernel_done();
+    __shared__ float sm[256];
+    const int L = c.levels - 1, base = L - 3;
+    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+    const int gx = blockIdx.x * 16 + tx, gy = blockIdx.y * 16 + ty;
+    if (gx < c.level_w[base] && gy < c.level_h[base])
+        sm[threadIdx.x] = c.mip[c.level_off[base] + (uint64_t)gy * c.level_w[base] + gx];
+    const int steps = min(4, base);
+    for (int j = 1; j <= steps; ++j) {
         __syncthreads();
+        const int l = base - j, half = 16 >> j;
+        const bool use_min = (L - l) <= min_levels;
+        const int bx = blockIdx.x * half + tx, by = blockIdx.y * half + ty;
+        const bool act = tx < half && ty < half && bx < c.level_w[l] && by < c.level_h[l];
+        float acc = hiz_identity(use_min);
+        if (act) {
+            for (int dy = 0; dy < 2; ++dy)
+                for (int dx = 0; dx < 2; ++dx)
+                    if (2 * bx + dx < c.level_w[l + 1] && 2 * by + dy < c.level_h[l + 1])
+                        acc = hiz_op(use_min, acc, sm[(2 * ty + dy) * 16 + 2 * tx + dx]);
+        }
+        __syncthreads();
+        if (act) {
+            sm[ty * 16 + tx] = acc;
+            c.mip[c.level_off[l] + (uint64_t)by * c.level_w[l] + bx] = acc;
+        }
     }
-    if (threadIdx.x == 0) *c.done = 0u;
+    hiz_coarse_levels(c, base - steps, min_levels);
 }
 
 // ---------------------------------------------------------------------------------
@@ -1927,10 +2055,24 @@ void launch_clear(uint64_t* buf, uint64_t entries, uint64_t value, cudaStream_t 
     if (entries & 1) cudaMemcpyAsync(buf + entries - 1, &buf[0], 8, cudaMemcpyDeviceToDevice, stream);
 }
 
-void launch_resolve(const ResolveArgs& a, bool depth_only, cudaStream_t stream) {
+template <bool kDepthOnly>
+void launch_resolve_staged(const ResolveArgs& a, const HizView& hiz, int ss_log2, int run_log2, unsigned grid,
+                           uint32_t px, cudaStream_t stream) {
+    const size_t smem = kDepthOnly ? (size_t)px * ((1u << (run_log2 - 1)) + 1u) * 4u
+                                   : (size_t)px * ((1u << run_log2) + 2u) * 8u;
+    if (ss_log2 == 0) launch_k(resolve_staged_kernel<kDepthOnly, 0>, grid, px, smem, stream, a, hiz, run_log2);
+    else if (ss_log2 == 1) launch_k(resolve_staged_kernel<kDepthOnly, 1>, grid, px, smem, stream, a, hiz, run_log2);
+    else if (ss_log2 == 2) launch_k(resolve_staged_kernel<kDepthOnly, 2>, grid, px, smem, stream, a, hiz, run_log2);
+    else launch_k(resolve_staged_kernel<kDepthOnly, 3>, grid, px, smem, stream, a, hiz, run_log2);
+}
+
+int launch_resolve(const ResolveArgs& args, const HizView* hiz, bool depth_only, cudaStream_t stream) {
+    ResolveArgs a = args;
+    const HizView none{};
     int ss_log2 = -1;
     for (int l = 0; l <= 3; ++l)
         if (a.ss == (1 << l)) ss_log2 = l;
+    a.hiz_fused = 0;
     if (ss_log2 >= 0) {
         const uint64_t tiles = ((uint64_t)(a.width * a.ss + kTileSize - 1) >> kTileBits) *
                                ((uint64_t)(a.height * a.ss + kTileSize - 1) >> kTileBits);
@@ -1939,29 +2081,41 @@ void launch_resolve(const ResolveArgs& a, bool depth_only, cudaStream_t stream) 
         int run_log2 = -1;
         for (int l = 1; l <= 12; ++l)
             if (run == (1u << l)) run_log2 = l;
-        const uint32_t run_bytes = (run + 1u) * 8u;                 // with the pad word
-        uint32_t px = GPS_RESOLVE_PIXELS;  // pixels (threads) per block
-        while (px > 32 && px * run_bytes > (uint32_t)kResolveStageBytes) px >>= 1;
-        if (run_log2 > 0 && px * run_bytes <= (uint32_t)kResolveStageBytes && (uint64_t)a.entries <= 0x7FFFFFFFull) {
+        const uint32_t run_bytes = (run + 2u) * 8u;                 // with the pad words
+        uint32_t px = kResolvePixels;  // pixels (threads) per block
+        if (px * run_bytes > (uint32_t)kResolveStageBytes) px >>= 1;
+        // staged: runs of up to 48 KB per block, and planes for which a key's depth is monotone
+        // (through zero or past the float range it is not); the fine Hi-Z levels need groups of 64 pixels and a chain of at least four levels
+        const bool staged = run_log2 > 0 && px * run_bytes <= (uint32_t)kResolveStageBytes &&
+                            (uint64_t)a.entries <= 0x7FFFFFFFull && a.near_plane >= 1.0e-6f &&
+                            a.far_plane <= 1.0e9f;
+        a.hiz_fused = hiz && hiz->levels >= 4 && (!staged || px == kResolvePixels) ? 1 : 0;
+        const HizView& h = a.hiz_fused ? *hiz : none;
+        if (staged) {
             const unsigned grid = (unsigned)((threads + px - 1) / px);
-            const size_t smem = (size_t)px * run_bytes;
-            if (depth_only) launch_k(resolve_staged_kernel<true>, grid, px, smem, stream, a, ss_log2, run_log2);
-            else launch_k(resolve_staged_kernel<false>, grid, px, smem, stream, a, ss_log2, run_log2);
-            return;
+            if (depth_only) launch_resolve_staged<true>(a, h, ss_log2, run_log2, grid, px, stream);
+            else launch_resolve_staged<false>(a, h, ss_log2, run_log2, grid, px, stream);
+        } else {
+            const unsigned grid = (unsigned)((threads + 255) / 256);
+            if (depth_only) launch_k(resolve_morton_kernel<true>, grid, 256, 0, stream, a, h, ss_log2);
+            else launch_k(resolve_morton_kernel<false>, grid, 256, 0, stream, a, h, ss_log2);
         }
-        const unsigned grid = (unsigned)((threads + 255) / 256);
-        if (depth_only) launch_k(resolve_morton_kernel<true>, grid, 256, 0, stream, a, ss_log2);
-        else launch_k(resolve_morton_kernel<false>, grid, 256, 0, stream, a, ss_log2);
-        return;
+    } else {
+        dim3 block(16, 16);
+        dim3 grid((a.width + 15) / 16, (a.height + 15) / 16);
+        if (depth_only) launch_k(resolve_kernel<true>, grid, block, 0, stream, a);
+        else launch_k(resolve_kernel<false>, grid, block, 0, stream, a);
     }
-    dim3 block(16, 16);
-    dim3 grid((a.width + 15) / 16, (a.height + 15) / 16);
-    if (depth_only) launch_k(resolve_kernel<true>, grid, block, 0, stream, a);
-    else launch_k(resolve_kernel<false>, grid, block, 0, stream, a);
+    return a.hiz_fused;
 }
 
-void launch_hiz_build(const HizView& h, const float* depth, int min_levels, cudaStream_t stream) {
+void launch_hiz_build(const HizView& h, const float* depth, int min_levels, bool fine_done, cudaStream_t stream) {
     const int L = h.levels - 1;
+    if (fine_done) {
+        if (L == 3) return;
+        launch_k(hiz_top_kernel, dim3((h.level_w[L - 3] + 15) / 16, (h.level_h[L - 3] + 15) / 16), 256, 0, stream, h, min_levels);
+        return;
+    }
     dim3 grid((h.level_w[L] + kHizTile - 1) / kHizTile, (h.level_h[L] + kHizTile - 1) / kHizTile);
     launch_k(hiz_build_kernel, grid, kHizThreads * kHizThreads, 0, stream, h, depth, min_levels);
 }

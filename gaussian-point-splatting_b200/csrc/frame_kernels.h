@@ -213,6 +213,8 @@ struct ResolveArgs {
     const PassCounters* report_from;
     PassCounters* report_to;  // [2], pinned host memory
     int report_passes;
+    int hiz_min_levels;
+    int hiz_fused;  // set by launch_resolve: the launch writes the fine Hi-Z levels
 };
 
 // launchers (all asynchronous on `stream`)
@@ -242,8 +244,11 @@ uint32_t scan_tile_count(uint32_t n);
 constexpr uint32_t kScanTileGaussians = 16384;  // Gaussians per scan tile (counts are padded to it)
 void launch_splat(const SplatArgs& a, int grid, int block, cudaStream_t stream);
 void launch_clear(uint64_t* buf, uint64_t entries, uint64_t value, cudaStream_t stream);
-void launch_resolve(const ResolveArgs& a, bool depth_only, cudaStream_t stream);
-void launch_hiz_build(const HizView& h, const float* depth, int min_levels, cudaStream_t stream);
+// hiz: also write its four finest levels where this view's resolve can (the result says so; a
+// depth-only launch then does not write a.depth).
+int launch_resolve(const ResolveArgs& a, const HizView* hiz, bool depth_only, cudaStream_t stream);
+// The Hi-Z chain of `depth`, or what is left of it after a resolve that wrote the fine levels.
+void launch_hiz_build(const HizView& h, const float* depth, int min_levels, bool fine_done, cudaStream_t stream);
 void launch_block_bounds(const float4* pos_op, const float4* rot, const float4* scale, uint32_t n,
                          uint32_t per_block, float4* nodes, cudaStream_t stream);
 // Scene order on the device: order[j] = the input index of the j-th Gaussian in 3D Morton order

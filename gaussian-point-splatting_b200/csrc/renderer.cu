@@ -972,14 +972,18 @@ gps_status render_frame_impl(gps_renderer* r, const gps_camera* cam, float* d_im
     ra.near_plane = r->s.near_view_plane;
     ra.far_plane = r->s.far_view_plane;
     ra.initial_value = bg;
+    ra.hiz_min_levels = r->s.occlusion_culling_min_reduce_count;
+    auto build_hiz = [&](bool fine_done) {
+        r->timer.mark(kStHiz, st);
+        launch_hiz_build(r->hiz, d_depth, r->s.occlusion_culling_min_reduce_count, fine_done, st);
+        if (!fine_done || r->hiz.levels > 4) count_launch(r, kStHiz);
+    };
     r->second_pass_last = false;
     if (r->s.enable_occlusion_culling) {
         r->timer.mark(kStResolve, st);
-        launch_resolve(ra, true, st);
+        const bool fine = launch_resolve(ra, &r->hiz, true, st) != 0;
         count_launch(r, kStResolve);
-        r->timer.mark(kStHiz, st);
-        launch_hiz_build(r->hiz, d_depth, r->s.occlusion_culling_min_reduce_count, st);
-        count_launch(r, kStHiz);
+        build_hiz(fine);
         if (r->n > 0) {
             render_pass(r, fc, cam->frame, false, st);
             r->second_pass_last = true;
@@ -989,13 +993,9 @@ gps_status render_frame_impl(gps_renderer* r, const gps_camera* cam, float* d_im
     ra.report_to = r->host_counters;
     ra.report_passes = r->n == 0 ? 0 : r->s.enable_occlusion_culling ? 2 : 1;
     r->timer.mark(kStResolve, st);
-    launch_resolve(ra, false, st);
+    const bool fine = launch_resolve(ra, r->s.enable_occlusion_culling ? &r->hiz : nullptr, false, st) != 0;
     count_launch(r, kStResolve);
-    if (r->s.enable_occlusion_culling) {
-        r->timer.mark(kStHiz, st);
-        launch_hiz_build(r->hiz, d_depth, r->s.occlusion_culling_min_reduce_count, st);
-        count_launch(r, kStHiz);
-    }
+    if (r->s.enable_occlusion_culling) build_hiz(fine);
     r->timer.mark(-1, st);
     cudaEventRecord(r->done, st);
     r->have_frame = true;
