@@ -1270,7 +1270,8 @@ __device__ __forceinline__ void hiz_fine_levels(const HizView& c, float depth, i
     const int L = c.levels - 1;  // the caller checked L >= 3
     const uint32_t m = threadIdx.x & 63u;
     bool exists = x < c.level_w[L] && y < c.level_h[L];
-    if (exists) c.mip[c.level_off[L] + (uint64_t)y * c.level_w[L] + x] = depth;
+    // (32-bit indices: a view has fewer than 2^31 samples)
+    if (exists) (c.mip + c.level_off[L])[(uint32_t)(y * c.level_w[L] + x)] = depth;
     float v = depth;
 #pragma unroll
     for (int j = 1; j <= 3; ++j) {
@@ -1288,7 +1289,7 @@ __device__ __forceinline__ void hiz_fine_levels(const HizView& c, float depth, i
         x >>= 1;
         y >>= 1;
         exists = x < c.level_w[l] && y < c.level_h[l];
-        if (exists && (m & ((1u << (2 * j)) - 1u)) == 0u) c.mip[c.level_off[l] + (uint64_t)y * c.level_w[l] + x] = v;
+        if (exists && (m & ((1u << (2 * j)) - 1u)) == 0u) (c.mip + c.level_off[l])[(uint32_t)(y * c.level_w[l] + x)] = v;
     }
 }
 
@@ -1345,16 +1346,27 @@ __global__ void __launch_bounds__(256) resolve_morton_kernel(ResolveArgs a, HizV
 
 // Staged variant: a block's pixels are consecutive in Morton-tile order, so their samples are
 // one contiguous run of the buffer (px_per_block x SS*SS*spp entries, at most 48 KB), which the
-// block reads with coalesced 16-byte loads.  Used when SS*SS*spp is a power of two >= 2.
+// block reads with coalesced 16-byte loads.  Used when SS*SS*spp is a power of two in 2..128.
 //   depth only: of every entry pair the smaller high word goes to shared memory; a pixel's depth
 //     is that of its smallest key.  The conversion to NDC does not decrease with the key (every
 //     step of it rounds monotonically for 0 < near < far; checked over all 2^28 keys for 40 pairs
-//     of planes between 1e-6 and 1e9, and launch_resolve keeps to that range), so the smallest key's depth is the smallest depth, bit for bit.
+//     of planes between 1e-6 and 1e9, and launch_resolve keeps to that range), so the smallest
+//     key's depth is the smallest depth, bit for bit.
 //   final: the run itself goes to shared memory, two pad words after each pixel's samples to keep
 //     a warp's 16-byte reads on different banks; the 12-bit channels become floats by their bits
 //     under 2^23 (exact), which keeps them off the conversion unit.
-constexpr int kResolveStageBytes = 48 * 1024;
-constexpr uint32_t kResolvePixels = 64;  // per block; 64 measured 155 us for both, 32 196, 256 162
+// The kernel was bound by instructions, not by the 8 bytes per sample: with run-time sizes, a
+// division per pixel and 64-bit indices it took 40 (depth) and 63 (final) instructions per sample
+// at 8 samples a pixel; sizes are now template parameters and the grid is tiles_x * blocks per
+// tile by tiles_y:
+// 28 and 44, and 1M town at 4K, 2 spp: 111 -> 88 us (depth; the 531 MB take 82 at the copy rate) and
+// 175 -> 136 us, the frame 995 -> 943; 500k town at 720p, 1 spp: 139 -> 127.
+constexpr int kResolveMaxRunLog2 = 7;
+// 64 pixels per block (155 us for both resolves at 1080p; 32 196, 256 162), 32 at 128 samples each
+__host__ __device__ constexpr uint32_t resolve_pixels(int run_log2) { return run_log2 <= 6 ? 64u : 32u; }
+__host__ __device__ constexpr int resolve_blocks_log2(int ss_log2, int run_log2) {  // blocks per tile
+    return 2 * (kTileBits - ss_log2) - (run_log2 <= 6 ? 6 : 5);
+}
 
 __device__ __forceinline__ float channel12(uint32_t c) { return __uint_as_float(0x4B000000u | (c & 0xFFFu)) - 8388608.0f; }
 
@@ -1363,43 +1375,45 @@ __device__ __forceinline__ float depth_of_key(uint32_t high_word, const ResolveA
     return gmin(1e9f, view_to_projected_depth(view_depth, a.near_plane, a.far_plane));
 }
 
-template <bool kDepthOnly, int kSsLog2>
-__global__ void __launch_bounds__(kResolvePixels) resolve_staged_kernel(ResolveArgs a, HizView hiz, int run_log2) {
+template <bool kDepthOnly, int kSsLog2, int kRunLog2>
+__global__ void __launch_bounds__(resolve_pixels(kRunLog2)) resolve_staged_kernel(ResolveArgs a, HizView hiz) {
     previous_kernel_done();
     report_counters(a);
-    extern __shared__ __align__(16) uint64_t stage[];
+    constexpr uint32_t kPx = resolve_pixels(kRunLog2), kRun = 1u << kRunLog2, kHalf = kRun / 2u;
+    constexpr int kBlocksLog2 = resolve_blocks_log2(kSsLog2, kRunLog2);
+    constexpr uint32_t kTilePxLog2 = (uint32_t)(kTileBits - kSsLog2);
+    // a pad word (depth only: 4 bytes, final: 16) follows the kHalf words of each pixel
+    __shared__ __align__(16) uint32_t stage[kPx * (kHalf + 1u) * (kDepthOnly ? 1u : 4u)];
     __shared__ float exchange[2];
     // blocks take the buffer from its end: the splat walks screen bins (buffer tiles) in
     // ascending order, so the tiles it touched last are the ones still in L2
-    const uint32_t g0 = (gridDim.x - 1u - blockIdx.x) * blockDim.x;
-    const uint32_t pairs = blockDim.x << (run_log2 - 1);
-    const ulonglong2* src = reinterpret_cast<const ulonglong2*>(a.buffer + ((uint64_t)g0 << run_log2));
-    int x, y;
-    morton_pixel(a, g0 + threadIdx.x, kSsLog2, x, y);
+    const uint32_t bx = gridDim.x - 1u - blockIdx.x, ty = gridDim.y - 1u - blockIdx.y;
+    const uint32_t tx = bx >> kBlocksLog2, sub = bx & ((1u << kBlocksLog2) - 1u);
+    const uint32_t tile = ty * (gridDim.x >> kBlocksLog2) + tx, t = threadIdx.x;
+    const ulonglong2* src = reinterpret_cast<const ulonglong2*>(a.buffer) +
+                            ((uint64_t)((tile << kBlocksLog2) + sub) * (kPx * kHalf) + t);
+    const int x = (int)((tx << kTilePxLog2) + morton_compact(sub * kPx) + morton_compact(t));
+    const int y = (int)((ty << kTilePxLog2) + morton_compact((sub * kPx) >> 1) + morton_compact(t >> 1));
     const bool inside = x < a.width && y < a.height;
-    float depth;
+    uint32_t nearest = 0xFFFFFFFFu;
     if (kDepthOnly) {
-        uint32_t* high = reinterpret_cast<uint32_t*>(stage);
-        const int half_log2 = run_log2 - 1;                    // words per pixel, then one pad word
-#pragma unroll 4
-        for (uint32_t i = threadIdx.x; i < pairs; i += blockDim.x) {
-            const uint4 q = __ldcs(reinterpret_cast<const uint4*>(src) + i);
-            high[i + (i >> half_log2)] = min(q.y, q.w);
+        uint32_t* put = stage + t + t / kHalf;
+#pragma unroll 8
+        for (uint32_t k = 0; k < kHalf; ++k) {
+            const uint4 q = __ldcs(reinterpret_cast<const uint4*>(src + k * kPx));
+            put[k * kPx + k * kPx / kHalf] = min(q.y, q.w);
         }
         __syncthreads();
-        const uint32_t* mine = high + threadIdx.x * ((1u << half_log2) + 1u);
-        uint32_t nearest = 0xFFFFFFFFu;
-#pragma unroll 8
-        for (int k = 0; k < (1 << half_log2); ++k) nearest = min(nearest, mine[k]);
-        depth = depth_of_key(nearest, a);
+        const uint32_t* mine = stage + t * (kHalf + 1u);
+#pragma unroll
+        for (uint32_t k = 0; k < kHalf; ++k) nearest = min(nearest, mine[k]);
     } else {
-        ulonglong2* put = reinterpret_cast<ulonglong2*>(stage);
-#pragma unroll 4
-        for (uint32_t i = threadIdx.x; i < pairs; i += blockDim.x) put[i + (i >> (run_log2 - 1))] = __ldcs(src + i);
+        ulonglong2* put = reinterpret_cast<ulonglong2*>(stage) + t + t / kHalf;
+#pragma unroll 8
+        for (uint32_t k = 0; k < kHalf; ++k) put[k * kPx + k * kPx / kHalf] = __ldcs(src + k * kPx);
         __syncthreads();
-        const uint64_t* mine = stage + threadIdx.x * ((1u << run_log2) + 2u);
+        const uint64_t* mine = reinterpret_cast<const uint64_t*>(stage) + t * (kRun + 2u);
         vec3 color = make_v3(0.0f, 0.0f, 0.0f);
-        uint32_t nearest = 0xFFFFFFFFu;
         auto add = [&](uint64_t val) {
             const uint32_t lo = (uint32_t)val, hi = (uint32_t)(val >> 32);
             nearest = min(nearest, hi);
@@ -1407,22 +1421,23 @@ __global__ void __launch_bounds__(kResolvePixels) resolve_staged_kernel(ResolveA
             color.y += channel12(lo >> 12) / 255.0f;
             color.z += channel12(lo) / 255.0f;
         };
+        constexpr uint32_t kPasses = kRun >> (2 * kSsLog2);
 #pragma unroll
         for (int dx = 0; dx < (1 << kSsLog2); ++dx)
 #pragma unroll
             for (int dy = 0; dy < (1 << kSsLog2); ++dy) {
-                const uint64_t* at = mine + morton_encode((uint32_t)dx, (uint32_t)dy) * (uint32_t)a.num_passes;
-                if (a.num_passes == 1) {
+                const uint64_t* at = mine + morton_encode((uint32_t)dx, (uint32_t)dy) * kPasses;
+                if constexpr (kPasses == 1u) {
                     add(*at);
                 } else {
-                    for (int p = 0; p < a.num_passes; p += 2) {
+#pragma unroll 8
+                    for (uint32_t p = 0; p < kPasses; p += 2u) {
                         const ulonglong2 q = *reinterpret_cast<const ulonglong2*>(at + p);
                         add(q.x);
                         add(q.y);
                     }
                 }
             }
-        depth = depth_of_key(nearest, a);
         if (inside) {
             const uint32_t idx = (uint32_t)(y * a.width + x);
             const float inv_passes = 1.0f / (float)(a.num_passes * a.ss * a.ss);
@@ -1431,8 +1446,11 @@ __global__ void __launch_bounds__(kResolvePixels) resolve_staged_kernel(ResolveA
             a.color[3 * idx + 2] = color.z * inv_passes;
         }
     }
-    if (inside && !(kDepthOnly && a.hiz_fused)) a.depth[y * a.width + x] = depth;
-    if (a.hiz_fused) hiz_fine_levels(hiz, depth, x, y, a.hiz_min_levels, exchange);
+    const float depth = depth_of_key(nearest, a);
+    if (inside && !(kDepthOnly && a.hiz_fused)) a.depth[(uint32_t)(y * a.width + x)] = depth;
+    if constexpr (kPx == 64u) {
+        if (a.hiz_fused) hiz_fine_levels(hiz, depth, x, y, a.hiz_min_levels, exchange);
+    }
 }
 
 // ---------------------------------------------------------------------------------
@@ -2055,15 +2073,19 @@ void launch_clear(uint64_t* buf, uint64_t entries, uint64_t value, cudaStream_t 
     if (entries & 1) cudaMemcpyAsync(buf + entries - 1, &buf[0], 8, cudaMemcpyDeviceToDevice, stream);
 }
 
-template <bool kDepthOnly>
-void launch_resolve_staged(const ResolveArgs& a, const HizView& hiz, int ss_log2, int run_log2, unsigned grid,
-                           uint32_t px, cudaStream_t stream) {
-    const size_t smem = kDepthOnly ? (size_t)px * ((1u << (run_log2 - 1)) + 1u) * 4u
-                                   : (size_t)px * ((1u << run_log2) + 2u) * 8u;
-    if (ss_log2 == 0) launch_k(resolve_staged_kernel<kDepthOnly, 0>, grid, px, smem, stream, a, hiz, run_log2);
-    else if (ss_log2 == 1) launch_k(resolve_staged_kernel<kDepthOnly, 1>, grid, px, smem, stream, a, hiz, run_log2);
-    else if (ss_log2 == 2) launch_k(resolve_staged_kernel<kDepthOnly, 2>, grid, px, smem, stream, a, hiz, run_log2);
-    else launch_k(resolve_staged_kernel<kDepthOnly, 3>, grid, px, smem, stream, a, hiz, run_log2);
+template <bool kDepthOnly, int kSsLog2, int kRunLog2>
+void launch_resolve_staged(const ResolveArgs& a, const HizView& hiz, dim3 tiles, int ss_log2, int run_log2,
+                           cudaStream_t stream) {
+    if constexpr (kSsLog2 <= 3 && kRunLog2 <= kResolveMaxRunLog2) {
+        if (ss_log2 == kSsLog2 && run_log2 == kRunLog2) {
+            launch_k(resolve_staged_kernel<kDepthOnly, kSsLog2, kRunLog2>,
+                     dim3(tiles.x << resolve_blocks_log2(kSsLog2, kRunLog2), tiles.y), resolve_pixels(kRunLog2), 0, stream, a, hiz);
+        } else if (kRunLog2 < kResolveMaxRunLog2) {
+            launch_resolve_staged<kDepthOnly, kSsLog2, kRunLog2 + 1>(a, hiz, tiles, ss_log2, run_log2, stream);
+        } else {
+            launch_resolve_staged<kDepthOnly, kSsLog2 + 1, (kSsLog2 ? 2 * kSsLog2 + 2 : 2)>(a, hiz, tiles, ss_log2, run_log2, stream);
+        }
+    }
 }
 
 int launch_resolve(const ResolveArgs& args, const HizView* hiz, bool depth_only, cudaStream_t stream) {
@@ -2074,28 +2096,22 @@ int launch_resolve(const ResolveArgs& args, const HizView* hiz, bool depth_only,
         if (a.ss == (1 << l)) ss_log2 = l;
     a.hiz_fused = 0;
     if (ss_log2 >= 0) {
-        const uint64_t tiles = ((uint64_t)(a.width * a.ss + kTileSize - 1) >> kTileBits) *
-                               ((uint64_t)(a.height * a.ss + kTileSize - 1) >> kTileBits);
-        const uint64_t threads = tiles << (2 * (kTileBits - ss_log2));
+        const dim3 tiles((unsigned)((a.width * a.ss + kTileSize - 1) >> kTileBits),
+                         (unsigned)((a.height * a.ss + kTileSize - 1) >> kTileBits));
         const uint32_t run = (uint32_t)(a.ss * a.ss * a.num_passes);
-        int run_log2 = -1;
-        for (int l = 1; l <= 12; ++l)
+        int run_log2 = 0;
+        for (int l = 1; l <= kResolveMaxRunLog2; ++l)
             if (run == (1u << l)) run_log2 = l;
-        const uint32_t run_bytes = (run + 2u) * 8u;                 // with the pad words
-        uint32_t px = kResolvePixels;  // pixels (threads) per block
-        if (px * run_bytes > (uint32_t)kResolveStageBytes) px >>= 1;
-        // staged: runs of up to 48 KB per block, and planes for which a key's depth is monotone
-        // (through zero or past the float range it is not); the fine Hi-Z levels need groups of 64 pixels and a chain of at least four levels
-        const bool staged = run_log2 > 0 && px * run_bytes <= (uint32_t)kResolveStageBytes &&
-                            (uint64_t)a.entries <= 0x7FFFFFFFull && a.near_plane >= 1.0e-6f &&
-                            a.far_plane <= 1.0e9f;
-        a.hiz_fused = hiz && hiz->levels >= 4 && (!staged || px == kResolvePixels) ? 1 : 0;
+        // staged: planes for which a key's depth is monotone (through zero or past the float
+        // range it is not); the fine Hi-Z levels need groups of 64 pixels, a chain of four levels
+        const bool staged = run_log2 > 0 && a.near_plane >= 1.0e-6f && a.far_plane <= 1.0e9f;
+        a.hiz_fused = hiz && hiz->levels >= 4 && (!staged || resolve_pixels(run_log2) == 64u) ? 1 : 0;
         const HizView& h = a.hiz_fused ? *hiz : none;
         if (staged) {
-            const unsigned grid = (unsigned)((threads + px - 1) / px);
-            if (depth_only) launch_resolve_staged<true>(a, h, ss_log2, run_log2, grid, px, stream);
-            else launch_resolve_staged<false>(a, h, ss_log2, run_log2, grid, px, stream);
+            if (depth_only) launch_resolve_staged<true, 0, 1>(a, h, tiles, ss_log2, run_log2, stream);
+            else launch_resolve_staged<false, 0, 1>(a, h, tiles, ss_log2, run_log2, stream);
         } else {
+            const uint64_t threads = ((uint64_t)tiles.x * tiles.y) << (2 * (kTileBits - ss_log2));
             const unsigned grid = (unsigned)((threads + 255) / 256);
             if (depth_only) launch_k(resolve_morton_kernel<true>, grid, 256, 0, stream, a, h, ss_log2);
             else launch_k(resolve_morton_kernel<false>, grid, 256, 0, stream, a, h, ss_log2);
