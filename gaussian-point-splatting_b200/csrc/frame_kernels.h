@@ -37,7 +37,9 @@ struct BlockView {
     uint32_t node_count;
     uint32_t words;
     uint32_t per_block;    // Gaussians per block
-    uint32_t* chunk_count; // visible-chunk counter, reset by the block cull
+    uint32_t* chunk_count; // visible-chunk counter, zero before the cull (the splat resets it)
+    const float4* supers;  // the box around every 32 nodes, 2 float4 each
+    uint32_t* outside;     // one bit per node: outside the frustum in the frame's first pass
 };
 
 // Device-side counters of one render pass, readable by later kernels without a host sync.
@@ -69,6 +71,23 @@ struct FrameConst {
     int enable_occlusion;
     int enable_hier;
     int width, height;
+};
+
+// The block cull of one pass and, in a frame's first launch, the splat buffer's clear.
+struct CullArgs {
+    BlockView b;
+    FrameConst fc;
+    HizView hiz;
+    uint32_t n;
+    uint32_t* list;              // out: chunks with a visible block, b.chunk_count of them
+    uint32_t* mask_pair[2];      // the culled chunks' words are zeroed in the one *mask_iter selects
+    const uint32_t* mask_iter;
+    int second_pass;             // same camera as the pass before: b.outside holds
+    ulonglong2* clear;
+    uint64_t clear_pairs;        // 0: no clear
+    unsigned long long clear_value;
+    uint32_t cull_blocks;        // set by launch_cull
+    uint32_t words_per_block;
 };
 
 struct PreprocessArgs {
@@ -155,6 +174,7 @@ struct SplatArgs {
     unsigned long long* clear_b;
     uint32_t clear_b_words;
     uint32_t* mask_iter;             // advanced after a pass with points (null: not here)
+    uint32_t* chunk_count;           // the cull's list length, zeroed for the next pass (null: no list)
 };
 
 // Screen bins: the splat walks a pass's survivors grouped by the 64x64 splat-buffer tile (or
@@ -218,13 +238,9 @@ struct ResolveArgs {
 };
 
 // launchers (all asynchronous on `stream`)
-void launch_block_cull(const BlockView& b, const FrameConst& fc, const HizView& hiz, cudaStream_t stream);
-// Lists the 32-Gaussian chunks that hold at least one unculled block and zeroes the survivor
-// mask words of the others.
-// Zeroes the survivor-mask words of chunks without a visible block in the current mask: mask_a,
-// or the one of (mask_a, mask_b) that *mask_iter selects when mask_iter is set.
-void launch_visible_chunks(const BlockView& b, uint32_t n, uint32_t* list, uint32_t* mask_a, uint32_t* mask_b,
-                           const uint32_t* mask_iter, cudaStream_t stream);
+void launch_cull(const CullArgs& a, cudaStream_t stream);
+// The boxes around every 32 block nodes (load time).
+void launch_super_bounds(const float4* nodes, uint32_t node_count, float4* supers, cudaStream_t stream);
 void launch_preprocess_fp32(const PreprocessArgs& a, const SceneFP32& s, cudaStream_t stream);
 void launch_preprocess_compressed(const PreprocessArgs& a, const SceneCompressed& s, cudaStream_t stream);
 void launch_preprocess_half(const PreprocessArgs& a, const SceneHalf& s, cudaStream_t stream);

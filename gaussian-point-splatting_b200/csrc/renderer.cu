@@ -103,6 +103,7 @@ struct gps_scene {
     // fixed-size blocks for the hierarchical cull (computed from the FP32 values, like
     // build_fixed_blocks on the host CPUGaussian array)
     dptr<float4> block_nodes;
+    dptr<float4> block_supers;  // the box around every 32 of them
     uint32_t per_block = 4;
     uint32_t block_count = 0;
 };
@@ -214,6 +215,8 @@ void scene_upload(gps_scene* s, const CpuGaussian* g, uint64_t n, bool device_so
     float4* nodes = dev_alloc<float4>((size_t)s->block_count * 2);
     s->block_nodes.reset(nodes);
     launch_block_bounds(d_pos, d_rot, d_scale, (uint32_t)n, s->per_block, nodes, 0);
+    s->block_supers.reset(dev_alloc<float4>(((size_t)s->block_count + 31) / 32 * 2));
+    launch_super_bounds(nodes, s->block_count, s->block_supers.get(), 0);
     GPS_CUDA(cudaGetLastError());
     if (s->format == GPS_SCENE_HALF) {
         s->h_rec.reset(dev_alloc<uint4>(n));
@@ -309,7 +312,7 @@ struct gps_renderer {
     uint64_t entries = 0;
     uint32_t n = 0, n_pad = 0;
     dptr<uint64_t> buffer;
-    dptr<uint32_t> counts, mask[2], surv_gid, surv_start, tile_first_rank, culled, chunk_list, chunk_count, loaded;
+    dptr<uint32_t> counts, mask[2], surv_gid, surv_start, tile_first_rank, culled, outside, chunk_list, chunk_count, loaded;
     dptr<SplatRecord> records;
     dptr<unsigned long long> tile_state;
     dptr<unsigned long long> bins;  // screen-bin histogram / cursors, kMaxBins + 1 words
@@ -399,7 +402,30 @@ BlockView block_view(gps_renderer* r) {
     b.node_count = r->scene->block_count;
     b.words = (b.node_count + 31) / 32;
     b.per_block = r->scene->per_block;
+    b.supers = r->scene->block_supers.get();
+    b.outside = r->outside.get();
     return b;
+}
+
+// The block cull and chunk list of a pass; the frame's first launch, which also clears the splat
+// buffer, when `clear_value` is given.
+void cull_blocks(gps_renderer* r, const FrameConst& fc, const unsigned long long* clear_value, cudaStream_t st) {
+    CullArgs a{};
+    a.b = block_view(r);
+    a.fc = fc;
+    a.hiz = r->hiz;
+    a.n = r->n;
+    a.list = r->chunk_list.get();
+    a.mask_pair[0] = r->mask[0].get();
+    a.mask_pair[1] = r->mask[1].get();
+    a.mask_iter = r->mask_iter.get();
+    a.second_pass = clear_value ? 0 : 1;
+    if (clear_value) {
+        a.clear = reinterpret_cast<ulonglong2*>(r->buffer.get());
+        a.clear_pairs = r->entries / 2;  // a multiple of 4096 entries
+        a.clear_value = *clear_value;
+    }
+    launch_cull(a, st);
 }
 
 void count_launch(gps_renderer* r, int stage, uint64_t n = 1) {
@@ -416,12 +442,10 @@ void render_pass(gps_renderer* r, const FrameConst& fc, int frame, bool first, c
     const int frame_seed = 4 * frame + (first ? 0 : 2);
     BlockView blocks = block_view(r);
     const bool listed = fc.enable_hier && blocks.node_count;
-    if (listed) {
+    if (listed && !first) {  // (the first pass's cull came with the clear)
         r->timer.mark(kStCull, st);
-        launch_block_cull(blocks, fc, r->hiz, st);
-        launch_visible_chunks(blocks, r->n, r->chunk_list.get(), r->mask[0].get(), r->mask[1].get(),
-                              r->mask_iter.get(), st);
-        count_launch(r, kStCull, 2);
+        cull_blocks(r, fc, nullptr, st);
+        count_launch(r, kStCull);
     }
     r->timer.mark(kStPreprocess, st);
     PreprocessArgs pa{};
@@ -529,6 +553,7 @@ void render_pass(gps_renderer* r, const FrameConst& fc, int frame, bool first, c
     sp.clear_b = binned ? r->bins.get() : nullptr;
     sp.clear_b_words = binned ? nbins : 0u;
     sp.mask_iter = r->mask_iter.get();
+    sp.chunk_count = listed ? r->chunk_count.get() : nullptr;
     launch_splat(sp, r->splat_grid, 256, st);
     count_launch(r, kStSplat);
 }
@@ -742,6 +767,8 @@ gps_status gps_scene_tile(const gps_scene* src, int32_t copies, const float* off
         }
         launch_tile_nodes(src->block_nodes.get(), src->per_block, (uint32_t)n, pb, (uint32_t)copies, offs.get(), total,
                           s->block_nodes.get(), s->block_count, 0);
+        s->block_supers.reset(dev_alloc<float4>(((size_t)s->block_count + 31) / 32 * 2));
+        launch_super_bounds(s->block_nodes.get(), s->block_count, s->block_supers.get(), 0);
         GPS_CUDA(cudaGetLastError());
         GPS_CUDA(cudaDeviceSynchronize());
     } catch (const CudaError& e) {
@@ -885,6 +912,7 @@ gps_status create_renderer(gps_scene* scene, const gps_settings* settings, const
         GPS_CUDA(cudaMemset(r->counters.get(), 0, sizeof(PassCounters) * 2));
         const uint32_t bwords = (r->cap_blocks + 31) / 32;
         r->culled.reset(dev_alloc<uint32_t>(bwords + 1));
+        r->outside.reset(dev_alloc<uint32_t>(bwords + 1));
         r->chunk_list.reset(dev_alloc<uint32_t>(words + 1));
         r->chunk_count.reset(dev_alloc<uint32_t>(1));
         GPS_CUDA(cudaMemset(r->chunk_count.get(), 0, sizeof(uint32_t)));
@@ -957,7 +985,9 @@ gps_status render_frame_impl(gps_renderer* r, const gps_camera* cam, float* d_im
                         rgb_to_36bits(make_v3(r->s.background[0], r->s.background[1], r->s.background[2]));
     r->frame_launches = 0;
     r->timer.mark(kStClear, st);
-    launch_clear(r->buffer.get(), r->entries, bg, st);
+    const unsigned long long clear_value = bg;
+    if (fc.enable_hier && r->scene->block_count && r->n > 0) cull_blocks(r, fc, &clear_value, st);
+    else launch_clear(r->buffer.get(), r->entries, bg, st);
     count_launch(r, kStClear);
     if (r->n > 0) render_pass(r, fc, cam->frame, true, st);
     ResolveArgs ra{};
