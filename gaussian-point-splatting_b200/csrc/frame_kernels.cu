@@ -494,8 +494,9 @@ __global__ void __launch_bounds__(256) preprocess_kernel(PreprocessArgs a, Scene
 }
 
 // ---------------------------------------------------------------------------------
-// Scan over (survivor count, point count) pairs in three fully parallel launches: per-tile
-// totals, one block scanning the tile totals, a downsweep writing the compacted survivors
+// Scan over (survivor count, point count) pairs in up to three launches: per-tile totals (the
+// render path's preprocess accumulates them instead), where needed a block scanning the tile
+// totals and one scanning the bin cursors, a downsweep writing the compacted survivors
 // (replaces workload_distributor.cu:62-145: 3 blocking D2H copies, an exclusive scan, a
 // scatter and a P-long max-scan).  Tile word: [63:32] survivors, [31:0] points (mod 2^32 like
 // the reference's u32 offsets).  No block waits on another, so there is no spin at all.
@@ -585,39 +586,24 @@ __global__ void __launch_bounds__(kScanThreads) scan_reduce_kernel(ScanArgs a) {
 // each thread scans 4 consecutive words and a block scan plus a running carry joins them.
 constexpr int kTileScanThreads = 1024;
 constexpr int kTileScanPer = 4;
-static_assert(kBinSubs <= (uint32_t)kTileScanPer && (kBinSubs & (kBinSubs - 1u)) == 0u,
-              "a scan thread's words must hold whole bins");
 
 // One block: exclusive prefix of `count` packed (survivors << 32 | points) words in place,
 // through shared memory in coalesced rounds; returns the totals.
-// Scans words_g in the order of its logical index L; with sub_log2 > 0, word L is stored at
-// (L mod 2^sub_log2) * stride + L / 2^sub_log2 (the bin cursors' layout).
 __device__ __forceinline__ void scan_words_inplace(unsigned long long* words_g, uint32_t count, uint32_t& total_s,
-                                                   uint32_t& total_p, uint32_t* max_s = nullptr,
-                                                   uint32_t sub_log2 = 0, uint32_t stride = 0) {
-    auto at = [&](uint32_t L) -> uint32_t {
-        return sub_log2 ? (L & ((1u << sub_log2) - 1u)) * stride + (L >> sub_log2) : L;
-    };
+                                                   uint32_t& total_p) {
     __shared__ unsigned long long words[kTileScanThreads * kTileScanPer];
-    __shared__ uint32_t s_max;
     constexpr uint32_t kRound = kTileScanThreads * kTileScanPer;
-    uint32_t carry_s = 0, carry_p = 0, my_max = 0;
-    if (threadIdx.x == 0) s_max = 0;
+    uint32_t carry_s = 0, carry_p = 0;
     for (uint32_t r0 = 0; r0 < count; r0 += kRound) {
         for (uint32_t i = threadIdx.x; i < kRound; i += kTileScanThreads)
-            words[i] = r0 + i < count ? words_g[at(r0 + i)] : 0ull;
+            words[i] = r0 + i < count ? words_g[r0 + i] : 0ull;
         __syncthreads();
-        uint32_t s = 0, p = 0, group = 0;
+        uint32_t s = 0, p = 0;
 #pragma unroll
         for (int k = 0; k < kTileScanPer; ++k) {
             const unsigned long long v = words[threadIdx.x * kTileScanPer + k];
             s += (uint32_t)(v >> 32);
             p += (uint32_t)v;
-            group += (uint32_t)(v >> 32);
-            if ((((uint32_t)k + 1u) & ((1u << sub_log2) - 1u)) == 0u) {  // a whole bin's cursors
-                my_max = max(my_max, group);
-                group = 0;
-            }
         }
         uint32_t ex_s, ex_p, tot_s, tot_p;
         block_scan_pair<kTileScanThreads>(s, p, ex_s, ex_p, tot_s, tot_p);
@@ -631,186 +617,318 @@ __device__ __forceinline__ void scan_words_inplace(unsigned long long* words_g, 
             ex_p += (uint32_t)v;
         }
         __syncthreads();
-        for (uint32_t i = threadIdx.x; i < kRound && r0 + i < count; i += kTileScanThreads) words_g[at(r0 + i)] = words[i];
+        for (uint32_t i = threadIdx.x; i < kRound && r0 + i < count; i += kTileScanThreads) words_g[r0 + i] = words[i];
         carry_s += tot_s;
         carry_p += tot_p;
         __syncthreads();
     }
     total_s = carry_s;
     total_p = carry_p;
-    if (max_s) {  // the largest survivor count of one bin (2^sub_log2 consecutive words)
-        my_max = __reduce_max_sync(0xffffffffu, my_max);
-        if ((threadIdx.x & 31u) == 0u) atomicMax(&s_max, my_max);
-        __syncthreads();
-        *max_s = s_max;
-    }
 }
 
-// Pass 2: block 0 turns the tile totals into exclusive tile prefixes (in place) and writes the
-// pass counters (points mod 2^32, like the reference's u32 offsets); block 1, when the pass is
-// screen-binned, does the same for the bin histogram.
+// One block of the downsweep: the bin cursors (cursor k of bin b at word k * bin_count + b) become
+// exclusive prefixes in (b, k) order, in place; returns the largest bin's survivors.  2048 words at
+// a time, eight per thread in registers, every load coalesced: it takes less than the downsweep beside it, where a launch of its own took 13.6 us
+// (8160 words, 1080p) to 24 us (16320, 4K).
+template <int kSubLog2>
+__device__ __forceinline__ uint32_t scan_bins_inplace(unsigned long long* bins, uint32_t bin_count) {
+    constexpr uint32_t kSubs = 1u << kSubLog2, kRounds = 8u >> kSubLog2, kWarps = kScanThreads / 32u;
+    __shared__ uint32_t sum_s[kRounds][kWarps], sum_p[kRounds][kWarps], s_max;
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    unsigned long long v[kRounds][kSubs];
+    if (threadIdx.x == 0) s_max = 0;
+    uint32_t carry_s = 0, carry_p = 0, most = 0;
+    for (uint32_t b0 = 0; b0 < bin_count; b0 += kRounds * kScanThreads) {
+        uint32_t es[kRounds], ep[kRounds];
+#pragma unroll
+        for (uint32_t r = 0; r < kRounds; ++r)
+#pragma unroll
+            for (uint32_t k = 0; k < kSubs; ++k) {
+                const uint32_t b = b0 + r * kScanThreads + threadIdx.x;
+                v[r][k] = b < bin_count ? __ldcg(bins + (size_t)k * bin_count + b) : 0ull;
+            }
+#pragma unroll
+        for (uint32_t r = 0; r < kRounds; ++r) {
+            uint32_t s = 0, p = 0;
+#pragma unroll
+            for (uint32_t k = 0; k < kSubs; ++k) {
+                s += (uint32_t)(v[r][k] >> 32);
+                p += (uint32_t)v[r][k];
+            }
+            most = max(most, s);
+            es[r] = s;
+            ep[r] = p;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t vs = __shfl_up_sync(0xffffffffu, es[r], o), vp = __shfl_up_sync(0xffffffffu, ep[r], o);
+                if (lane >= (uint32_t)o) {
+                    es[r] += vs;
+                    ep[r] += vp;
+                }
+            }
+            if (lane == 31u) {
+                sum_s[r][warp] = es[r];
+                sum_p[r][warp] = ep[r];
+            }
+            es[r] -= s;
+            ep[r] -= p;
+        }
+        __syncthreads();
+#pragma unroll
+        for (uint32_t r = 0; r < kRounds; ++r) {
+            uint32_t ps = 0, pp = 0, all_s = 0, all_p = 0;
+#pragma unroll
+            for (uint32_t w = 0; w < kWarps; ++w) {
+                if (w == warp) {
+                    ps = all_s;
+                    pp = all_p;
+                }
+                all_s += sum_s[r][w];
+                all_p += sum_p[r][w];
+            }
+            const uint32_t b = b0 + r * kScanThreads + threadIdx.x;
+            uint32_t s = carry_s + ps + es[r], q = carry_p + pp + ep[r];
+#pragma unroll
+            for (uint32_t k = 0; k < kSubs; ++k) {
+                if (b < bin_count) bins[(size_t)k * bin_count + b] = ((unsigned long long)s << 32) | q;
+                s += (uint32_t)(v[r][k] >> 32);
+                q += (uint32_t)v[r][k];
+            }
+            carry_s += all_s;
+            carry_p += all_p;
+        }
+        __syncthreads();
+    }
+    most = __reduce_max_sync(0xffffffffu, most);
+    if (lane == 0u) atomicMax(&s_max, most);
+    __syncthreads();
+    return s_max;
+}
+
+__device__ __forceinline__ void write_counters(const ScanArgs& a, uint32_t survivors, uint32_t points) {
+    a.counters->survivors = survivors;
+    a.counters->total_points = points;
+    a.counters->points = points < a.max_points ? points : a.max_points;
+    a.counters->truncated = points > a.max_points ? 1u : 0u;
+    a.counters->scan_timeouts = 0u;
+    a.counters->loaded = a.loaded ? *a.loaded : 0u;
+    if (a.loaded) *a.loaded = 0u;  // the next pass's preprocess tallies from zero
+    a.counters->pad = 0u;
+    if (!a.bins) a.counters->crowded = 0u;
+}
+
+// Pass 2, for more tiles than kDirectTiles: one block turns the tile totals into exclusive tile
+// prefixes (in place) and writes the pass counters.
 __global__ void __launch_bounds__(kTileScanThreads) scan_tiles_kernel(ScanArgs a, uint32_t num_tiles) {
     previous_kernel_done();
     uint32_t carry_s, carry_p;
-    if (blockIdx.x == 1) {
-        uint32_t most = 0;
-        scan_words_inplace(a.bins, a.nbins, carry_s, carry_p, &most, (uint32_t)a.bin_sub_log2, a.bin_count);
-        // a bin crowded past bin_crowded survivors would serialise the downsweep on its
+    scan_words_inplace(a.tile_state, num_tiles, carry_s, carry_p);
+    if (threadIdx.x == 0) write_counters(a, carry_s, carry_p);
+}
+
+// Records survivor `rank` as the owner of every 256-point splat tile that starts inside its points
+// [first, first + count): one or none for most, but a Gaussian right in front of the camera owns
+// thousands, which its whole warp then writes.  All lanes call it; count 0: nothing to do.
+// (tiles starting at or past P are never walked, and the array holds max_points / 256 + 2)
+__device__ __forceinline__ void own_tiles(uint32_t* __restrict__ tile_first_rank, uint32_t first, uint32_t count,
+                                          uint32_t rank, uint32_t P) {
+    const uint64_t end = min((uint64_t)first + count, (uint64_t)P);
+    const uint32_t t0 = (uint32_t)(((uint64_t)first + 255u) >> 8), t1 = count ? (uint32_t)((end + 255u) >> 8) : 0u;
+    const uint32_t n = t1 > t0 ? t1 - t0 : 0u;
+    if (n <= 4u)
+        for (uint32_t i = 0; i < n; ++i) tile_first_rank[t0 + i] = rank;
+    const uint32_t lane = threadIdx.x & 31u;
+    for (unsigned big = __ballot_sync(0xffffffffu, n > 4u); big; big &= big - 1u) {
+        const int src = __ffs(big) - 1;
+        const uint32_t t = __shfl_sync(0xffffffffu, t0, src), m = __shfl_sync(0xffffffffu, n, src),
+                       r = __shfl_sync(0xffffffffu, rank, src);
+        for (uint32_t i = lane; i < m; i += 32u) tile_first_rank[t + i] = r;
+    }
+}
+
+// Pass 3, the downsweep: each tile of Gaussians writes its compacted survivors' ids and first
+// points and, where the splat walks the Gaussian order, the owners of its 256-point tiles (points
+// past P dropped as the reference drops them).  In a screen-binned pass the block before the first
+// tile scans the bin cursors.  The survivors of 4096 Gaussians are gathered in shared memory, then
+// taken one per thread: their writes are coalesced, and a thread whose own 16 Gaussians all
+// survive doesn't hold up its block (60k town at 320x180: frame 73.4 -> 64.5 us,
+// with the launch that scanned the tile totals gone).
+//
+// kDirect: the tile words are plain totals and every block adds up those before its own, which
+// takes less time than a launch that scans them (up to kDirectTiles words, 32 KB from L2).
+constexpr uint32_t kDirectTiles = 4096;
+
+template <int kScanRounds, bool kDirect, bool kBinned>
+__global__ void __launch_bounds__(kScanThreads, kBinned ? 4 : 5) scan_write_kernel(ScanArgs a, uint32_t tiles) {
+    previous_kernel_done();
+    __shared__ uint16_t list_g[kScanTileSmall];
+    __shared__ uint32_t list_p[kScanTileSmall + 1];
+    __shared__ uint32_t sums[4][kScanThreads / 32];
+    const uint32_t lane = threadIdx.x & 31u;
+    if (kBinned && blockIdx.x == 0u) {
+        const uint32_t most = a.bin_sub_log2 == 2   ? scan_bins_inplace<2>(a.bins, a.bin_count)
+                              : a.bin_sub_log2 == 1 ? scan_bins_inplace<1>(a.bins, a.bin_count)
+                                                    : scan_bins_inplace<0>(a.bins, a.bin_count);
+        // a bin crowded past bin_crowded survivors would serialise the binning on its
         // cursors: the pass is then walked in Gaussian order
         if (threadIdx.x == 0) a.counters->crowded = most > a.bin_crowded ? 1u : 0u;
         return;
     }
-    scan_words_inplace(a.tile_state, num_tiles, carry_s, carry_p);
-    if (threadIdx.x == 0) {
-        a.counters->survivors = carry_s;
-        a.counters->total_points = carry_p;
-        a.counters->points = carry_p < a.max_points ? carry_p : a.max_points;
-        a.counters->truncated = carry_p > a.max_points ? 1u : 0u;
-        a.counters->scan_timeouts = 0u;
-        a.counters->loaded = a.loaded ? *a.loaded : 0u;
-        if (a.loaded) *a.loaded = 0u;  // the next pass's preprocess tallies from zero
-        a.counters->pad = 0u;
-        if (!a.bins) a.counters->crowded = 0u;
+    const uint32_t tile = blockIdx.x - (kBinned ? 1u : 0u);
+    uint32_t r0, p0, P;
+    if (kDirect) {
+        // a tile without survivors has nothing to write (the first one writes the counters)
+        if (tile != 0u && (a.tile_state[tile] >> 32) == 0ull) return;
+        uint32_t s_pre = 0, p_pre = 0, s_all = 0, p_all = 0;
+        for (uint32_t i = threadIdx.x; i < tiles; i += kScanThreads) {
+            const unsigned long long v = a.tile_state[i];
+            s_all += (uint32_t)(v >> 32);
+            p_all += (uint32_t)v;
+            if (i < tile) {
+                s_pre += (uint32_t)(v >> 32);
+                p_pre += (uint32_t)v;
+            }
+        }
+        s_pre = __reduce_add_sync(0xffffffffu, s_pre);
+        p_pre = __reduce_add_sync(0xffffffffu, p_pre);
+        s_all = __reduce_add_sync(0xffffffffu, s_all);
+        p_all = __reduce_add_sync(0xffffffffu, p_all);
+        if (lane == 0u) {
+            sums[0][threadIdx.x >> 5] = s_pre;
+            sums[1][threadIdx.x >> 5] = p_pre;
+            sums[2][threadIdx.x >> 5] = s_all;
+            sums[3][threadIdx.x >> 5] = p_all;
+        }
+        __syncthreads();
+        r0 = p0 = s_all = p_all = 0u;
+#pragma unroll
+        for (int w = 0; w < kScanThreads / 32; ++w) {
+            r0 += sums[0][w];
+            p0 += sums[1][w];
+            s_all += sums[2][w];
+            p_all += sums[3][w];
+        }
+        if (tile == 0u && threadIdx.x == 0u) write_counters(a, s_all, p_all);
+        P = min(p_all, a.max_points);
+    } else {
+        const unsigned long long pre = a.tile_state[tile];
+        r0 = (uint32_t)(pre >> 32);
+        p0 = (uint32_t)pre;
+        // culled regions of the scene cost two loads, not a pass over their masks
+        // (256M town: scan 0.586 -> 0.548 ms/frame)
+        if (r0 == (tile + 1u < tiles ? (uint32_t)(a.tile_state[tile + 1u] >> 32) : a.counters->survivors)) return;
+        P = a.counters->points;
     }
-}
-
-// Pass 3: each tile rescans its Gaussians from its prefix and writes the compacted survivor
-// ids and first points.
-template <int kScanRounds>
-__global__ void __launch_bounds__(kScanThreads) scan_write_kernel(ScanArgs a) {
-    previous_kernel_done();
     const uint32_t* mask = a.mask;  // (a select, not a runtime index into the parameter array)
     if (a.mask_iter) mask = (*a.mask_iter & 1u) ? a.mask_pair[1] : a.mask_pair[0];
-    const uint32_t tile = blockIdx.x;
-    const uint32_t base = tile * (kScanThreads * kScanItems * kScanRounds) + threadIdx.x * (kScanItems * kScanRounds);
-    uint32_t surv = 0, pts = 0;
-#pragma unroll
     for (int q = 0; q < kScanRounds; ++q) {
-        uint32_t cnt[kScanItems];
-        surv += __popc(scan_load(a, mask, base + q * kScanItems, cnt));
+        const uint32_t base = (tile * kScanRounds + (uint32_t)q) * kScanTileSmall;
+        if (base >= a.n) break;
+        uint32_t tot_s, tot_p;
+        {
+            uint32_t cnt[kScanItems], pts = 0, at, pt;
+            uint32_t bits = scan_load(a, mask, base + threadIdx.x * kScanItems, cnt);
 #pragma unroll
-        for (int i = 0; i < kScanItems; ++i) pts += cnt[i];
-    }
-    uint32_t ex_s, ex_p, tot_s, tot_p;
-    block_scan_pair<kScanThreads>(surv, pts, ex_s, ex_p, tot_s, tot_p);
-    if (surv == 0u) return;
-    const unsigned long long pre = a.tile_state[tile];
-    uint32_t r = (uint32_t)(pre >> 32) + ex_s;
-    uint32_t pt = (uint32_t)pre + ex_p;
-    for (int q = 0; q < kScanRounds; ++q) {  // again, now writing (the counts come from L1/L2)
-        uint32_t cnt[kScanItems];
-        const uint32_t b = base + q * kScanItems;
-        const uint32_t bits = scan_load(a, mask, b, cnt);
+            for (int i = 0; i < kScanItems; ++i) pts += cnt[i];
+            block_scan_pair<kScanThreads>((uint32_t)__popc(bits), pts, at, pt, tot_s, tot_p);
 #pragma unroll
-        for (int i = 0; i < kScanItems; ++i) {
-            if ((bits >> i) & 1u) {
-                a.surv_gid[r] = b + i;
-                a.surv_start[r] = pt;
-                ++r;
-                pt += cnt[i];
-            }
-        }
-    }
-}
-
-// The render path's downsweep: as scan_write_kernel, and then for every survivor the splat's
-// work order.  Screen-binned (bins set, pass not truncated): the survivor takes its slot and
-// first walk position from one of its bin's cursors with one 64-bit atomic, so that slot and position
-// stay consistent and positions increase with the slot; otherwise the Gaussian order itself,
-// with the points past P dropped as the reference drops them.  Either way the survivor then
-// records itself as the owner of every 256-point splat tile that starts inside its points.
-// (tiles starting at or past P are never walked, and the array holds max_points / 256 + 2)
-__device__ __forceinline__ void own_tiles(uint32_t* __restrict__ tile_first_rank, uint64_t first, uint64_t count,
-                                          uint32_t rank, uint32_t P) {
-    const uint64_t end = min(first + count, (uint64_t)P);
-    for (uint64_t t = (first + 255u) >> 8; (t << 8) < end; ++t) tile_first_rank[t] = rank;
-}
-
-template <int kScanRounds>
-__global__ void __launch_bounds__(kScanThreads) scan_write_fused_kernel(ScanArgs a) {
-    previous_kernel_done();
-    const uint32_t tile = blockIdx.x;
-    // a tile without survivors (its exclusive survivor prefix equals the next tile's) has
-    // nothing to write: culled regions of the scene cost two loads, not a pass over their masks
-    // (256M town: scan 0.586 -> 0.548 ms/frame)
-    {
-        const uint32_t s0 = (uint32_t)(a.tile_state[tile] >> 32);
-        const uint32_t s1 = tile + 1u < gridDim.x ? (uint32_t)(a.tile_state[tile + 1u] >> 32) : a.counters->survivors;
-        if (s0 == s1) return;
-    }
-    const uint32_t* mask = a.mask;
-    if (a.mask_iter) mask = (*a.mask_iter & 1u) ? a.mask_pair[1] : a.mask_pair[0];
-    const uint32_t base = tile * (kScanThreads * kScanItems * kScanRounds) + threadIdx.x * (kScanItems * kScanRounds);
-    uint32_t surv = 0, pts = 0;
-#pragma unroll
-    for (int q = 0; q < kScanRounds; ++q) {
-        uint32_t cnt[kScanItems];
-        surv += __popc(scan_load(a, mask, base + q * kScanItems, cnt));
-#pragma unroll
-        for (int i = 0; i < kScanItems; ++i) pts += cnt[i];
-    }
-    uint32_t ex_s, ex_p, tot_s, tot_p;
-    block_scan_pair<kScanThreads>(surv, pts, ex_s, ex_p, tot_s, tot_p);
-    if (surv == 0u) return;
-    const uint32_t P = a.counters->points;
-    const bool binned = a.bins && a.counters->truncated == 0u && a.counters->crowded == 0u;
-    const unsigned long long pre = a.tile_state[tile];
-    uint32_t r = (uint32_t)(pre >> 32) + ex_s;
-    uint32_t pt = (uint32_t)pre + ex_p;
-    for (int q = 0; q < kScanRounds; ++q) {  // again, now writing (the counts come from L1/L2)
-        uint32_t cnt[kScanItems];
-        const uint32_t b = base + q * kScanItems;
-        const uint32_t bits = scan_load(a, mask, b, cnt);
-#pragma unroll
-        for (int i = 0; i < kScanItems; ++i) {
-            if ((bits >> i) & 1u) {
-                const uint32_t g = b + i;
-                a.surv_gid[r] = g;
-                a.surv_start[r] = pt;
-                if (binned) {
-                    const float2 pm = __ldg(reinterpret_cast<const float2*>(a.records + g));
-                    const uint32_t bin = screen_bin(pm.x, pm.y, a.up_width, a.up_height, a.bin_shift, a.bins_x, a.bins_y) +
-                                         ((g >> 5) & ((1u << a.bin_sub_log2) - 1u)) * a.bin_count;
-                    const unsigned long long old = atomicAdd(a.bins + bin, (1ull << 32) | cnt[i]);
-                    const uint32_t slot = (uint32_t)(old >> 32);
-                    a.sorted_gid[slot] = g;
-                    a.sorted_pstart[slot] = pt;
-                    a.sorted_qstart[slot] = (uint32_t)old;
-                    own_tiles(a.tile_first_rank, (uint32_t)old, cnt[i], slot, P);
-                } else if (pt < P) {
-                    own_tiles(a.tile_first_rank, pt, cnt[i], r, P);
+            for (int i = 0; i < kScanItems; ++i)
+                if ((bits >> i) & 1u) {
+                    list_g[at] = (uint16_t)(threadIdx.x * kScanItems + i);
+                    list_p[at++] = pt;
+                    pt += cnt[i];
                 }
-                ++r;
-                pt += cnt[i];
-            }
+            if (threadIdx.x == 0u) list_p[tot_s] = tot_p;
         }
+        __syncthreads();
+        for (uint32_t k0 = threadIdx.x & ~31u; k0 < tot_s; k0 += kScanThreads) {
+            const uint32_t k = k0 + lane;
+            const bool live = k < tot_s;
+            const uint32_t g = base + list_g[live ? k : 0u], pt = p0 + list_p[live ? k : 0u];
+            const uint32_t cnt = live ? list_p[k + 1u] - list_p[k] : 0u;
+            if (live) {
+                a.surv_gid[r0 + k] = g;
+                a.surv_start[r0 + k] = pt;
+            }
+            if (!kBinned) own_tiles(a.tile_first_rank, pt, pt < P ? cnt : 0u, r0 + k, P);
+        }
+        r0 += tot_s;
+        p0 += tot_p;
+        __syncthreads();
     }
 }
 
-// First survivor of every splat tile: tile t (points [t*tile_points, ...)) starts inside the
-// survivor with the largest rank whose first point is <= t*tile_points.  One thread per tile,
-// a binary search over the survivors' first points (monotone below 2^32 points per pass).  A
-// survivor can own thousands of tiles (a Gaussian right in front of the camera), so this is
-// done per tile rather than per survivor.
-__global__ void __launch_bounds__(256) tile_owner_kernel(const uint32_t* __restrict__ surv_start,
-                                                         uint32_t* __restrict__ tile_first_rank,
-                                                         const PassCounters* __restrict__ counters,
-                                                         uint32_t tile_points, uint32_t* __restrict__ mask_iter) {
+// The last step of a screen-binned pass: every survivor takes its slot and first walk position from
+// one of its bin's cursors, with one 64-bit atomic per distinct cursor among a warp's 32 survivors, so
+// that slot and position stay consistent and positions increase with the slot, and records itself
+// as the owner of the 256-point tiles that start inside its points.  A pass that cannot be binned
+// (truncated, or a crowded bin) records the owners of the Gaussian order here.
+//
+// The survivors are split evenly over the warps.  Inside the downsweep the chain record -> cursor
+// -> stores (a DRAM access and a contended atomic with a result, 2 us) ran once per survivor of
+// the fullest thread or tile: survivors are neighbours in the scene's order, so a few tiles hold
+// most of them.  Scan stage, both passes: 107 -> 53 us (4M town, 1080p), 120 -> 59 (1M, 4K), 255 -> 91
+// (33.6M, 2.6M survivors in pass 2).
+__global__ void __launch_bounds__(256) bin_survivors_kernel(ScanArgs a) {
     previous_kernel_done();
-    const uint32_t points = counters->points;
-    const uint32_t survivors = counters->survivors;
-    if (mask_iter && points > 0 && blockIdx.x == 0 && threadIdx.x == 0) *mask_iter += 1u;
-    if (points == 0 || survivors == 0) return;
-    const uint32_t tiles = (uint32_t)(((unsigned long long)points + tile_points - 1) / tile_points);
-    for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < tiles; t += gridDim.x * blockDim.x) {
-        const uint32_t target = t * tile_points;
-        uint32_t lo = 0, hi = survivors - 1;
-        while (lo < hi) {
-            const uint32_t mid = lo + ((hi - lo + 1) >> 1);
-            if (__ldg(surv_start + mid) <= target) lo = mid;
-            else hi = mid - 1;
+    const uint32_t survivors = a.counters->survivors, P = a.counters->points;
+    const bool binned = a.counters->truncated == 0u && a.counters->crowded == 0u;
+    const uint32_t lane = threadIdx.x & 31u;
+    for (uint32_t k0 = (blockIdx.x * blockDim.x + threadIdx.x) & ~31u; k0 < survivors; k0 += gridDim.x * blockDim.x) {
+        const uint32_t k = k0 + lane;
+        const bool live = k < survivors;
+        uint32_t g = 0, pt = 0, cnt = 0, bin = 0xffffffffu;
+        if (live) {
+            g = a.surv_gid[k];
+            pt = a.surv_start[k];
+            cnt = a.counts[g];
         }
-        tile_first_rank[t] = lo;
+        if (!binned) {
+            own_tiles(a.tile_first_rank, pt, pt < P ? cnt : 0u, k, P);
+            continue;
+        }
+        if (live) {
+            const float2 pm = __ldg(reinterpret_cast<const float2*>(a.records + g));
+            bin = screen_bin(pm.x, pm.y, a.up_width, a.up_height, a.bin_shift, a.bins_x, a.bins_y) +
+                  ((g >> 5) & ((1u << a.bin_sub_log2) - 1u)) * a.bin_count;
+        }
+        // the lanes of each distinct cursor: their leader, place and points before them
+        uint32_t leader = lane, rank = 0, before = 0;
+        unsigned long long add = 0;
+        for (unsigned todo = __ballot_sync(0xffffffffu, live); todo;) {
+            const int src = __ffs(todo) - 1;
+            const uint32_t key = __shfl_sync(0xffffffffu, bin, src);
+            const bool mine = bin == key;
+            const unsigned members = __ballot_sync(0xffffffffu, mine);
+            if (members == (1u << src)) {
+                if (mine) add = (1ull << 32) | cnt;
+            } else {
+                uint32_t sum = mine ? cnt : 0u;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const uint32_t v = __shfl_up_sync(0xffffffffu, sum, o);
+                    if (lane >= (uint32_t)o) sum += v;
+                }
+                const uint32_t total = __shfl_sync(0xffffffffu, sum, 31);
+                if (mine) {
+                    leader = (uint32_t)src;
+                    rank = (uint32_t)__popc(members & ((1u << lane) - 1u));
+                    before = sum - cnt;
+                    if (lane == (uint32_t)src) add = ((unsigned long long)__popc(members) << 32) | total;
+                }
+            }
+            todo &= ~members;
+        }
+        unsigned long long old = 0;
+        if (live && leader == lane) old = atomicAdd(a.bins + bin, add);
+        old = __shfl_sync(0xffffffffu, old, (int)leader);
+        const uint32_t slot = (uint32_t)(old >> 32) + rank, first = (uint32_t)old + before;
+        if (live) {
+            a.sorted_gid[slot] = g;
+            a.sorted_pstart[slot] = pt;
+            a.sorted_qstart[slot] = first;
+        }
+        own_tiles(a.tile_first_rank, first, cnt, slot, P);
     }
 }
 
@@ -2090,16 +2208,37 @@ uint32_t scan_tile_count(uint32_t n) { return (uint32_t)(((uint64_t)n + kScanTil
 
 int scan_tile_shift(uint32_t n) { return n >= kScanBigScene ? 14 : 12; }
 
-void launch_scan_fused(const ScanArgs& a, cudaStream_t stream) {
+template <bool kBinned>
+void launch_scan_write(const ScanArgs& a, uint32_t tiles, bool big, bool direct, cudaStream_t stream) {
+    const uint32_t grid = tiles + (kBinned ? 1u : 0u);
+    if (big && direct) launch_k(scan_write_kernel<kScanRoundsMax, true, kBinned>, grid, kScanThreads, 0, stream, a, tiles);
+    else if (big) launch_k(scan_write_kernel<kScanRoundsMax, false, kBinned>, grid, kScanThreads, 0, stream, a, tiles);
+    else if (direct) launch_k(scan_write_kernel<1, true, kBinned>, grid, kScanThreads, 0, stream, a, tiles);
+    else launch_k(scan_write_kernel<1, false, kBinned>, grid, kScanThreads, 0, stream, a, tiles);
+}
+
+// The scan of the tile totals that many tiles need, the downsweep, the binning; returns the launches.
+int launch_scan_passes(const ScanArgs& a, cudaStream_t stream) {
+    const bool big = a.n >= kScanBigScene;  // fewer, larger tiles
+    const uint32_t per = big ? kScanTile : kScanTileSmall;
+    const uint32_t tiles = (uint32_t)(((uint64_t)a.n + per - 1) / per);
+    const bool direct = tiles <= kDirectTiles;
+    if (!direct) launch_k(scan_tiles_kernel, 1, kTileScanThreads, 0, stream, a, tiles);
+    if (a.bins) launch_scan_write<true>(a, tiles, big, direct, stream);
+    else launch_scan_write<false>(a, tiles, big, direct, stream);
+    if (a.bins) {
+        const uint32_t blocks = (a.n + 255u) / 256u;
+        launch_k(bin_survivors_kernel, blocks < 148u * 8u ? blocks : 148u * 8u, 256, 0, stream, a);
+    }
+    return (direct ? 1 : 2) + (a.bins ? 1 : 0);
+}
+
+int launch_scan_fused(const ScanArgs& a, cudaStream_t stream) {
     if (a.n == 0) {
         cudaMemsetAsync(a.counters, 0, sizeof(PassCounters), stream);
-        return;
+        return 0;
     }
-    const bool big = a.n >= kScanBigScene;
-    const uint32_t tiles = (uint32_t)(((uint64_t)a.n + (big ? kScanTile : kScanTileSmall) - 1) / (big ? kScanTile : kScanTileSmall));
-    launch_k(scan_tiles_kernel, a.bins ? 2 : 1, kTileScanThreads, 0, stream, a, tiles);
-    if (big) launch_k(scan_write_fused_kernel<kScanRoundsMax>, tiles, kScanThreads, 0, stream, a);
-    else launch_k(scan_write_fused_kernel<1>, tiles, kScanThreads, 0, stream, a);
+    return launch_scan_passes(a, stream);
 }
 
 void launch_scan(const ScanArgs& a, uint32_t scan_tiles, cudaStream_t stream) {
@@ -2107,22 +2246,11 @@ void launch_scan(const ScanArgs& a, uint32_t scan_tiles, cudaStream_t stream) {
         cudaMemsetAsync(a.counters, 0, sizeof(PassCounters), stream);
         return;
     }
-    if (a.n >= kScanBigScene) {  // fewer, larger tiles: four rounds per thread
-        const uint32_t tiles = (uint32_t)(((uint64_t)a.n + kScanTile - 1) / kScanTile);
-        launch_k(scan_reduce_kernel<kScanRoundsMax>, tiles, kScanThreads, 0, stream, a);
-        launch_k(scan_tiles_kernel, 1, kTileScanThreads, 0, stream, a, tiles);
-        launch_k(scan_write_kernel<kScanRoundsMax>, tiles, kScanThreads, 0, stream, a);
-    } else {
-        const uint32_t tiles = (uint32_t)(((uint64_t)a.n + kScanTileSmall - 1) / kScanTileSmall);
-        launch_k(scan_reduce_kernel<1>, tiles, kScanThreads, 0, stream, a);
-        launch_k(scan_tiles_kernel, 1, kTileScanThreads, 0, stream, a, tiles);
-        launch_k(scan_write_kernel<1>, tiles, kScanThreads, 0, stream, a);
-    }
-    const uint64_t max_tiles = ((uint64_t)a.max_points + a.tile_points - 1) / a.tile_points;
-    const uint64_t want = (max_tiles + 255) / 256;
-    const int owner_grid = (int)(want < 1184 ? (want ? want : 1) : 1184);  // 148 SMs x 8
-    launch_k(tile_owner_kernel, owner_grid, 256, 0, stream, a.surv_start, a.tile_first_rank, a.counters, a.tile_points,
-             a.mask_iter);
+    if (a.n >= kScanBigScene)
+        launch_k(scan_reduce_kernel<kScanRoundsMax>, (unsigned)(((uint64_t)a.n + kScanTile - 1) / kScanTile), kScanThreads, 0, stream, a);
+    else
+        launch_k(scan_reduce_kernel<1>, (unsigned)(((uint64_t)a.n + kScanTileSmall - 1) / kScanTileSmall), kScanThreads, 0, stream, a);
+    launch_scan_passes(a, stream);
 }
 
 template <int K>

@@ -136,7 +136,7 @@ struct ScanArgs {
     uint32_t* surv_gid;          // [n] compacted Gaussian ids of survivors
     uint32_t* surv_start;        // [n] first point of each survivor
     uint32_t* tile_first_rank;   // [ceil(max_points / tile_points) + 1]
-    unsigned long long* tile_state;  // [scan tiles] tile totals, then tile prefixes
+    unsigned long long* tile_state;  // [scan tiles] tile totals (prefixes once scanned)
     PassCounters* counters;
     uint32_t* loaded;            // the preprocess's tally: moved into counters->loaded and reset
     // Screen binning in the downsweep (render path; null bins: Gaussian order): the bin scan runs
@@ -251,10 +251,10 @@ void launch_translate_origins(const float4* src, uint32_t count, float dx, float
 void launch_tile_nodes(const float4* src, uint32_t src_pb, uint32_t src_n, uint32_t pb, uint32_t copies,
                        const float2* offsets, uint64_t total, float4* dst, uint32_t nodes, cudaStream_t stream);
 void launch_scan(const ScanArgs& a, uint32_t scan_tiles, cudaStream_t stream);
-// The render path's scan over the tile totals the preprocess accumulated: the tile scan (and the
-// bin scan), then the downsweep that compacts the survivors, bins them and finds each splat
-// tile's first survivor.  Two launches.
-void launch_scan_fused(const ScanArgs& a, cudaStream_t stream);
+// The render path's scan over the tile totals the preprocess accumulated: the tile scan of a very
+// large scene, the downsweep that compacts the survivors and finds each splat tile's first
+// survivor, and the binning of a screen-binned pass.  Returns the launches, one to three.
+int launch_scan_fused(const ScanArgs& a, cudaStream_t stream);
 int scan_tile_shift(uint32_t n);
 uint32_t scan_tile_count(uint32_t n);
 constexpr uint32_t kScanTileGaussians = 16384;  // Gaussians per scan tile (counts are padded to it)

@@ -532,8 +532,7 @@ void render_pass(gps_renderer* r, const FrameConst& fc, int frame, bool first, c
     sa.sorted_gid = r->sorted_gid.get();
     sa.sorted_pstart = r->sorted_pstart.get();
     sa.sorted_qstart = r->sorted_qstart.get();
-    launch_scan_fused(sa, st);
-    count_launch(r, kStScan, 2);  // tile (and bin) scan, downsweep with binning and tile owners
+    count_launch(r, kStScan, (uint64_t)launch_scan_fused(sa, st));
     r->timer.mark(kStSplat, st);
     SplatArgs sp{};
     sp.fc = fc;
