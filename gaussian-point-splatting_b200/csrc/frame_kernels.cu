@@ -12,6 +12,7 @@
 // Every floating-point expression that decides a sample position, a count or a packed
 // value follows the reference's expression shape (see gps_math.cuh) so that the 64-bit
 // splat buffer is bit-identical to the reference kernels' for the same inputs.
+#include <algorithm>
 #include <type_traits>
 #include <cstdio>
 #include <mutex>
@@ -713,7 +714,7 @@ __device__ __forceinline__ void write_counters(const ScanArgs& a, uint32_t survi
     a.counters->scan_timeouts = 0u;
     a.counters->loaded = a.loaded ? *a.loaded : 0u;
     if (a.loaded) *a.loaded = 0u;  // the next pass's preprocess tallies from zero
-    a.counters->pad = 0u;
+    a.counters->work = 0u;
     if (!a.bins) a.counters->crowded = 0u;
 }
 
@@ -1114,7 +1115,8 @@ struct SampleConst {
     const uint32_t* spread;  // shared-memory Morton table (GPS_SPLAT_MORTON_LUT)
 };
 
-__device__ __forceinline__ bool draw_sample(u32x2& seed, const SampleConst& c, int p, uint32_t& slot) {
+// One sample: whether it is live, its splat-buffer tile and the Morton code of its place there.
+__device__ __forceinline__ bool draw_sample(u32x2& seed, const SampleConst& c, uint32_t& tile, uint32_t& code) {
     const vec2 u = pcg2d(seed);
     float a = c.inv_alpha * inv_dilog((1.0f - u.x) * c.li2_alpha);
     a = gclamp(a, 1.e-37f, 1.0f);
@@ -1133,12 +1135,11 @@ __device__ __forceinline__ bool draw_sample(u32x2& seed, const SampleConst& c, i
     const bool inside = ((uint32_t)x - (uint32_t)c.minx < c.span_x) & ((uint32_t)y - (uint32_t)c.miny < c.span_y);
     const float alpha = c.opacity * gaussian_value(c.conic, delta);
 #if GPS_SPLAT_MORTON_LUT
-    const uint32_t code = c.spread[x & (kTileSize - 1)] | (c.spread[y & (kTileSize - 1)] << 1);
+    code = c.spread[x & (kTileSize - 1)] | (c.spread[y & (kTileSize - 1)] << 1);
 #else
-    const uint32_t code = morton_encode((uint32_t)(x & (kTileSize - 1)), (uint32_t)(y & (kTileSize - 1)));
+    code = morton_encode((uint32_t)(x & (kTileSize - 1)), (uint32_t)(y & (kTileSize - 1)));
 #endif
-    const uint32_t tile = (uint32_t)((y >> kTileBits) * c.tiles_per_row + (x >> kTileBits));
-    slot = (tile * (uint32_t)(kTileSize * kTileSize) + code) * (uint32_t)c.passes + (uint32_t)p;
+    tile = (uint32_t)((y >> kTileBits) * c.tiles_per_row + (x >> kTileBits));
     return inside & !(alpha < 1.0f / 255.0f);
 }
 
@@ -1152,7 +1153,7 @@ __device__ __forceinline__ bool draw_sample(u32x2& seed, const SampleConst& c, i
 // scalar instruction would.  The transcendental and per-lane steps stay scalar.  Same values
 // as draw_sample, bit for bit.
 template <int K>
-__device__ __forceinline__ void draw_samples_paired(u32x2& seed, const SampleConst& c, int p, uint32_t* slot,
+__device__ __forceinline__ void draw_samples_paired(u32x2& seed, const SampleConst& c, uint32_t* tile, uint32_t* code,
                                                     bool* live) {
     static_assert(K % 2 == 0, "samples are drawn in pairs");
     const float2 one = make_float2(1.0f, 1.0f);
@@ -1220,22 +1221,17 @@ __device__ __forceinline__ void draw_samples_paired(u32x2& seed, const SampleCon
             const bool inside = ((uint32_t)xi - (uint32_t)c.minx < c.span_x) & ((uint32_t)yi - (uint32_t)c.miny < c.span_y);
             const float alpha = l ? al.y : al.x;
 #if GPS_SPLAT_MORTON_LUT
-            const uint32_t code = c.spread[xi & (kTileSize - 1)] | (c.spread[yi & (kTileSize - 1)] << 1);
+            code[j + l] = c.spread[xi & (kTileSize - 1)] | (c.spread[yi & (kTileSize - 1)] << 1);
 #else
-            const uint32_t code = morton_encode((uint32_t)(xi & (kTileSize - 1)), (uint32_t)(yi & (kTileSize - 1)));
+            code[j + l] = morton_encode((uint32_t)(xi & (kTileSize - 1)), (uint32_t)(yi & (kTileSize - 1)));
 #endif
-            const uint32_t tile = (uint32_t)((yi >> kTileBits) * c.tiles_per_row + (xi >> kTileBits));
-            slot[j + l] = (tile * (uint32_t)(kTileSize * kTileSize) + code) * (uint32_t)c.passes + (uint32_t)p;
+            tile[j + l] = (uint32_t)((yi >> kTileBits) * c.tiles_per_row + (xi >> kTileBits));
             live[j + l] = inside & !(alpha < 1.0f / 255.0f);
         }
     }
 }
 
-template <int K>
-__device__ __forceinline__ void splat_point_unbiased_k(uint32_t point, const SplatRecord& rec, const FrameConst& fc,
-                                                       int frame_seed, uint64_t* __restrict__ buffer,
-                                                       const uint32_t* spread) {
-    u32x2 seed = make_seed(point, (uint32_t)frame_seed);
+__device__ __forceinline__ SampleConst sample_const(const SplatRecord& rec, const FrameConst& fc, const uint32_t* spread) {
     SampleConst c;
     c.spread = spread;
     c.pixel_mean = make_v2(rec.a.x, rec.a.y);
@@ -1255,6 +1251,30 @@ __device__ __forceinline__ void splat_point_unbiased_k(uint32_t point, const Spl
     c.li2_alpha = dilog(c.opacity);
     c.passes = fc.num_passes;
     c.tiles_per_row = (fc.up_width + kTileSize - 1) >> kTileBits;
+    return c;
+}
+
+// The K samples of one spp pass.
+template <int K>
+__device__ __forceinline__ void draw_pass(u32x2& seed, const SampleConst& c, uint32_t* tile, uint32_t* code, bool* live) {
+    if constexpr (GPS_SPLAT_PAIRED && K % 2 == 0) {
+        draw_samples_paired<K>(seed, c, tile, code, live);
+    } else {
+#pragma unroll
+        for (int j = 0; j < K; ++j) live[j] = draw_sample(seed, c, tile[j], code[j]);
+    }
+}
+
+__device__ __forceinline__ uint32_t sample_slot(const SampleConst& c, uint32_t tile, uint32_t code, int p) {
+    return (tile * (uint32_t)(kTileSize * kTileSize) + code) * (uint32_t)c.passes + (uint32_t)p;
+}
+
+template <int K>
+__device__ __forceinline__ void splat_point_unbiased_k(uint32_t point, const SplatRecord& rec, const FrameConst& fc,
+                                                       int frame_seed, uint64_t* __restrict__ buffer,
+                                                       const uint32_t* spread) {
+    u32x2 seed = make_seed(point, (uint32_t)frame_seed);
+    const SampleConst c = sample_const(rec, fc, spread);
     const unsigned long long key = (unsigned long long)rec.d.z | ((unsigned long long)rec.d.w << 32);
     unsigned long long* buf = reinterpret_cast<unsigned long long*>(buffer);
 #if GPS_SPLAT_PRETEST && GPS_SPLAT_PIPELINE
@@ -1265,17 +1285,10 @@ __device__ __forceinline__ void splat_point_unbiased_k(uint32_t point, const Spl
     bool la[K], lb[K];
     unsigned long long va[K], vb[K];
     auto draw = [&](int p, uint32_t* sl, bool* lv, unsigned long long* vv) {
-#if GPS_SPLAT_PAIRED
-        if constexpr (K % 2 == 0) {
-            draw_samples_paired<K>(seed, c, p, sl, lv);
-        } else {
+        uint32_t tile[K], code[K];
+        draw_pass<K>(seed, c, tile, code, lv);
 #pragma unroll
-            for (int j = 0; j < K; ++j) lv[j] = draw_sample(seed, c, p, sl[j]);
-        }
-#else
-#pragma unroll
-        for (int j = 0; j < K; ++j) lv[j] = draw_sample(seed, c, p, sl[j]);
-#endif
+        for (int j = 0; j < K; ++j) sl[j] = sample_slot(c, tile[j], code[j], p);
 #pragma unroll
         for (int j = 0; j < K; ++j)
             vv[j] = lv[j] ? (GPS_SPLAT_PRETEST == 1 ? __ldca(buf + sl[j]) : __ldcg(buf + sl[j])) : 0ull;
@@ -1296,20 +1309,51 @@ __device__ __forceinline__ void splat_point_unbiased_k(uint32_t point, const Spl
     }
 #else
     for (int p = 0; p < c.passes; ++p) {
-        uint32_t slot[K];
+        uint32_t tile[K], code[K];
         bool live[K];
-#pragma unroll
-        for (int j = 0; j < K; ++j) live[j] = draw_sample(seed, c, p, slot[j]);
+        draw_pass<K>(seed, c, tile, code, live);
 #pragma unroll
         for (int j = 0; j < K; ++j) {
+            unsigned long long* at = buf + sample_slot(c, tile[j], code[j], p);
 #if GPS_SPLAT_PRETEST
-            if (live[j] && (GPS_SPLAT_PRETEST == 1 ? __ldca(buf + slot[j]) : __ldcg(buf + slot[j])) > key) atomicMin(buf + slot[j], key);
+            if (live[j] && (GPS_SPLAT_PRETEST == 1 ? __ldca(at) : __ldcg(at)) > key) atomicMin(at, key);
 #else
-            if (live[j]) atomicMin(buf + slot[j], key);
+            if (live[j]) atomicMin(at, key);
 #endif
         }
     }
 #endif
+}
+
+// The same samples with the pre-test in shared memory: `nearest` holds the high words (the depth and
+// the top colour bits) of one splat-buffer tile's smallest keys that this block knows of, a plane
+// of kNearPlane words per spp pass.  A sample there whose high word is larger can't change its
+// slot; one whose word is equal or smaller goes on to the buffer.  Samples of other tiles go to
+// the buffer untested.
+constexpr uint32_t kNearPlane = kTileSize * kTileSize + 8;  // (8: planes p and p + 2 on other banks)
+
+template <int K>
+__device__ __forceinline__ void splat_point_in_tile(uint32_t point, const SplatRecord& rec, const FrameConst& fc,
+                                                    int frame_seed, uint64_t* __restrict__ buffer, const uint32_t* spread,
+                                                    uint32_t* nearest, uint32_t my_tile) {
+    u32x2 seed = make_seed(point, (uint32_t)frame_seed);
+    const SampleConst c = sample_const(rec, fc, spread);
+    const uint32_t key_high = rec.d.w;
+    const unsigned long long key = (unsigned long long)rec.d.z | ((unsigned long long)rec.d.w << 32);
+    unsigned long long* buf = reinterpret_cast<unsigned long long*>(buffer);
+    for (int p = 0; p < c.passes; ++p, nearest += kNearPlane) {
+        uint32_t tile[K], code[K], seen[K];
+        bool live[K];
+        draw_pass<K>(seed, c, tile, code, live);
+#pragma unroll
+        for (int j = 0; j < K; ++j) seen[j] = live[j] && tile[j] == my_tile ? nearest[code[j]] : 0xFFFFFFFFu;
+#pragma unroll
+        for (int j = 0; j < K; ++j)
+            if (live[j] && key_high <= seen[j]) {
+                atomicMin(buf + sample_slot(c, tile[j], code[j], p), key);
+                if (tile[j] == my_tile) atomicMin(nearest + code[j], key_high);
+            }
+    }
 }
 
 // Points per thread between two block barriers: a block takes kSplatRounds consecutive 256-point
@@ -1324,6 +1368,102 @@ __device__ __forceinline__ void splat_point_unbiased_k(uint32_t point, const Spl
 constexpr int kSplatRounds = GPS_SPLAT_ROUNDS;
 constexpr int kSplatWindow = kSplatTile * kSplatRounds;
 
+// The order in which a pass's points are walked.
+struct PointOrder {
+    uint32_t points, survivors;
+    bool binned;
+    const uint32_t *gids, *first_q, *point_base;
+};
+
+__device__ __forceinline__ PointOrder point_order(const SplatArgs& a) {
+    PointOrder o;
+    o.points = a.counters->points;
+    o.survivors = a.counters->survivors;
+    // the pass's work order: screen bins unless the scan had to truncate the pass or a bin was
+    // too crowded to sort into
+    o.binned = a.sorted_gid && a.counters->truncated == 0u && a.counters->crowded == 0u;
+    o.gids = o.binned ? a.sorted_gid : a.surv_gid;
+    o.first_q = o.binned ? a.sorted_qstart : a.surv_start;
+    o.point_base = o.binned ? a.sorted_pstart : nullptr;
+    return o;
+}
+
+// What the next pass's kernels accumulate into is cleared here; nothing in the splat reads it.
+__device__ __forceinline__ void clear_for_next_pass(const SplatArgs& a, uint32_t points) {
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < a.clear_a_words; i += gridDim.x * blockDim.x)
+        a.clear_a[i] = 0ull;
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < a.clear_b_words; i += gridDim.x * blockDim.x)
+        a.clear_b[i] = 0ull;
+    if (a.mask_iter && points > 0u && blockIdx.x == 0 && threadIdx.x == 0) *a.mask_iter += 1u;
+    if (a.chunk_count && blockIdx.x == 0 && threadIdx.x == 0) *a.chunk_count = 0u;
+}
+
+// Group `group` of kThreads * kRounds consecutive walk positions: the starts of the survivors that
+// may own them (the first position's owner and as many as there are positions) go to `starts`,
+// then every thread takes kRounds positions and calls point(reference point index, record).
+template <uint32_t kThreads, uint32_t kRounds, class Point>
+__device__ __forceinline__ void splat_group(const SplatArgs& a, const PointOrder& o, uint32_t group, uint32_t* starts,
+                                            Point&& point) {
+    constexpr uint32_t group_points = kThreads * kRounds;
+    static_assert(group_points % 256u == 0u && 256u % 32u == 0u, "groups are whole 256-point tiles");
+    const uint32_t r0 = a.tile_first_rank[group * (group_points / 256u)];
+#pragma unroll
+    for (uint32_t q = 0; q < kRounds; ++q) {
+        const uint32_t k = q * kThreads + threadIdx.x, r = r0 + k;
+        starts[k] = (r0 < o.survivors && r < o.survivors) ? o.first_q[r] : 0xFFFFFFFFu;
+    }
+    __syncthreads();
+    for (uint32_t q = 0; q < kRounds; ++q) {
+        const uint32_t at = group * group_points + q * kThreads + threadIdx.x;
+        if (at < o.points && starts[0] <= at) {
+            // the position's owner is that of its 256-point tile's first point, of the next tile's,
+            // or one between: the search starts from that range (splat 1.562 -> 1.545 ms/frame on
+            // the 16M orbit)
+            const uint32_t t = at >> 8;
+            int hi = (int)group_points - 1;
+            int lo = min((int)(__ldg(&a.tile_first_rank[t]) - r0), hi);
+            if ((unsigned long long)(t + 1u) * 256u < o.points)
+                hi = max(lo, min((int)(__ldg(&a.tile_first_rank[t + 1u]) - r0), hi));
+            while (lo < hi) {  // largest k with starts[k] <= at
+                const int mid = (lo + hi + 1) >> 1;
+                if (starts[mid] <= at) lo = mid;
+                else hi = mid - 1;
+            }
+            // the reference's point index (the seed): the walk position itself in Gaussian
+            // order, the survivor's first point plus the offset in screen-bin order
+            const uint32_t p = o.point_base ? __ldg(&o.point_base[r0 + lo]) + (at - starts[lo]) : at;
+            const uint32_t g = __ldg(&o.gids[r0 + lo]);
+            if (g < a.n) {  // always true unless the scan gave up (device_timeouts)
+                const float4* rp = reinterpret_cast<const float4*>(a.records + g);
+                SplatRecord rec;
+                rec.a = __ldg(rp + 0);
+                rec.b = __ldg(rp + 1);
+                rec.c = __ldg(rp + 2);
+                rec.d = __ldg(reinterpret_cast<const uint4*>(rp + 3));
+                point(p, rec);
+            }
+        }
+    }
+    __syncthreads();
+}
+
+// Groups of kRounds positions per thread while there are at least two per block; a small pass keeps
+// one position per thread and barrier so that its points still spread over every block.
+template <uint32_t kThreads, uint32_t kRounds, class Point>
+__device__ __forceinline__ void splat_walk(const SplatArgs& a, const PointOrder& o, uint32_t* starts, Point&& point) {
+    auto walk = [&](auto rounds) {
+        constexpr uint32_t r = decltype(rounds)::value;
+        for (uint32_t group = blockIdx.x; (unsigned long long)group * (kThreads * r) < o.points; group += gridDim.x)
+            splat_group<kThreads, r>(a, o, group, starts, point);
+    };
+    if ((unsigned long long)o.points >= 2ull * gridDim.x * (kThreads * kRounds)) walk(std::integral_constant<uint32_t, kRounds>{});
+    else walk(std::integral_constant<uint32_t, 1u>{});
+}
+
+__device__ __forceinline__ void fill_spread(uint32_t* spread) {
+    if (GPS_SPLAT_MORTON_LUT && threadIdx.x < kTileSize) spread[threadIdx.x] = morton_spread(threadIdx.x);
+}
+
 // K > 0: unbiased splatting with K points per thread per pass; K = 0: any other setting.
 template <int K>
 #ifndef GPS_SPLAT_MIN_BLOCKS
@@ -1334,85 +1474,82 @@ __global__ void __launch_bounds__(kSplatTile, kSplatRounds > 1 ? (K >= 8 ? 2 : G
     previous_kernel_done();
     __shared__ uint32_t s_start[kSplatWindow];
     __shared__ uint32_t s_spread[kTileSize];
-    if (GPS_SPLAT_MORTON_LUT && threadIdx.x < kTileSize) s_spread[threadIdx.x] = morton_spread(threadIdx.x);
-    const uint32_t points = a.counters->points;
-    const uint32_t survivors = a.counters->survivors;
-    // the pass's work order: screen bins unless the scan had to truncate the pass or a bin was
-    // too crowded to sort into
-    const bool binned = a.sorted_gid && a.counters->truncated == 0u && a.counters->crowded == 0u;
-    const uint32_t* __restrict__ gids = binned ? a.sorted_gid : a.surv_gid;
-    const uint32_t* __restrict__ first_q = binned ? a.sorted_qstart : a.surv_start;
-    const uint32_t* __restrict__ point_base = binned ? a.sorted_pstart : nullptr;
-    // the preprocess of the next pass accumulates into these; nothing here reads them
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < a.clear_a_words; i += gridDim.x * blockDim.x)
-        a.clear_a[i] = 0ull;
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < a.clear_b_words; i += gridDim.x * blockDim.x)
-        a.clear_b[i] = 0ull;
-    if (a.mask_iter && points > 0u && blockIdx.x == 0 && threadIdx.x == 0) *a.mask_iter += 1u;
-    if (a.chunk_count && blockIdx.x == 0 && threadIdx.x == 0) *a.chunk_count = 0u;
-    // splats walk position q0 + threadIdx.x of a tile whose survivor starts are in `starts`
-    auto splat_tile_point = [&](uint32_t q0, uint32_t r0, const uint32_t* starts, int window, int lo0, int hi0) {
-        const uint32_t q = q0 + threadIdx.x;
-        if (q < points && starts[0] <= q) {
-            int lo = lo0, hi = hi0;  // largest k with starts[k] <= q
-            while (lo < hi) {
-                int mid = (lo + hi + 1) >> 1;
-                if (starts[mid] <= q) lo = mid;
-                else hi = mid - 1;
-            }
-            // the reference's point index (the seed): the walk position itself in Gaussian
-            // order, the survivor's first point plus the offset in screen-bin order
-            const uint32_t p = point_base ? __ldg(&point_base[r0 + lo]) + (q - starts[lo]) : q;
-            const uint32_t g = __ldg(&gids[r0 + lo]);
-            if (g < a.n) {  // always true unless the scan gave up (device_timeouts)
-                const float4* rp = reinterpret_cast<const float4*>(a.records + g);
-                SplatRecord rec;
-                rec.a = __ldg(rp + 0);
-                rec.b = __ldg(rp + 1);
-                rec.c = __ldg(rp + 2);
-                rec.d = __ldg(reinterpret_cast<const uint4*>(rp + 3));
-                if constexpr (K > 0) {
-                    splat_point_unbiased_k<K>(p, rec, a.fc, a.frame_seed, a.buffer, s_spread);
-                } else {
-                    if (a.fc.use_unbiased) splat_point_unbiased(p, rec, a.fc, a.frame_seed, a.buffer);
-                    else splat_point_biased(p, rec, a.fc, a.frame_seed, a.buffer);
-                }
-            }
+    fill_spread(s_spread);
+    const PointOrder o = point_order(a);
+    clear_for_next_pass(a, o.points);
+    splat_walk<kSplatTile, kSplatRounds>(a, o, s_start, [&](uint32_t p, const SplatRecord& rec) {
+        if constexpr (K > 0) {
+            splat_point_unbiased_k<K>(p, rec, a.fc, a.frame_seed, a.buffer, s_spread);
+        } else {
+            if (a.fc.use_unbiased) splat_point_unbiased(p, rec, a.fc, a.frame_seed, a.buffer);
+            else splat_point_biased(p, rec, a.fc, a.frame_seed, a.buffer);
         }
-    };
-    auto start_of = [&](uint32_t r0, uint32_t k) {
-        const uint32_t r = r0 + k;
-        return (r0 < survivors && r < survivors) ? first_q[r] : 0xFFFFFFFFu;
-    };
-    // grouped tiles only while there are at least two groups per block; a small pass keeps one
-    // tile per barrier so that its points still spread over every block
-    auto walk = [&](auto rounds_c) {
-        constexpr uint32_t rounds = decltype(rounds_c)::value;
-        constexpr uint32_t group_points = kSplatTile * rounds;
-        for (uint32_t group = blockIdx.x; (unsigned long long)group * group_points < points; group += gridDim.x) {
-            const uint32_t r0 = a.tile_first_rank[group * rounds];
-#pragma unroll
-            for (uint32_t q = 0; q < rounds; ++q)
-                s_start[q * kSplatTile + threadIdx.x] = start_of(r0, q * kSplatTile + threadIdx.x);
-            __syncthreads();
-            for (uint32_t q = 0; q < rounds; ++q) {
-                // the tile's points belong to the owners of its first point and of the next
-                // tile's first point, and to those between: the owner search starts from that
-                // range (splat 1.562 -> 1.545 ms/frame on the 16M orbit)
-                const uint32_t t = group * rounds + q;
-                int hi0 = (int)group_points - 1;
-                const int lo0 = min((int)(__ldg(&a.tile_first_rank[t]) - r0), hi0);
-                if ((unsigned long long)(t + 1) * kSplatTile < points)
-                    hi0 = max(lo0, min((int)(__ldg(&a.tile_first_rank[t + 1]) - r0), hi0));
-                splat_tile_point(group * group_points + q * kSplatTile, r0, s_start, (int)group_points, lo0, hi0);
+    });
+}
+
+// A frame's first pass in screen-bin order.  Its groups lie in one bin (a splat-buffer tile) each,
+// but for the small bins and a bin's last group, so the block keeps that tile's nearest high words
+// in shared memory, 16 KB per spp pass, and tests its samples there.
+//
+// Random 8-byte accesses bound this pass before its arithmetic did: every pre-test load and every
+// atomic is an L1 set access of its own (4M town at 1080p, 4 spp: 106M of them for 68M samples, 72%
+// of the cycles, warps waiting 8.7 cycles per issue for those loads, issue 50%), and an L1 line
+// holds what the slot was when the line came in.  Tested in shared memory: 60M set accesses, issue
+// 67%, and the pass 503 -> 373 us (33.6M town 232 -> 214, 1M town at 4K and 2 spp 448 -> 421).
+//
+// The buffer starts cleared, so a block starts a tile empty; what other blocks put there it does not
+// know, which costs some atomics, and reading it (or giving every bin whole groups) cost more.
+// The second pass would have to read its tiles, 128 KB each at 4 spp: 160 -> 209 us on the 4M town, so
+// it keeps the test in L1.
+//
+// A block takes a.work's next run of consecutive groups, so that a tile serves several groups.  Passes
+// with less than two groups per block take the other walk, which spreads them over more blocks.
+constexpr uint32_t kBinnedThreads = 256, kBinnedRounds = 4, kBinnedGroup = kBinnedThreads * kBinnedRounds;
+constexpr int kBinnedBlocks = 4;  // per SM, as far as their shared memory allows
+
+template <int K>
+__global__ void __launch_bounds__(kBinnedThreads, kBinnedBlocks) splat_binned_kernel(SplatArgs a) {
+    previous_kernel_done();
+    __shared__ uint32_t s_start[kBinnedGroup];
+    __shared__ uint32_t s_spread[kTileSize];
+    __shared__ uint32_t s_next;
+    extern __shared__ __align__(16) uint32_t s_nearest[];  // num_passes planes of kNearPlane words
+    fill_spread(s_spread);
+    const PointOrder o = point_order(a);
+    clear_for_next_pass(a, o.points);
+    if (!o.binned || (unsigned long long)o.points < 2ull * gridDim.x * kBinnedGroup) {
+        splat_walk<kBinnedThreads, kBinnedRounds>(a, o, s_start, [&](uint32_t p, const SplatRecord& rec) {
+            splat_point_unbiased_k<K>(p, rec, a.fc, a.frame_seed, a.buffer, s_spread);
+        });
+        return;
+    }
+    const uint32_t quads = (uint32_t)a.fc.num_passes * (kNearPlane / 4u);
+    const uint32_t tiles_per_row = (uint32_t)(a.fc.up_width + kTileSize - 1) >> kTileBits;
+    const uint32_t groups = (o.points + kBinnedGroup - 1u) / kBinnedGroup;
+    const uint32_t run = min(max(groups / (gridDim.x * 8u), 1u), 8u);
+    uint32_t my_tile = 0xFFFFFFFFu;
+    for (;;) {
+        if (threadIdx.x == 0u) s_next = atomicAdd(a.work, run);
+        __syncthreads();
+        const uint32_t first = s_next;
+        if (first >= groups) break;
+        for (uint32_t group = first; group < min(first + run, groups); ++group) {
+            // the tile of the group's middle point
+            const uint32_t mid = min(group * kBinnedGroup + kBinnedGroup / 2u, o.points - 1u);
+            const uint32_t g = __ldg(&o.gids[__ldg(&a.tile_first_rank[mid >> 8])]);
+            const float2 pm = __ldg(reinterpret_cast<const float2*>(a.records + g));
+            const uint32_t tile = screen_bin(pm.x, pm.y, a.fc.up_width, a.fc.up_height, kTileBits, (int)tiles_per_row,
+                                             (a.fc.up_height + kTileSize - 1) >> kTileBits);
+            if (tile != my_tile) {  // (the last group's samples are done: splat_group ends in a barrier)
+                my_tile = tile;
+                for (uint32_t i = threadIdx.x; i < quads; i += kBinnedThreads)
+                    reinterpret_cast<uint4*>(s_nearest)[i] = make_uint4(0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu);
             }
-            __syncthreads();
+            splat_group<kBinnedThreads, kBinnedRounds>(a, o, group, s_start, [&](uint32_t p, const SplatRecord& rec) {
+                splat_point_in_tile<K>(p, rec, a.fc, a.frame_seed, a.buffer, s_spread, s_nearest, my_tile);
+            });
         }
-    };
-    if ((unsigned long long)points >= 2ull * gridDim.x * kSplatWindow)
-        walk(std::integral_constant<uint32_t, (uint32_t)kSplatRounds>{});
-    else
-        walk(std::integral_constant<uint32_t, 1u>{});
+    }
 }
 
 // ---------------------------------------------------------------------------------
@@ -2273,9 +2410,35 @@ int splat_grid_size(int block) {
     return g_num_sms * splat_blocks_per_sm<0>();
 }
 
+// The shared-memory pre-test needs bins of one tile (up to 8192 x 8192 pixels), a buffer that starts
+// cleared, and planes that leave room for at least two blocks in an SM's 227 KB: up to 6 samples
+// per pixel.
+constexpr int kBinnedMaxPasses = 6;
+constexpr int kSmemPerSm = 227 * 1024;
+
+template <int K>
+bool launch_splat_binned(const SplatArgs& a, cudaStream_t stream) {
+    const int smem = a.fc.num_passes * (int)kNearPlane * 4;
+    // (the limit is the device context's, so it is not remembered here; one value for all callers)
+    if (cudaFuncSetAttribute(splat_binned_kernel<K>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             kBinnedMaxPasses * (int)kNearPlane * 4) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    const int blocks = std::min(kBinnedBlocks, kSmemPerSm / (smem + (int)(kBinnedGroup + kTileSize + 4u) * 4 + 1024));
+    launch_k(splat_binned_kernel<K>, g_num_sms * blocks, kBinnedThreads, (size_t)smem, stream, a);
+    return true;
+}
+
 void launch_splat(const SplatArgs& a, int grid, int block, cudaStream_t stream) {
     (void)block;
     if (g_num_sms == 0) splat_grid_size(kSplatTile);
+    if (a.sorted_gid && a.bin_is_tile && a.fresh && a.fc.use_unbiased && a.fc.num_passes <= kBinnedMaxPasses) {
+        const int k = a.fc.k_points;
+        if (k == 4 ? launch_splat_binned<4>(a, stream) : k == 2 ? launch_splat_binned<2>(a, stream)
+            : k == 1 ? launch_splat_binned<1>(a, stream) : false)
+            return;
+    }
     // a persistent grid: as many blocks as fit on the device at once
     if (a.fc.use_unbiased && a.fc.k_points == 4) {
         launch_k(splat_kernel<4>, g_num_sms * splat_blocks_per_sm<4>(), kSplatTile, 0, stream, a);

@@ -53,7 +53,7 @@ struct PassCounters {
                              // block cull and pass 2's previous-mask test); 0 without a tally
     uint32_t crowded;        // 1 if a screen bin held more than kBinCrowded survivors: the
                              // pass is walked in Gaussian order
-    uint32_t pad;
+    uint32_t work;           // groups of a screen-binned pass that splat blocks have taken
 };
 
 struct FrameConst {
@@ -175,6 +175,9 @@ struct SplatArgs {
     uint32_t clear_b_words;
     uint32_t* mask_iter;             // advanced after a pass with points (null: not here)
     uint32_t* chunk_count;           // the cull's list length, zeroed for the next pass (null: no list)
+    uint32_t* work;                  // next group of a screen-binned pass; zero before the splat
+    int bin_is_tile;                 // a screen bin is one tile of the splat buffer
+    int fresh;                       // the buffer starts cleared (a frame's first pass)
 };
 
 // Screen bins: the splat walks a pass's survivors grouped by the 64x64 splat-buffer tile (or

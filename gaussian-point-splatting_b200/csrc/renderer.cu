@@ -552,6 +552,9 @@ void render_pass(gps_renderer* r, const FrameConst& fc, int frame, bool first, c
     sp.clear_b = binned ? r->bins.get() : nullptr;
     sp.clear_b_words = binned ? nbins : 0u;
     sp.mask_iter = r->mask_iter.get();
+    sp.work = &pc->work;
+    sp.bin_is_tile = bin_shift == kTileBits ? 1 : 0;
+    sp.fresh = first ? 1 : 0;
     sp.chunk_count = listed ? r->chunk_count.get() : nullptr;
     launch_splat(sp, r->splat_grid, 256, st);
     count_launch(r, kStSplat);
