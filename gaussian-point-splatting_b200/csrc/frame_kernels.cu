@@ -1112,10 +1112,20 @@ struct SampleConst {
     int minx, miny, maxx, maxy;
     uint32_t span_x, span_y;  // max(maxx - minx, 0), max(maxy - miny, 0)
     int tiles_per_row, passes;
+    uint32_t tile_bias;      // added to every tile index below, and taken off again with the slot
+    uint32_t slot_bias;
     const uint32_t* spread;  // shared-memory Morton table (GPS_SPLAT_MORTON_LUT)
 };
 
-// One sample: whether it is live, its splat-buffer tile and the Morton code of its place there.
+// Adding 1.5 * 2^23 with rounding down leaves floor(v) in the low mantissa bits for |v| < 2^22:
+// floor and conversion in one addition that pairs.  Outside that range the bits, less
+// kFloorBits, are at least 200,000 as an unsigned number, so that no bounds test passes (checked
+// over all floats).
+constexpr float kFloorMagic = 12582912.0f;
+constexpr uint32_t kFloorBits = 0x4B400000u;
+
+// One sample: whether it is live, its splat-buffer tile (plus c.tile_bias) and the Morton code of its
+// place there.
 __device__ __forceinline__ bool draw_sample(u32x2& seed, const SampleConst& c, uint32_t& tile, uint32_t& code) {
     const vec2 u = pcg2d(seed);
     float a = c.inv_alpha * inv_dilog((1.0f - u.x) * c.li2_alpha);
@@ -1139,95 +1149,87 @@ __device__ __forceinline__ bool draw_sample(u32x2& seed, const SampleConst& c, u
 #else
     code = morton_encode((uint32_t)(x & (kTileSize - 1)), (uint32_t)(y & (kTileSize - 1)));
 #endif
-    tile = (uint32_t)((y >> kTileBits) * c.tiles_per_row + (x >> kTileBits));
+    tile = (uint32_t)((y >> kTileBits) * c.tiles_per_row + (x >> kTileBits)) + c.tile_bias;
     return inside & !(alpha < 1.0f / 255.0f);
 }
 
-#ifndef GPS_SPLAT_PAIRED
-#define GPS_SPLAT_PAIRED 1  // splat 1.547 -> 1.461 ms/frame (16M)
-#endif
-// The K samples of a pass drawn two at a time: the random words come off the seed in stream
-// order, and the floating-point steps two samples share (the opacity-corrected inverse dilog
-// polynomial, the Box-Muller products, the pixel position and its offset, the Gaussian weight)
-// run as sm_100 paired FP32 instructions (FFMA2 / FMUL2 / FADD2), each lane rounded as the
-// scalar instruction would.  The transcendental and per-lane steps stay scalar.  Same values
-// as draw_sample, bit for bit.
-template <int K>
-__device__ __forceinline__ void draw_samples_paired(u32x2& seed, const SampleConst& c, uint32_t* tile, uint32_t* code,
-                                                    bool* live) {
-    static_assert(K % 2 == 0, "samples are drawn in pairs");
-    const float2 one = make_float2(1.0f, 1.0f);
-    const float2 li2 = make_float2(c.li2_alpha, c.li2_alpha);
-    const float2 inva = make_float2(c.inv_alpha, c.inv_alpha);
-    const float2 c0 = make_float2(c.c0, c.c0), c1 = make_float2(c.c1, c.c1), c2 = make_float2(c.c2, c.c2);
-    const float2 pmx = make_float2(c.pixel_mean.x, c.pixel_mean.x), pmy = make_float2(c.pixel_mean.y, c.pixel_mean.y);
+// Two samples drawn together: the random words come off the seed in stream order, and the
+// floating-point steps the two share (the opacity-corrected inverse dilog polynomial, the square
+// root, the Box-Muller products, the pixel position and its offset, the Gaussian weight) run as
+// sm_100 paired FP32 instructions (FFMA2 / FMUL2 / FADD2), each lane rounded as the scalar
+// instruction would.  The transcendental and per-lane steps stay scalar.  Same values as
+// draw_sample, bit for bit, where wide_sample(c) is false:
+//   - the square root is rsqrt with one correction step (Markstein's, in the residual x - g^2): the
+//     correctly rounded root for every float from 1e-30 to 2^10 (checked against __fsqrt_rn), and x
+//     here is 0 or between 1e-7 and 171; a root of zero comes out as -0, which changes no sum below
+//   - dividing by kLi2Max is what the compiler makes of it, a product with the reciprocal (equal
+//     for all operands up to 2)
+//   - the root, the offset and the mixed conic term are kept with the opposite sign where that
+//     saves a negation: products of two of them, and sums, only change sign with it
+// With the pairing alone the draw took 117 instructions a sample, floor and conversion on the
+// conversion unit and the root through the compiler's sequence; now 104 (4M town, both passes: 385 ->
+// 340 million warp instructions, pass 2 160 -> 152 us, frame 846 -> 827; 33.6M town 1180 -> 1143). The
+// first pass is by now bound by its atomics: 61M random ones in 368 us, of the 185 G/s that L2 does.
+__device__ __forceinline__ float2 both(float v) { return make_float2(v, v); }
+
+__device__ __forceinline__ void draw_pair(u32x2& seed, const SampleConst& c, uint32_t* tile, uint32_t* code, bool* live) {
+    const u32x2 s0 = pcg2d_step(seed);
+    const u32x2 s1 = pcg2d_step(s0);
+    seed = s1;
+    const float2 nux = __fmul2_rn(make_float2((float)s0.x, (float)s1.x), both(-kRecip2e32));
+    const float2 uy = __fmul2_rn(make_float2((float)s0.y, (float)s1.y), both(kRecip2e32));
+    // inv_dilog((1 - u.x) * Li2(alpha)) (random.cuh:110-127, 132-141)
+    const float2 x = __fmul2_rn(__fmul2_rn(__fadd2_rn(both(1.0f), nux), both(c.li2_alpha)), both(1.0f / kLi2Max));
+    const float2 t = make_float2(fminf(x.x, 1.0f), fminf(x.y, 1.0f));
+    float2 y = both(-1.27463503e+01f);
+    y = __ffma2_rn(y, t, both(5.88993459e+01f));
+    y = __ffma2_rn(y, t, both(-1.16025780e+02f));
+    y = __ffma2_rn(y, t, both(1.26945827e+02f));
+    y = __ffma2_rn(y, t, both(-8.43108826e+01f));
+    y = __ffma2_rn(y, t, both(3.48799862e+01f));
+    y = __ffma2_rn(y, t, both(-8.89606235e+00f));
+    y = __ffma2_rn(y, t, both(1.38640936e+00f));
+    y = __ffma2_rn(y, t, both(-7.80640876e-01f));
+    y = __ffma2_rn(y, t, both(1.64841888e+00f));
+    y = __ffma2_rn(y, t, both(-2.82836687e-05f));
+    const float2 a2 = __fmul2_rn(both(c.inv_alpha), y);
+    // minus the radicand -2 log(a) (scaling by 2 is exact) and minus its root
+    const float2 m = __fmul2_rn(both(2.0f), make_float2(__logf(gclamp(a2.x, 1.e-37f, 1.0f)), __logf(gclamp(a2.y, 1.e-37f, 1.0f))));
+    const float2 rs = make_float2(rsqrtf(fmaxf(-m.x, 1.0e-30f)), rsqrtf(fmaxf(-m.y, 1.0e-30f)));
+    const float2 ng = __fmul2_rn(m, rs);
+    const float2 nr = __ffma2_rn(__ffma2_rn(ng, ng, m), __fmul2_rn(both(0.5f), rs), ng);
+    const float2 th = __fmul2_rn(both(2.0f * kPiF), uy);
+    float sn[2], cs[2];
+    __sincosf(th.x, &sn[0], &cs[0]);
+    __sincosf(th.y, &sn[1], &cs[1]);
+    const float2 nxyx = __fmul2_rn(nr, make_float2(cs[0], cs[1]));
+    const float2 nxyy = __fmul2_rn(nr, make_float2(sn[0], sn[1]));
+    const float2 px = __ffma2_rn(both(-c.c0), nxyx, both(c.pixel_mean.x));
+    const float2 py = __ffma2_rn(both(-c.c2), nxyy, __ffma2_rn(both(-c.c1), nxyx, both(c.pixel_mean.y)));
+    const float2 bx = __fadd2_rd(px, both(kFloorMagic)), by = __fadd2_rd(py, both(kFloorMagic));
+    // minus the offset pixel_mean - floor(pixel)
+    const float2 ndx = __ffma2_rn(both(c.pixel_mean.x), both(-1.0f), __fadd2_rn(bx, both(-kFloorMagic)));
+    const float2 ndy = __ffma2_rn(both(c.pixel_mean.y), both(-1.0f), __fadd2_rn(by, both(-kFloorMagic)));
+    // gaussian_value (linalg.cuh:309-317) on both samples.  Its sums of two products are fused
+    // as the compiler contracts them, the left product into the FMA: x*x-part first
+    // (fma(cx dx, dx, (cz dy) dy)), then fma(-0.5, quad, -((cy dx) dy)).  The tests pin this:
+    // fusing the right-hand products instead changed one entry of the 4K parity case.
+    const float2 quad = __ffma2_rn(__fmul2_rn(both(c.conic.x), ndx), ndx, __fmul2_rn(__fmul2_rn(both(c.conic.z), ndy), ndy));
+    const float2 nhh = __fmul2_rn(__fmul2_rn(both(-c.conic.y), ndx), ndy);
+    const float2 sig = __ffma2_rn(both(-0.5f), quad, nhh);
+    const float2 gv = make_float2(sig.x > 0.f ? 0.0f : __expf(sig.x), sig.y > 0.f ? 0.0f : __expf(sig.y));
+    const float2 al = __fmul2_rn(both(c.opacity), gv);
 #pragma unroll
-    for (int j = 0; j < K; j += 2) {
-        u32x2 s0 = pcg2d_step(seed);
-        u32x2 s1 = pcg2d_step(s0);
-        seed = s1;
-        const float2 rk = make_float2(kRecip2e32, kRecip2e32);
-        const float2 ux = __fmul2_rn(make_float2((float)s0.x, (float)s1.x), rk);
-        const float2 uy = __fmul2_rn(make_float2((float)s0.y, (float)s1.y), rk);
-        // inv_dilog((1 - u.x) * Li2(alpha)) (random.cuh:110-127, 132-141)
-        const float2 x = __fmul2_rn(__fadd2_rn(one, make_float2(-ux.x, -ux.y)), li2);
-        const float2 t = make_float2(fminf(x.x / kLi2Max, 1.0f), fminf(x.y / kLi2Max, 1.0f));
-        float2 y = make_float2(-1.27463503e+01f, -1.27463503e+01f);
-        y = __ffma2_rn(y, t, make_float2(5.88993459e+01f, 5.88993459e+01f));
-        y = __ffma2_rn(y, t, make_float2(-1.16025780e+02f, -1.16025780e+02f));
-        y = __ffma2_rn(y, t, make_float2(1.26945827e+02f, 1.26945827e+02f));
-        y = __ffma2_rn(y, t, make_float2(-8.43108826e+01f, -8.43108826e+01f));
-        y = __ffma2_rn(y, t, make_float2(3.48799862e+01f, 3.48799862e+01f));
-        y = __ffma2_rn(y, t, make_float2(-8.89606235e+00f, -8.89606235e+00f));
-        y = __ffma2_rn(y, t, make_float2(1.38640936e+00f, 1.38640936e+00f));
-        y = __ffma2_rn(y, t, make_float2(-7.80640876e-01f, -7.80640876e-01f));
-        y = __ffma2_rn(y, t, make_float2(1.64841888e+00f, 1.64841888e+00f));
-        y = __ffma2_rn(y, t, make_float2(-2.82836687e-05f, -2.82836687e-05f));
-        const float2 a2 = __fmul2_rn(inva, y);
-        float r[2], sn[2], cs[2];
-        // -2 log(a) and the angle 2 pi u: one product each, paired (scaling by -2 is exact, so
-        // the pair equals the scalar (lg2(a) ln2) (-2) however the scalar form groups it)
-        const float2 lg = __fmul2_rn(make_float2(-2.0f, -2.0f), make_float2(__logf(gclamp(a2.x, 1.e-37f, 1.0f)),
-                                                                             __logf(gclamp(a2.y, 1.e-37f, 1.0f))));
-        const float2 th = __fmul2_rn(make_float2(2.0f * kPiF, 2.0f * kPiF), uy);
-#pragma unroll
-        for (int l = 0; l < 2; ++l) {
-            r[l] = __fsqrt_rn(fmaxf(l ? lg.y : lg.x, 0.0f));
-            __sincosf(l ? th.y : th.x, &sn[l], &cs[l]);
-        }
-        const float2 rr = make_float2(r[0], r[1]);
-        const float2 xyx = __fmul2_rn(rr, make_float2(cs[0], cs[1]));
-        const float2 xyy = __fmul2_rn(rr, make_float2(sn[0], sn[1]));
-        const float2 px = __ffma2_rn(c0, xyx, pmx);
-        const float2 py = __ffma2_rn(c2, xyy, __ffma2_rn(c1, xyx, pmy));
-        const float2 fx = make_float2(floorf(px.x), floorf(px.y)), fy = make_float2(floorf(py.x), floorf(py.y));
-        const float2 dx = __fadd2_rn(pmx, make_float2(-fx.x, -fx.y));
-        const float2 dy = __fadd2_rn(pmy, make_float2(-fy.x, -fy.y));
-        // gaussian_value (linalg.cuh:309-317) on both samples.  Its sums of two products are fused
-        // as the compiler contracts them, the left product into the FMA: x*x-part first
-        // (fma(cx dx, dx, (cz dy) dy)), then fma(-0.5, quad, -((cy dx) dy)).  The tests pin this:
-        // fusing the right-hand products instead changed one entry of the 4K parity case.
-        const float2 cx = make_float2(c.conic.x, c.conic.x), cyv = make_float2(c.conic.y, c.conic.y),
-                     cz = make_float2(c.conic.z, c.conic.z);
-        const float2 quad = __ffma2_rn(__fmul2_rn(cx, dx), dx, __fmul2_rn(__fmul2_rn(cz, dy), dy));
-        const float2 hh = __fmul2_rn(__fmul2_rn(cyv, dx), dy);
-        const float2 sig = __ffma2_rn(make_float2(-0.5f, -0.5f), quad, make_float2(-hh.x, -hh.y));
-        const float2 gv = make_float2(sig.x > 0.f ? 0.0f : __expf(sig.x), sig.y > 0.f ? 0.0f : __expf(sig.y));
-        const float2 al = __fmul2_rn(make_float2(c.opacity, c.opacity), gv);
-#pragma unroll
-        for (int l = 0; l < 2; ++l) {
-            const int xi = (int)(l ? fx.y : fx.x);
-            const int yi = (int)(l ? fy.y : fy.x);
-            const bool inside = ((uint32_t)xi - (uint32_t)c.minx < c.span_x) & ((uint32_t)yi - (uint32_t)c.miny < c.span_y);
-            const float alpha = l ? al.y : al.x;
+    for (int l = 0; l < 2; ++l) {
+        const uint32_t xb = __float_as_uint(l ? bx.y : bx.x), yb = __float_as_uint(l ? by.y : by.x);  // pixel + kFloorBits
+        const bool inside = (xb - (kFloorBits + (uint32_t)c.minx) < c.span_x) & (yb - (kFloorBits + (uint32_t)c.miny) < c.span_y);
 #if GPS_SPLAT_MORTON_LUT
-            code[j + l] = c.spread[xi & (kTileSize - 1)] | (c.spread[yi & (kTileSize - 1)] << 1);
+        code[l] = c.spread[xb & (kTileSize - 1)] | (c.spread[yb & (kTileSize - 1)] << 1);
 #else
-            code[j + l] = morton_encode((uint32_t)(xi & (kTileSize - 1)), (uint32_t)(yi & (kTileSize - 1)));
+        code[l] = morton_encode(xb & (kTileSize - 1), yb & (kTileSize - 1));
 #endif
-            tile[j + l] = (uint32_t)((yi >> kTileBits) * c.tiles_per_row + (xi >> kTileBits));
-            live[j + l] = inside & !(alpha < 1.0f / 255.0f);
-        }
+        tile[l] = (yb >> kTileBits) * (uint32_t)c.tiles_per_row + (xb >> kTileBits);  // plus c.tile_bias
+        live[l] = inside & !((l ? al.y : al.x) < 1.0f / 255.0f);
     }
 }
 
@@ -1251,14 +1253,24 @@ __device__ __forceinline__ SampleConst sample_const(const SplatRecord& rec, cons
     c.li2_alpha = dilog(c.opacity);
     c.passes = fc.num_passes;
     c.tiles_per_row = (fc.up_width + kTileSize - 1) >> kTileBits;
+    c.tile_bias = (kFloorBits >> kTileBits) * ((uint32_t)c.tiles_per_row + 1u);
+    c.slot_bias = 0u - c.tile_bias * (uint32_t)(kTileSize * kTileSize) * (uint32_t)c.passes;
     return c;
+}
+
+// Means or factors for which a pixel position may overflow or be no number: draw_pair leaves those
+// to draw_sample, whose conversion takes a NaN to pixel 0.
+__device__ __forceinline__ bool wide_sample(const SampleConst& c) {
+    const float sum = fabsf(c.c0) + fabsf(c.c1) + fabsf(c.c2) + fabsf(c.pixel_mean.x) + fabsf(c.pixel_mean.y);
+    return __float_as_uint(sum) >= __float_as_uint(1.0e30f);  // (by the bits: a NaN too)
 }
 
 // The K samples of one spp pass.
 template <int K>
 __device__ __forceinline__ void draw_pass(u32x2& seed, const SampleConst& c, uint32_t* tile, uint32_t* code, bool* live) {
-    if constexpr (GPS_SPLAT_PAIRED && K % 2 == 0) {
-        draw_samples_paired<K>(seed, c, tile, code, live);
+    if constexpr (K % 2 == 0) {
+#pragma unroll
+        for (int j = 0; j < K; j += 2) draw_pair(seed, c, tile + j, code + j, live + j);
     } else {
 #pragma unroll
         for (int j = 0; j < K; ++j) live[j] = draw_sample(seed, c, tile[j], code[j]);
@@ -1266,7 +1278,19 @@ __device__ __forceinline__ void draw_pass(u32x2& seed, const SampleConst& c, uin
 }
 
 __device__ __forceinline__ uint32_t sample_slot(const SampleConst& c, uint32_t tile, uint32_t code, int p) {
-    return (tile * (uint32_t)(kTileSize * kTileSize) + code) * (uint32_t)c.passes + (uint32_t)p;
+    return (tile * (uint32_t)(kTileSize * kTileSize) + code) * (uint32_t)c.passes + ((uint32_t)p + c.slot_bias);
+}
+
+// A point that draw_pass leaves out (even K and wide_sample): one sample after the other, untested.
+template <int K>
+__device__ __forceinline__ bool splat_wide_point(u32x2 seed, const SampleConst& c, unsigned long long key,
+                                                 unsigned long long* buf) {
+    if (K % 2 != 0 || !wide_sample(c)) return false;
+    for (int i = 0; i < c.passes * K; ++i) {
+        uint32_t tile, code;
+        if (draw_sample(seed, c, tile, code)) atomicMin(buf + sample_slot(c, tile, code, i / K), key);
+    }
+    return true;
 }
 
 template <int K>
@@ -1277,6 +1301,7 @@ __device__ __forceinline__ void splat_point_unbiased_k(uint32_t point, const Spl
     const SampleConst c = sample_const(rec, fc, spread);
     const unsigned long long key = (unsigned long long)rec.d.z | ((unsigned long long)rec.d.w << 32);
     unsigned long long* buf = reinterpret_cast<unsigned long long*>(buffer);
+    if (splat_wide_point<K>(seed, c, key, buf)) return;
 #if GPS_SPLAT_PRETEST && GPS_SPLAT_PIPELINE
     // Software-pipelined over passes: pass p+1's samples are drawn and their pre-test loads
     // issued before pass p's atomics consume its loads, so the load latency hides behind the
@@ -1341,6 +1366,8 @@ __device__ __forceinline__ void splat_point_in_tile(uint32_t point, const SplatR
     const uint32_t key_high = rec.d.w;
     const unsigned long long key = (unsigned long long)rec.d.z | ((unsigned long long)rec.d.w << 32);
     unsigned long long* buf = reinterpret_cast<unsigned long long*>(buffer);
+    if (splat_wide_point<K>(seed, c, key, buf)) return;
+    my_tile += c.tile_bias;
     for (int p = 0; p < c.passes; ++p, nearest += kNearPlane) {
         uint32_t tile[K], code[K], seen[K];
         bool live[K];
