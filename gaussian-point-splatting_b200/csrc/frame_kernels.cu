@@ -438,7 +438,7 @@ __global__ void __launch_bounds__(256) preprocess_kernel(PreprocessArgs a, Scene
         const unsigned m = __ballot_sync(0xffffffffu, splats);
         loaded_tally += (uint32_t)__popc(__ballot_sync(0xffffffffu, loaded));
         if (lane == 0) mask_cur[c] = m;
-        if (a.tile_totals && m) {
+        if (m) {
             const uint32_t t = (c << 5) >> a.tile_shift;
             if (t != tile) {
                 flush_tile();
@@ -460,35 +460,22 @@ __global__ void __launch_bounds__(256) preprocess_kernel(PreprocessArgs a, Scene
             }
         }
     };
-    if (a.chunk_list) {
-        const uint32_t count = *a.chunk_count;
-        if (a.tile_totals) {  // contiguous ranges of the (ascending) list, so tile totals merge
-            const uint32_t per = (count + warps - 1) / warps;
-            const uint32_t b = first * per, e = min(count, b + per);
-            // the next chunk's attributes are prefetched into L2 while this one is worked on
-            // (256M town: preprocess 1.149 -> 1.130 ms/frame)
-            uint32_t next = b < e ? __ldg(a.chunk_list + b) : 0u;
-            for (uint32_t i = b; i < e; ++i) {
-                const uint32_t c = next;
-                if (i + 1 < e) {
-                    next = __ldg(a.chunk_list + i + 1);
-                    const uint32_t g = (next << 5) + lane;
-                    if (g < a.n) scene.prefetch(g);
-                }
-                chunk(c);
-            }
-        } else {
-            for (uint32_t i = first; i < count; i += warps) chunk(__ldg(a.chunk_list + i));
+    // contiguous ranges of the list (or of all chunks), so that tile totals merge; the next listed
+    // chunk's attributes are prefetched into L2 while this one is worked on (256M town: preprocess
+    // 1.149 -> 1.130 ms/frame)
+    const uint32_t count = a.chunk_list ? *a.chunk_count : (a.n + 31u) >> 5;
+    const uint32_t per = (count + warps - 1) / warps;
+    const uint32_t b = first * per, e = min(count, b + per);
+    uint32_t next = b < e && a.chunk_list ? __ldg(a.chunk_list + b) : b;
+    for (uint32_t i = b; i < e; ++i) {
+        const uint32_t c = next;
+        ++next;
+        if (a.chunk_list && i + 1 < e) {
+            next = __ldg(a.chunk_list + i + 1);
+            const uint32_t g = (next << 5) + lane;
+            if (g < a.n) scene.prefetch(g);
         }
-    } else {
-        const uint32_t chunks = (a.n + 31u) >> 5;
-        if (a.tile_totals) {
-            const uint32_t per = (chunks + warps - 1) / warps;
-            const uint32_t b = first * per, e = min(chunks, b + per);
-            for (uint32_t c = b; c < e; ++c) chunk(c);
-        } else {
-            for (uint32_t c = first; c < chunks; c += warps) chunk(c);
-        }
+        chunk(c);
     }
     flush_tile();
     if (a.loaded && lane == 0 && loaded_tally) atomicAdd(a.loaded, loaded_tally);
@@ -938,10 +925,10 @@ __global__ void __launch_bounds__(256) bin_survivors_kernel(ScanArgs a) {
 // ---------------------------------------------------------------------------------
 constexpr int kSplatTile = 256;
 
-__device__ __forceinline__ void atomic_add_color(unsigned long long* address, uint64_t value) {
-    // post_processing_kernels.cuh:13-42 with add_if_equal = true
+// post_processing_kernels.cuh:13-42 with add_if_equal = true; `old` is a value the slot held
+__device__ __forceinline__ void atomic_add_color(unsigned long long* address, unsigned long long old, uint64_t value) {
     const uint64_t target_depth = value & kDepthMask;
-    unsigned long long old = *address, assumed;
+    unsigned long long assumed;
     do {
         assumed = old;
         uint64_t assumed_depth = assumed & kDepthMask;
@@ -955,9 +942,14 @@ __device__ __forceinline__ void atomic_add_color(unsigned long long* address, ui
     } while (assumed != old);
 }
 
-// Biased mode (use_unbiased_2d_splatting = false): samples in the reference's order, each
-// pre-tested and colour-added before the next one is drawn.
-// One point's samples from `seed` onwards (the seed advances, as splatGaussianPoint's does).
+// Biased mode (use_unbiased_2d_splatting = false): one point's samples from `seed` onwards (the seed
+// advances, as splatGaussianPoint's does), kBiasedBatch at a time: their slots, then their
+// pre-test loads together, then the additions, which start from the loaded values.  A load that
+// missed an addition made since costs a second compare-and-swap, no more: a slot's depth only
+// decreases.  (Before, one sample waited for the last one's two loads: 300k town,
+// 999x571, 4 spp: frame 110.3 -> 109.5 us)
+constexpr int kBiasedBatch = 4;
+
 __device__ __forceinline__ void splat_samples_biased(u32x2& seed, const SplatRecord& rec, const FrameConst& fc,
                                                      uint64_t* __restrict__ buffer) {
     const vec2 pixel_mean = make_v2(rec.a.x, rec.a.y);
@@ -970,22 +962,40 @@ __device__ __forceinline__ void splat_samples_biased(u32x2& seed, const SplatRec
     const uint64_t view_depth_bits = key & kDepthMask;
     const int k = fc.k_points;
     const int samples = fc.num_passes * k;
-    for (int p = 0; p < samples; ++p) {
-        vec2 u = pcg2d(seed);
-        vec2 xy = box_muller(u.x, u.y);
-        vec2 pixel = make_v2(pixel_mean.x + c0 * xy.x, pixel_mean.y + c1 * xy.x + c2 * xy.y);
-        pixel = make_v2(floorf(pixel.x), floorf(pixel.y));
-        int x = (int)pixel.x;
-        int y = (int)pixel.y;
-        vec2 delta = make_v2(pixel_mean.x - pixel.x, pixel_mean.y - pixel.y);
-        if (x < minx || x >= maxx || y < miny || y >= maxy) continue;
-        float gw = gaussian_value(conic, delta);
-        float alpha = opacity * gw;
-        if (alpha < 1.0f / 255.0f) continue;
-        int index = splat_index(x, y, p / k, fc.num_passes, fc.up_width, fc.up_height);
-        unsigned long long* slot = reinterpret_cast<unsigned long long*>(buffer + index);
-        if ((uint64_t)__ldcg(slot) <= view_depth_bits) continue;
-        atomic_add_color(slot, key);
+    unsigned long long* buf = reinterpret_cast<unsigned long long*>(buffer);
+    int pass = 0, j = 0;  // sample s0 + b is draw j of spp pass `pass`
+    for (int s0 = 0; s0 < samples; s0 += kBiasedBatch) {
+        int slot[kBiasedBatch];
+        bool live[kBiasedBatch];
+#pragma unroll
+        for (int b = 0; b < kBiasedBatch; ++b) {
+            live[b] = false;
+            slot[b] = 0;
+            if (s0 + b >= samples) continue;
+            vec2 u = pcg2d(seed);
+            vec2 xy = box_muller(u.x, u.y);
+            vec2 pixel = make_v2(pixel_mean.x + c0 * xy.x, pixel_mean.y + c1 * xy.x + c2 * xy.y);
+            pixel = make_v2(floorf(pixel.x), floorf(pixel.y));
+            int x = (int)pixel.x;
+            int y = (int)pixel.y;
+            vec2 delta = make_v2(pixel_mean.x - pixel.x, pixel_mean.y - pixel.y);
+            if (x >= minx && x < maxx && y >= miny && y < maxy) {
+                float gw = gaussian_value(conic, delta);
+                float alpha = opacity * gw;
+                live[b] = !(alpha < 1.0f / 255.0f);
+                slot[b] = splat_index(x, y, pass, fc.num_passes, fc.up_width, fc.up_height);
+            }
+            if (++j == k) {
+                j = 0;
+                ++pass;
+            }
+        }
+        unsigned long long seen[kBiasedBatch];
+#pragma unroll
+        for (int b = 0; b < kBiasedBatch; ++b) seen[b] = live[b] ? __ldcg(buf + slot[b]) : 0ull;
+#pragma unroll
+        for (int b = 0; b < kBiasedBatch; ++b)
+            if (live[b] && (uint64_t)seen[b] > view_depth_bits) atomic_add_color(buf + slot[b], seen[b], key);
     }
 }
 
@@ -995,17 +1005,13 @@ __device__ __forceinline__ void splat_point_biased(uint32_t point, const SplatRe
     splat_samples_biased(seed, rec, fc, buffer);
 }
 
-// Unbiased mode (the default): the same sample stream, drawn kSplatBatch samples at a time.
-// Each batch computes its slots first, then issues their pre-test loads together (several
-// loads in flight per thread instead of one), then the atomicMins.  Order does not matter for
-// a min, and a slot is skipped only when it already holds a value <= this Gaussian's key, the
-// exact condition under which atomicMin would leave it unchanged (the reference skips when
-// the slot is <= the depth bits alone, a subset of these cases), so the buffer is identical.
-// Slot values only decrease during the kernel, so an L1-cached (possibly stale, hence larger)
-// pre-test value can only cause an extra atomic, never a wrong skip.
-#ifndef GPS_SPLAT_BATCH
-#define GPS_SPLAT_BATCH 4
-#endif
+// Unbiased mode (the default).  A sample's slot is loaded before its atomicMin is issued (the
+// pre-test), several loads in flight per thread.  Order does not matter for a min, and a slot is
+// skipped only when it already holds a value <= this Gaussian's key, the exact condition under
+// which atomicMin would leave it unchanged (the reference skips when the slot is <= the depth bits
+// alone, a subset of these cases), so the buffer is identical.  Slot values only decrease during
+// the kernel, so an L1-cached (possibly stale, hence larger) pre-test value can only cause an
+// extra atomic, never a wrong skip.
 // Pre-test before the atomic: 1 = L1-cached load, 2 = L2 load, 0 = none (every live sample
 // issues its atomicMin; the buffer is the same in all three).  On the 16M-Gaussian town orbit
 // (1080p, ss 2, 4 spp) the L1-cached pre-test measured fastest on B200 (splat 2.04 ms/frame vs
@@ -1014,97 +1020,8 @@ __device__ __forceinline__ void splat_point_biased(uint32_t point, const SplatRe
 #ifndef GPS_SPLAT_PRETEST
 #define GPS_SPLAT_PRETEST 1
 #endif
-#ifndef GPS_SPLAT_PIPELINE
-#define GPS_SPLAT_PIPELINE 1
-#endif
-// 1: a sample's in-tile Morton code comes from a 64-entry shared-memory table of spread 6-bit
-// coordinates (two table loads) instead of two 4-step bit spreads; the codes are identical.
-// Measured on the 16M-Gaussian town orbit (1080p, ss 2, 4 spp): splat 1.90 vs 1.96 ms/frame.
-#ifndef GPS_SPLAT_MORTON_LUT
-#define GPS_SPLAT_MORTON_LUT 1
-#endif
-constexpr int kSplatBatch = GPS_SPLAT_BATCH;
-
-__device__ __forceinline__ void splat_samples_unbiased(u32x2& seed, const SplatRecord& rec, const FrameConst& fc,
-                                                       uint64_t* __restrict__ buffer) {
-    const vec2 pixel_mean = make_v2(rec.a.x, rec.a.y);
-    const float c0 = rec.a.z, c1 = rec.a.w, c2 = rec.b.x;
-    const vec3 conic = make_v3(rec.b.y, rec.b.z, rec.b.w);
-    const float opacity = rec.c.x;
-    const int minx = (int)(rec.d.x & 0xFFFFu), miny = (int)(rec.d.x >> 16);
-    const int maxx = (int)(rec.d.y & 0xFFFFu), maxy = (int)(rec.d.y >> 16);
-    const unsigned long long key = (unsigned long long)rec.d.z | ((unsigned long long)rec.d.w << 32);
-    // the per-Gaussian factors of correctedBoxMuller (random.cuh:132-141), evaluated once
-    const float inv_alpha = 1.0f / fmaxf(opacity, 1.e-37f);
-    const float li2_alpha = dilog(opacity);
-    const int k = fc.k_points;
-    const int samples = fc.num_passes * k;
-    const int passes = fc.num_passes;
-    const int tiles_per_row = (fc.up_width + kTileSize - 1) >> kTileBits;
-    int p = 0, j = 0;
-    for (int s0 = 0; s0 < samples; s0 += kSplatBatch) {
-        uint32_t slot[kSplatBatch];
-        uint32_t live = 0;
-#pragma unroll
-        for (int b = 0; b < kSplatBatch; ++b) {
-            slot[b] = 0;
-            if (s0 + b < samples) {
-                vec2 u = pcg2d(seed);
-                float a = inv_alpha * inv_dilog((1.0f - u.x) * li2_alpha);
-                a = gclamp(a, 1.e-37f, 1.0f);
-                float r = __fsqrt_rn(fmaxf(-2.0f * __logf(a), 0.0f));
-                float theta = 2.0f * kPiF * u.y;
-                float sn, cs;
-                __sincosf(theta, &sn, &cs);
-                vec2 xy = make_v2(r * cs, r * sn);
-                vec2 pixel = make_v2(pixel_mean.x + c0 * xy.x, pixel_mean.y + c1 * xy.x + c2 * xy.y);
-                pixel = make_v2(floorf(pixel.x), floorf(pixel.y));
-                int x = (int)pixel.x;
-                int y = (int)pixel.y;
-                vec2 delta = make_v2(pixel_mean.x - pixel.x, pixel_mean.y - pixel.y);
-                if (x >= minx && x < maxx && y >= miny && y < maxy) {
-                    float alpha = opacity * gaussian_value(conic, delta);
-                    if (!(alpha < 1.0f / 255.0f)) {
-                        const uint32_t code = morton_encode((uint32_t)(x & (kTileSize - 1)), (uint32_t)(y & (kTileSize - 1)));
-                        const uint32_t tile = (uint32_t)((y >> kTileBits) * tiles_per_row + (x >> kTileBits));
-                        slot[b] = (tile * (uint32_t)(kTileSize * kTileSize) + code) * (uint32_t)passes + (uint32_t)p;
-                        live |= 1u << b;
-                    }
-                }
-                if (++j == k) {
-                    j = 0;
-                    ++p;
-                }
-            }
-        }
-#if GPS_SPLAT_PRETEST
-        unsigned long long seen[kSplatBatch];
-#pragma unroll
-        for (int b = 0; b < kSplatBatch; ++b) {
-            const unsigned long long* at = reinterpret_cast<const unsigned long long*>(buffer) + slot[b];
-            seen[b] = ((live >> b) & 1u) ? (GPS_SPLAT_PRETEST == 1 ? __ldca(at) : __ldcg(at)) : 0ull;
-        }
-#pragma unroll
-        for (int b = 0; b < kSplatBatch; ++b)
-            if (((live >> b) & 1u) && seen[b] > key)
-                atomicMin(reinterpret_cast<unsigned long long*>(buffer) + slot[b], key);
-#else
-#pragma unroll
-        for (int b = 0; b < kSplatBatch; ++b)
-            if ((live >> b) & 1u) atomicMin(reinterpret_cast<unsigned long long*>(buffer) + slot[b], key);
-#endif
-    }
-}
-
-__device__ __forceinline__ void splat_point_unbiased(uint32_t point, const SplatRecord& rec, const FrameConst& fc,
-                                                     int frame_seed, uint64_t* __restrict__ buffer) {
-    u32x2 seed = make_seed(point, (uint32_t)frame_seed);
-    splat_samples_unbiased(seed, rec, fc, buffer);
-}
-
-// The same stream with K (points per thread per pass, ss*ss) known at compile time: the K
-// samples of a pass are drawn without branches (bounds and alpha tests become predicates), so
-// their independent transcendental chains can be interleaved, then the live ones are splatted.
+// Samples are drawn without branches (bounds and alpha tests become predicates), so that the
+// independent transcendental chains of several interleave, then the live ones are splatted.
 struct SampleConst {
     vec2 pixel_mean;
     float c0, c1, c2, opacity, inv_alpha, li2_alpha;
@@ -1114,7 +1031,7 @@ struct SampleConst {
     int tiles_per_row, passes;
     uint32_t tile_bias;      // added to every tile index below, and taken off again with the slot
     uint32_t slot_bias;
-    const uint32_t* spread;  // shared-memory Morton table (GPS_SPLAT_MORTON_LUT)
+    const uint32_t* spread;  // shared-memory Morton table (null: codes are computed)
 };
 
 // Adding 1.5 * 2^23 with rounding down leaves floor(v) in the low mantissa bits for |v| < 2^22:
@@ -1123,6 +1040,15 @@ struct SampleConst {
 // over all floats).
 constexpr float kFloorMagic = 12582912.0f;
 constexpr uint32_t kFloorBits = 0x4B400000u;
+
+// The Morton code in its tile of a pixel: two loads from a 64-entry shared-memory table of spread
+// 6-bit coordinates instead of two 4-step bit spreads (16M town, 1080p, ss 2, 4 spp: splat 1.90 vs 1.96
+// ms/frame).  (The null test folds away where the kernel has a table.)
+__device__ __forceinline__ uint32_t morton_code(const SampleConst& c, uint32_t x, uint32_t y) {
+    x &= kTileSize - 1;
+    y &= kTileSize - 1;
+    return c.spread ? c.spread[x] | (c.spread[y] << 1) : morton_encode(x, y);
+}
 
 // One sample: whether it is live, its splat-buffer tile (plus c.tile_bias) and the Morton code of its
 // place there.
@@ -1144,11 +1070,7 @@ __device__ __forceinline__ bool draw_sample(u32x2& seed, const SampleConst& c, u
     // splat 1.572 -> 1.563 ms/frame on the 16M orbit
     const bool inside = ((uint32_t)x - (uint32_t)c.minx < c.span_x) & ((uint32_t)y - (uint32_t)c.miny < c.span_y);
     const float alpha = c.opacity * gaussian_value(c.conic, delta);
-#if GPS_SPLAT_MORTON_LUT
-    code = c.spread[x & (kTileSize - 1)] | (c.spread[y & (kTileSize - 1)] << 1);
-#else
-    code = morton_encode((uint32_t)(x & (kTileSize - 1)), (uint32_t)(y & (kTileSize - 1)));
-#endif
+    code = morton_code(c, (uint32_t)x, (uint32_t)y);
     tile = (uint32_t)((y >> kTileBits) * c.tiles_per_row + (x >> kTileBits)) + c.tile_bias;
     return inside & !(alpha < 1.0f / 255.0f);
 }
@@ -1223,14 +1145,33 @@ __device__ __forceinline__ void draw_pair(u32x2& seed, const SampleConst& c, uin
     for (int l = 0; l < 2; ++l) {
         const uint32_t xb = __float_as_uint(l ? bx.y : bx.x), yb = __float_as_uint(l ? by.y : by.x);  // pixel + kFloorBits
         const bool inside = (xb - (kFloorBits + (uint32_t)c.minx) < c.span_x) & (yb - (kFloorBits + (uint32_t)c.miny) < c.span_y);
-#if GPS_SPLAT_MORTON_LUT
-        code[l] = c.spread[xb & (kTileSize - 1)] | (c.spread[yb & (kTileSize - 1)] << 1);
-#else
-        code[l] = morton_encode(xb & (kTileSize - 1), yb & (kTileSize - 1));
-#endif
+        code[l] = morton_code(c, xb, yb);
         tile[l] = (yb >> kTileBits) * (uint32_t)c.tiles_per_row + (xb >> kTileBits);  // plus c.tile_bias
         live[l] = inside & !((l ? al.y : al.x) < 1.0f / 255.0f);
     }
+}
+
+// One sample the same way (not where wide_sample(c)).
+__device__ __forceinline__ bool draw_one(u32x2& seed, const SampleConst& c, uint32_t& tile, uint32_t& code) {
+    const vec2 u = pcg2d(seed);
+    const float a = c.inv_alpha * inv_dilog((1.0f - u.x) * c.li2_alpha);
+    const float m = 2.0f * __logf(gclamp(a, 1.e-37f, 1.0f));
+    const float rs = rsqrtf(fmaxf(-m, 1.0e-30f)), ng = __fmul_rn(m, rs);
+    const float nr = __fmaf_rn(__fmaf_rn(ng, ng, m), __fmul_rn(0.5f, rs), ng);
+    float sn, cs;
+    __sincosf(2.0f * kPiF * u.y, &sn, &cs);
+    const float nx = __fmul_rn(nr, cs), ny = __fmul_rn(nr, sn);
+    const float bx = __fadd_rd(__fmaf_rn(-c.c0, nx, c.pixel_mean.x), kFloorMagic);
+    const float by = __fadd_rd(__fmaf_rn(-c.c2, ny, __fmaf_rn(-c.c1, nx, c.pixel_mean.y)), kFloorMagic);
+    const float dx = __fsub_rn(c.pixel_mean.x, __fadd_rn(bx, -kFloorMagic)), dy = __fsub_rn(c.pixel_mean.y, __fadd_rn(by, -kFloorMagic));
+    const float quad = __fmaf_rn(__fmul_rn(c.conic.x, dx), dx, __fmul_rn(__fmul_rn(c.conic.z, dy), dy));
+    const float sig = __fmaf_rn(-0.5f, quad, -__fmul_rn(__fmul_rn(c.conic.y, dx), dy));
+    const float alpha = c.opacity * (sig > 0.f ? 0.0f : __expf(sig));
+    const uint32_t xb = __float_as_uint(bx), yb = __float_as_uint(by);
+    code = morton_code(c, xb, yb);
+    tile = (yb >> kTileBits) * (uint32_t)c.tiles_per_row + (xb >> kTileBits);
+    return (xb - (kFloorBits + (uint32_t)c.minx) < c.span_x) & (yb - (kFloorBits + (uint32_t)c.miny) < c.span_y) &
+           !(alpha < 1.0f / 255.0f);
 }
 
 __device__ __forceinline__ SampleConst sample_const(const SplatRecord& rec, const FrameConst& fc, const uint32_t* spread) {
@@ -1265,89 +1206,139 @@ __device__ __forceinline__ bool wide_sample(const SampleConst& c) {
     return __float_as_uint(sum) >= __float_as_uint(1.0e30f);  // (by the bits: a NaN too)
 }
 
-// The K samples of one spp pass.
-template <int K>
-__device__ __forceinline__ void draw_pass(u32x2& seed, const SampleConst& c, uint32_t* tile, uint32_t* code, bool* live) {
-    if constexpr (K % 2 == 0) {
-#pragma unroll
-        for (int j = 0; j < K; j += 2) draw_pair(seed, c, tile + j, code + j, live + j);
-    } else {
-#pragma unroll
-        for (int j = 0; j < K; ++j) live[j] = draw_sample(seed, c, tile[j], code[j]);
-    }
-}
-
 __device__ __forceinline__ uint32_t sample_slot(const SampleConst& c, uint32_t tile, uint32_t code, int p) {
     return (tile * (uint32_t)(kTileSize * kTileSize) + code) * (uint32_t)c.passes + ((uint32_t)p + c.slot_bias);
 }
 
-// A point that draw_pass leaves out (even K and wide_sample): one sample after the other, untested.
+// The draws of one step of a point: the K samples of an spp pass, or with K = 1 those of two passes
+// (one, if that is the last), so that there is a pair to draw together.  Draw j belongs to
+// pass + step_pass(j).
 template <int K>
-__device__ __forceinline__ bool splat_wide_point(u32x2 seed, const SampleConst& c, unsigned long long key,
-                                                 unsigned long long* buf) {
-    if (K % 2 != 0 || !wide_sample(c)) return false;
-    for (int i = 0; i < c.passes * K; ++i) {
-        uint32_t tile, code;
-        if (draw_sample(seed, c, tile, code)) atomicMin(buf + sample_slot(c, tile, code, i / K), key);
+struct DrawStep {
+    static_assert(K == 1 || K % 2 == 0, "samples are drawn in pairs");
+    static constexpr int kPasses = K == 1 ? 2 : 1, kDraws = K == 1 ? 2 : K;
+    uint32_t tile[kDraws], code[kDraws];
+    bool live[kDraws];
+    static __device__ __forceinline__ int step_pass(int j) { return K == 1 ? j : 0; }
+    __device__ __forceinline__ void draw(u32x2& seed, const SampleConst& c, int pass) {
+        if (K == 1 && pass + 1 >= c.passes) {
+            live[0] = draw_one(seed, c, tile[0], code[0]);
+            live[kDraws - 1] = false;
+            tile[kDraws - 1] = code[kDraws - 1] = 0u;
+            return;
+        }
+#pragma unroll
+        for (int j = 0; j < kDraws; j += 2) draw_pair(seed, c, tile + j, code + j, live + j);
     }
+};
+
+// A point that draw_pair leaves out: one sample after the other, untested.  False for any other.
+__device__ __forceinline__ bool splat_wide_point(u32x2& seed, const SampleConst& c, int k, unsigned long long key,
+                                                 unsigned long long* buf) {
+    if (!wide_sample(c)) return false;
+    for (int p = 0; p < c.passes; ++p)
+        for (int j = 0; j < k; ++j) {
+            uint32_t tile, code;
+            if (draw_sample(seed, c, tile, code)) atomicMin(buf + sample_slot(c, tile, code, p), key);
+        }
     return true;
 }
 
+__device__ __forceinline__ unsigned long long pretest_load(const unsigned long long* at) {
+    return GPS_SPLAT_PRETEST == 1 ? __ldca(at) : GPS_SPLAT_PRETEST == 2 ? __ldcg(at) : ~0ull;
+}
+
+// One point's samples from `seed` onwards, any k (the seed advances, as splatGaussianPoint's does).
+__device__ __forceinline__ void splat_samples_unbiased(u32x2& seed, const SplatRecord& rec, const FrameConst& fc,
+                                                       uint64_t* __restrict__ buffer) {
+    const SampleConst c = sample_const(rec, fc, nullptr);
+    const unsigned long long key = (unsigned long long)rec.d.z | ((unsigned long long)rec.d.w << 32);
+    unsigned long long* buf = reinterpret_cast<unsigned long long*>(buffer);
+    const int k = fc.k_points, samples = fc.num_passes * k;
+    if (splat_wide_point(seed, c, k, key, buf)) return;
+    int p = 0, j = 0;  // sample s0 + b is draw j of spp pass p
+    for (int s0 = 0; s0 < samples; s0 += 4) {
+        uint32_t tile[4], code[4], slot[4];
+        bool live[4];
+#pragma unroll
+        for (int b = 0; b < 4; b += 2) {
+            live[b] = live[b + 1] = false;
+            tile[b] = tile[b + 1] = code[b] = code[b + 1] = 0u;
+            if (s0 + b + 1 < samples) draw_pair(seed, c, tile + b, code + b, live + b);
+            else if (s0 + b < samples) live[b] = draw_one(seed, c, tile[b], code[b]);
+        }
+        unsigned long long seen[4];
+#pragma unroll
+        for (int b = 0; b < 4; ++b) {
+            slot[b] = sample_slot(c, tile[b], code[b], p);
+            if (++j == k) {
+                j = 0;
+                ++p;
+            }
+            seen[b] = live[b] ? pretest_load(buf + slot[b]) : 0ull;
+        }
+#pragma unroll
+        for (int b = 0; b < 4; ++b)
+            if (live[b] && seen[b] > key) atomicMin(buf + slot[b], key);
+    }
+}
+
+__device__ __forceinline__ void splat_point_unbiased(uint32_t point, const SplatRecord& rec, const FrameConst& fc,
+                                                     int frame_seed, uint64_t* __restrict__ buffer) {
+    u32x2 seed = make_seed(point, (uint32_t)frame_seed);
+    splat_samples_unbiased(seed, rec, fc, buffer);
+}
+
+// The same samples with K known at compile time.
 template <int K>
 __device__ __forceinline__ void splat_point_unbiased_k(uint32_t point, const SplatRecord& rec, const FrameConst& fc,
                                                        int frame_seed, uint64_t* __restrict__ buffer,
                                                        const uint32_t* spread) {
+    using Step = DrawStep<K>;
     u32x2 seed = make_seed(point, (uint32_t)frame_seed);
     const SampleConst c = sample_const(rec, fc, spread);
     const unsigned long long key = (unsigned long long)rec.d.z | ((unsigned long long)rec.d.w << 32);
     unsigned long long* buf = reinterpret_cast<unsigned long long*>(buffer);
-    if (splat_wide_point<K>(seed, c, key, buf)) return;
-#if GPS_SPLAT_PRETEST && GPS_SPLAT_PIPELINE
-    // Software-pipelined over passes: pass p+1's samples are drawn and their pre-test loads
-    // issued before pass p's atomics consume its loads, so the load latency hides behind the
-    // next pass's arithmetic.  Samples are still drawn in stream order.
-    uint32_t sa[K], sb[K];
-    bool la[K], lb[K];
-    unsigned long long va[K], vb[K];
+    if (splat_wide_point(seed, c, K, key, buf)) return;
+    if (K == 1 && c.passes == 1) {  // nothing to pair or to pipeline
+        uint32_t tile, code;
+        const bool live = draw_one(seed, c, tile, code);
+        unsigned long long* at = buf + sample_slot(c, tile, code, 0);
+        if (live && pretest_load(at) > key) atomicMin(at, key);
+        return;
+    }
+    // Software-pipelined over steps: the next step's samples are drawn and their pre-test loads
+    // issued before this step's atomics consume its loads, so the load latency hides behind the
+    // next step's arithmetic.  Samples are still drawn in stream order.
+    uint32_t sa[Step::kDraws], sb[Step::kDraws];
+    bool la[Step::kDraws], lb[Step::kDraws];
+    unsigned long long va[Step::kDraws], vb[Step::kDraws];
     auto draw = [&](int p, uint32_t* sl, bool* lv, unsigned long long* vv) {
-        uint32_t tile[K], code[K];
-        draw_pass<K>(seed, c, tile, code, lv);
+        Step step;
+        step.draw(seed, c, p);
 #pragma unroll
-        for (int j = 0; j < K; ++j) sl[j] = sample_slot(c, tile[j], code[j], p);
+        for (int j = 0; j < Step::kDraws; ++j) {
+            sl[j] = sample_slot(c, step.tile[j], step.code[j], p + Step::step_pass(j));
+            lv[j] = step.live[j];
+        }
 #pragma unroll
-        for (int j = 0; j < K; ++j)
-            vv[j] = lv[j] ? (GPS_SPLAT_PRETEST == 1 ? __ldca(buf + sl[j]) : __ldcg(buf + sl[j])) : 0ull;
+        for (int j = 0; j < Step::kDraws; ++j) vv[j] = lv[j] ? pretest_load(buf + sl[j]) : 0ull;
     };
     auto commit = [&](const uint32_t* sl, const bool* lv, const unsigned long long* vv) {
 #pragma unroll
-        for (int j = 0; j < K; ++j)
+        for (int j = 0; j < Step::kDraws; ++j)
             if (lv[j] && vv[j] > key) atomicMin(buf + sl[j], key);
     };
+    constexpr int s = Step::kPasses;
     if (c.passes > 0) draw(0, sa, la, va);
-    for (int p = 0; p < c.passes; p += 2) {
-        if (p + 1 < c.passes) draw(p + 1, sb, lb, vb);
+    for (int p = 0; p < c.passes; p += 2 * s) {
+        if (p + s < c.passes) draw(p + s, sb, lb, vb);
         commit(sa, la, va);
-        if (p + 1 < c.passes) {
-            if (p + 2 < c.passes) draw(p + 2, sa, la, va);
+        if (p + s < c.passes) {
+            if (p + 2 * s < c.passes) draw(p + 2 * s, sa, la, va);
             commit(sb, lb, vb);
         }
     }
-#else
-    for (int p = 0; p < c.passes; ++p) {
-        uint32_t tile[K], code[K];
-        bool live[K];
-        draw_pass<K>(seed, c, tile, code, live);
-#pragma unroll
-        for (int j = 0; j < K; ++j) {
-            unsigned long long* at = buf + sample_slot(c, tile[j], code[j], p);
-#if GPS_SPLAT_PRETEST
-            if (live[j] && (GPS_SPLAT_PRETEST == 1 ? __ldca(at) : __ldcg(at)) > key) atomicMin(at, key);
-#else
-            if (live[j]) atomicMin(at, key);
-#endif
-        }
-    }
-#endif
 }
 
 // The same samples with the pre-test in shared memory: `nearest` holds the high words (the depth and
@@ -1355,30 +1346,32 @@ __device__ __forceinline__ void splat_point_unbiased_k(uint32_t point, const Spl
 // of kNearPlane words per spp pass.  A sample there whose high word is larger can't change its
 // slot; one whose word is equal or smaller goes on to the buffer.  Samples of other tiles go to
 // the buffer untested.
-constexpr uint32_t kNearPlane = kTileSize * kTileSize + 8;  // (8: planes p and p + 2 on other banks)
+constexpr uint32_t kNearPlane = kTileSize * kTileSize + 8;
 
 template <int K>
 __device__ __forceinline__ void splat_point_in_tile(uint32_t point, const SplatRecord& rec, const FrameConst& fc,
                                                     int frame_seed, uint64_t* __restrict__ buffer, const uint32_t* spread,
                                                     uint32_t* nearest, uint32_t my_tile) {
+    using Step = DrawStep<K>;
     u32x2 seed = make_seed(point, (uint32_t)frame_seed);
     const SampleConst c = sample_const(rec, fc, spread);
     const uint32_t key_high = rec.d.w;
     const unsigned long long key = (unsigned long long)rec.d.z | ((unsigned long long)rec.d.w << 32);
     unsigned long long* buf = reinterpret_cast<unsigned long long*>(buffer);
-    if (splat_wide_point<K>(seed, c, key, buf)) return;
+    if (splat_wide_point(seed, c, K, key, buf)) return;
     my_tile += c.tile_bias;
-    for (int p = 0; p < c.passes; ++p, nearest += kNearPlane) {
-        uint32_t tile[K], code[K], seen[K];
-        bool live[K];
-        draw_pass<K>(seed, c, tile, code, live);
+    for (int p = 0; p < c.passes; p += Step::kPasses, nearest += Step::kPasses * kNearPlane) {
+        Step step;
+        uint32_t seen[Step::kDraws];
+        step.draw(seed, c, p);
 #pragma unroll
-        for (int j = 0; j < K; ++j) seen[j] = live[j] && tile[j] == my_tile ? nearest[code[j]] : 0xFFFFFFFFu;
+        for (int j = 0; j < Step::kDraws; ++j)
+            seen[j] = step.live[j] && step.tile[j] == my_tile ? nearest[step.code[j] + Step::step_pass(j) * kNearPlane] : 0xFFFFFFFFu;
 #pragma unroll
-        for (int j = 0; j < K; ++j)
-            if (live[j] && key_high <= seen[j]) {
-                atomicMin(buf + sample_slot(c, tile[j], code[j], p), key);
-                if (tile[j] == my_tile) atomicMin(nearest + code[j], key_high);
+        for (int j = 0; j < Step::kDraws; ++j)
+            if (step.live[j] && key_high <= seen[j]) {
+                atomicMin(buf + sample_slot(c, step.tile[j], step.code[j], p + Step::step_pass(j)), key);
+                if (step.tile[j] == my_tile) atomicMin(nearest + step.code[j] + Step::step_pass(j) * kNearPlane, key_high);
             }
     }
 }
@@ -1488,7 +1481,7 @@ __device__ __forceinline__ void splat_walk(const SplatArgs& a, const PointOrder&
 }
 
 __device__ __forceinline__ void fill_spread(uint32_t* spread) {
-    if (GPS_SPLAT_MORTON_LUT && threadIdx.x < kTileSize) spread[threadIdx.x] = morton_spread(threadIdx.x);
+    if (threadIdx.x < kTileSize) spread[threadIdx.x] = morton_spread(threadIdx.x);
 }
 
 // K > 0: unbiased splatting with K points per thread per pass; K = 0: any other setting.
