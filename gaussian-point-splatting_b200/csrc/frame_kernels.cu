@@ -1616,11 +1616,64 @@ __device__ __forceinline__ float resolve_pixel(const ResolveArgs& a, int x, int 
     return depth;
 }
 
+// A 12-bit channel as a float by its bits under 2^23 (exact): no conversion instruction.
+__device__ __forceinline__ float channel12(uint32_t c) { return __uint_as_float(0x4B000000u | (c & 0xFFFu)) - 8388608.0f; }
+
+__device__ __forceinline__ float depth_of_key(uint32_t high_word, const ResolveArgs& a) {
+    const float view_depth = view_depth_from_key((uint64_t)(high_word >> 4), a.near_plane, a.far_plane);
+    return gmin(1e9f, view_to_projected_depth(view_depth, a.near_plane, a.far_plane));
+}
+
+// resolve_pixel with the factor known: the kSs x kSs samples of a pass are in flight together, and the
+// nearest depth is that of the smallest key (see resolve_staged_kernel).  Sums in the reference's order.
+template <bool kDepthOnly, int kSs>
+__device__ __forceinline__ float resolve_pixel_ss(const ResolveArgs& a, int x, int y) {
+    const uint32_t idx = (uint32_t)(y * a.width + x);
+    vec3 color = make_v3(0.0f, 0.0f, 0.0f);
+    uint32_t nearest = 0xFFFFFFFFu;
+    const unsigned long long* buf = reinterpret_cast<const unsigned long long*>(a.buffer);
+    auto add = [&](unsigned long long val) {
+        const uint32_t lo = (uint32_t)val, hi = (uint32_t)(val >> 32);
+        nearest = min(nearest, hi);
+        color.x += channel12(__funnelshift_r(lo, hi, 24)) / 255.0f;
+        color.y += channel12(lo >> 12) / 255.0f;
+        color.z += channel12(lo) / 255.0f;
+    };
+    uint32_t at[kSs * kSs];
+#pragma unroll
+    for (int s = 0; s < kSs * kSs; ++s)
+        at[s] = (uint32_t)splat_index(x * kSs + s / kSs, y * kSs + s % kSs, 0, a.num_passes, a.width * kSs, a.height * kSs);
+    if (kDepthOnly || a.num_passes == 1) {  // the order of the samples makes no difference, or is this one
+        for (int p = 0; p < a.num_passes; ++p) {
+            unsigned long long v[kSs * kSs];
+#pragma unroll
+            for (int s = 0; s < kSs * kSs; ++s) v[s] = __ldg(buf + at[s] + p);
+#pragma unroll
+            for (int s = 0; s < kSs * kSs; ++s) {
+                if (kDepthOnly) nearest = min(nearest, (uint32_t)(v[s] >> 32));
+                else add(v[s]);
+            }
+        }
+    } else {
+#pragma unroll
+        for (int s = 0; s < kSs * kSs; ++s)
+#pragma unroll 4
+            for (int p = 0; p < a.num_passes; ++p) add(__ldg(buf + at[s] + p));
+    }
+    if (!kDepthOnly) {
+        const float inv_passes = 1.0f / (float)(a.num_passes * a.ss * a.ss);
+        a.color[3 * idx + 0] = color.x * inv_passes;
+        a.color[3 * idx + 1] = color.y * inv_passes;
+        a.color[3 * idx + 2] = color.z * inv_passes;
+    }
+    return depth_of_key(nearest, a);
+}
+
 // The frame's counters written to pinned host memory by the first block of the final resolve: a
 // copy in the stream after it would hold up the kernels behind it by some microseconds.
 __device__ __forceinline__ void report_counters(const ResolveArgs& a) {
     constexpr uint32_t kWords = sizeof(PassCounters) / 4u;
-    if (!a.report_to || (blockIdx.x | blockIdx.y) != 0u || threadIdx.y != 0u || threadIdx.x >= 2u * kWords) return;
+    if (!a.report_to || (blockIdx.x | blockIdx.y) != 0u || threadIdx.x >= 2u * kWords) return;
     const bool ran = (int)(threadIdx.x / kWords) < a.report_passes;
     reinterpret_cast<volatile uint32_t*>(a.report_to)[threadIdx.x] =
         ran ? reinterpret_cast<const uint32_t*>(a.report_from)[threadIdx.x] : 0u;
@@ -1665,21 +1718,6 @@ __device__ __forceinline__ void hiz_fine_levels(const HizView& c, float depth, i
     }
 }
 
-// Row-major pixels (any supersampling factor).
-template <bool kDepthOnly>
-__global__ void __launch_bounds__(256) resolve_kernel(ResolveArgs a) {
-    previous_kernel_done();
-    report_counters(a);
-    const int x = blockIdx.x * blockDim.x + threadIdx.x;
-    const int y = blockIdx.y * blockDim.y + threadIdx.y;
-    if (x >= a.width || y >= a.height) return;
-    a.depth[y * a.width + x] = resolve_pixel<kDepthOnly>(a, x, y);
-}
-
-// Power-of-two supersampling: the pixels of each 64x64 splat tile in Morton order.  An
-// output pixel's sub-pixels are then one contiguous Morton range, its samples one contiguous
-// run of the buffer, and a warp reads 32 consecutive runs (4 KB at SS 2, 4 spp) instead of
-// runs scattered over a tile.
 __device__ __forceinline__ uint32_t morton_compact(uint32_t a) {
     a &= 0x55555555u;
     a = (a | (a >> 1)) & 0x33333333u;
@@ -1689,6 +1727,29 @@ __device__ __forceinline__ uint32_t morton_compact(uint32_t a) {
     return a;
 }
 
+// Any supersampling factor: 16 x 16 pixels per block, in Morton order so that groups of 64 threads
+// are 8 x 8 pixels (hiz_fine_levels).  kSs: the factor at compile time, whose samples of a pass are then
+// loaded together (0: any), for planes that launch_resolve calls monotone.
+template <bool kDepthOnly, int kSs>
+__global__ void __launch_bounds__(256) resolve_kernel(ResolveArgs a, HizView hiz) {
+    previous_kernel_done();
+    report_counters(a);
+    __shared__ float exchange[8];
+    const int x = (int)(blockIdx.x * 16u + morton_compact(threadIdx.x)), y = (int)(blockIdx.y * 16u + morton_compact(threadIdx.x >> 1));
+    const bool inside = x < a.width && y < a.height;
+    float depth = 0.0f;
+    if (inside) {
+        if constexpr (kSs > 0) depth = resolve_pixel_ss<kDepthOnly, kSs>(a, x, y);
+        else depth = resolve_pixel<kDepthOnly>(a, x, y);
+        if (!(kDepthOnly && a.hiz_fused)) a.depth[y * a.width + x] = depth;
+    }
+    if (a.hiz_fused) hiz_fine_levels(hiz, depth, x, y, a.hiz_min_levels, exchange);
+}
+
+// Power-of-two supersampling: the pixels of each 64x64 splat tile in Morton order.  An
+// output pixel's sub-pixels are then one contiguous Morton range, its samples one contiguous
+// run of the buffer, and a warp reads 32 consecutive runs (4 KB at SS 2, 4 spp) instead of
+// runs scattered over a tile.
 // Pixel of thread g in Morton-tile order.
 __device__ __forceinline__ void morton_pixel(const ResolveArgs& a, uint32_t g, int ss_log2, int& x, int& y) {
     const uint32_t tile_px = (uint32_t)kTileSize >> ss_log2;
@@ -1718,14 +1779,16 @@ __global__ void __launch_bounds__(256) resolve_morton_kernel(ResolveArgs a, HizV
 
 // Staged variant: a block's pixels are consecutive in Morton-tile order, so their samples are
 // one contiguous run of the buffer (px_per_block x SS*SS*spp entries, at most 48 KB), which the
-// block reads with coalesced 16-byte loads.  Used when SS*SS*spp is a power of two in 2..128.
+// block reads with coalesced 16-byte loads.  Used for SS 1, 2, 4, 8 with 1 to 8 or a power of two of
+// samples per pixel and 2 to 128 samples in all.
 //   depth only: of every entry pair the smaller high word goes to shared memory; a pixel's depth
 //     is that of its smallest key.  The conversion to NDC does not decrease with the key (every
 //     step of it rounds monotonically for 0 < near < far; checked over all 2^28 keys for 40 pairs
 //     of planes between 1e-6 and 1e9, and launch_resolve keeps to that range), so the smallest
 //     key's depth is the smallest depth, bit for bit.
 //   final: the run itself goes to shared memory, two pad words after each pixel's samples to keep
-//     a warp's 16-byte reads on different banks; the 12-bit channels become floats by their bits
+//     a warp's 16-byte reads on different banks (an odd number of words per pixel where the run is no
+//     power of two and read word by word); the 12-bit channels become floats by their bits
 //     under 2^23 (exact), which keeps them off the conversion unit.
 // The kernel was bound by instructions, not by the 8 bytes per sample: with run-time sizes, a
 // division per pixel and 64-bit indices it took 40 (depth) and 63 (final) instructions per sample
@@ -1733,29 +1796,25 @@ __global__ void __launch_bounds__(256) resolve_morton_kernel(ResolveArgs a, HizV
 // tile by tiles_y:
 // 28 and 44, and 1M town at 4K, 2 spp: 111 -> 88 us (depth; the 531 MB take 82 at the copy rate) and
 // 175 -> 136 us, the frame 995 -> 943; 500k town at 720p, 1 spp: 139 -> 127.
-constexpr int kResolveMaxRunLog2 = 7;
-// 64 pixels per block (155 us for both resolves at 1080p; 32 196, 256 162), 32 at 128 samples each
-__host__ __device__ constexpr uint32_t resolve_pixels(int run_log2) { return run_log2 <= 6 ? 64u : 32u; }
-__host__ __device__ constexpr int resolve_blocks_log2(int ss_log2, int run_log2) {  // blocks per tile
-    return 2 * (kTileBits - ss_log2) - (run_log2 <= 6 ? 6 : 5);
+constexpr int kResolveMaxRun = 128;
+// 64 pixels per block (155 us for both resolves at 1080p; 32 196, 256 162), 32 above 64 samples each
+__host__ __device__ constexpr uint32_t resolve_pixels(int run) { return run <= 64 ? 64u : 32u; }
+__host__ __device__ constexpr int resolve_blocks_log2(int ss_log2, int run) {  // blocks per tile
+    return 2 * (kTileBits - ss_log2) - (run <= 64 ? 6 : 5);
 }
 
-__device__ __forceinline__ float channel12(uint32_t c) { return __uint_as_float(0x4B000000u | (c & 0xFFFu)) - 8388608.0f; }
-
-__device__ __forceinline__ float depth_of_key(uint32_t high_word, const ResolveArgs& a) {
-    const float view_depth = view_depth_from_key((uint64_t)(high_word >> 4), a.near_plane, a.far_plane);
-    return gmin(1e9f, view_to_projected_depth(view_depth, a.near_plane, a.far_plane));
-}
-
-template <bool kDepthOnly, int kSsLog2, int kRunLog2>
-__global__ void __launch_bounds__(resolve_pixels(kRunLog2)) resolve_staged_kernel(ResolveArgs a, HizView hiz) {
+template <bool kDepthOnly, int kSsLog2, int kPasses>
+__global__ void __launch_bounds__(resolve_pixels(kPasses << (2 * kSsLog2))) resolve_staged_kernel(ResolveArgs a, HizView hiz) {
     previous_kernel_done();
     report_counters(a);
-    constexpr uint32_t kPx = resolve_pixels(kRunLog2), kRun = 1u << kRunLog2, kHalf = kRun / 2u;
-    constexpr int kBlocksLog2 = resolve_blocks_log2(kSsLog2, kRunLog2);
+    constexpr uint32_t kRun = (uint32_t)kPasses << (2 * kSsLog2), kHalf = kRun / 2u, kPx = resolve_pixels((int)kRun);
+    constexpr int kBlocksLog2 = resolve_blocks_log2(kSsLog2, (int)kRun);
     constexpr uint32_t kTilePxLog2 = (uint32_t)(kTileBits - kSsLog2);
-    // a pad word (depth only: 4 bytes, final: 16) follows the kHalf words of each pixel
-    __shared__ __align__(16) uint32_t stage[kPx * (kHalf + 1u) * (kDepthOnly ? 1u : 4u)];
+    constexpr bool kPow2 = (kRun & (kRun - 1u)) == 0u;
+    // words per pixel.  A power of two: pairs of entries and a pad (depth only: 4 bytes a pair, final:
+    // 16).  Otherwise entries, an odd number of places (4 or 8 bytes an entry)
+    constexpr uint32_t kStride = kPow2 ? kHalf + 1u : kRun | 1u;
+    __shared__ __align__(16) uint32_t stage[kPx * kStride * (kPow2 ? (kDepthOnly ? 1u : 4u) : (kDepthOnly ? 1u : 2u))];
     __shared__ float exchange[2];
     // blocks take the buffer from its end: the splat walks screen bins (buffer tiles) in
     // ascending order, so the tiles it touched last are the ones still in L2
@@ -1763,15 +1822,40 @@ __global__ void __launch_bounds__(resolve_pixels(kRunLog2)) resolve_staged_kerne
     const uint32_t tx = bx >> kBlocksLog2, sub = bx & ((1u << kBlocksLog2) - 1u);
     const uint32_t tile = ty * (gridDim.x >> kBlocksLog2) + tx, t = threadIdx.x;
     const ulonglong2* src = reinterpret_cast<const ulonglong2*>(a.buffer) +
-                            ((uint64_t)((tile << kBlocksLog2) + sub) * (kPx * kHalf) + t);
+                            ((uint64_t)((tile << kBlocksLog2) + sub) * (kPx * kRun / 2u) + t);
     const int x = (int)((tx << kTilePxLog2) + morton_compact(sub * kPx) + morton_compact(t));
     const int y = (int)((ty << kTilePxLog2) + morton_compact((sub * kPx) >> 1) + morton_compact(t >> 1));
     const bool inside = x < a.width && y < a.height;
     uint32_t nearest = 0xFFFFFFFFu;
-    if (kDepthOnly) {
+    constexpr uint32_t kLoads = kRun / 2u;  // 16-byte loads per thread (kRun entries each, kPx even)
+    if constexpr (!kPow2) {
+        // entry e of the block's run: place e % kRun of pixel e / kRun
+        static_assert(kPx == 64u, "runs that are no power of two stay below 64 samples");
+        uint64_t* words = reinterpret_cast<uint64_t*>(stage);
+#pragma unroll 8
+        for (uint32_t k = 0; k < (kRun + 1u) / 2u; ++k) {
+            const uint32_t i = k * kPx + t;  // pair
+            if (i >= kPx * kRun / 2u) break;
+            const ulonglong2 q = __ldcs(src + k * kPx);
+            const uint32_t e0 = 2u * i, e1 = e0 + 1u;
+            const uint32_t d0 = e0 / kRun * kStride + e0 % kRun, d1 = e1 / kRun * kStride + e1 % kRun;
+            if (kDepthOnly) {
+                stage[d0] = (uint32_t)(q.x >> 32);
+                stage[d1] = (uint32_t)(q.y >> 32);
+            } else {
+                words[d0] = q.x;
+                words[d1] = q.y;
+            }
+        }
+        __syncthreads();
+        if (kDepthOnly) {
+#pragma unroll
+            for (uint32_t k = 0; k < kRun; ++k) nearest = min(nearest, stage[t * kStride + k]);
+        }
+    } else if (kDepthOnly) {
         uint32_t* put = stage + t + t / kHalf;
 #pragma unroll 8
-        for (uint32_t k = 0; k < kHalf; ++k) {
+        for (uint32_t k = 0; k < kLoads; ++k) {
             const uint4 q = __ldcs(reinterpret_cast<const uint4*>(src + k * kPx));
             put[k * kPx + k * kPx / kHalf] = min(q.y, q.w);
         }
@@ -1782,9 +1866,11 @@ __global__ void __launch_bounds__(resolve_pixels(kRunLog2)) resolve_staged_kerne
     } else {
         ulonglong2* put = reinterpret_cast<ulonglong2*>(stage) + t + t / kHalf;
 #pragma unroll 8
-        for (uint32_t k = 0; k < kHalf; ++k) put[k * kPx + k * kPx / kHalf] = __ldcs(src + k * kPx);
+        for (uint32_t k = 0; k < kLoads; ++k) put[k * kPx + k * kPx / kHalf] = __ldcs(src + k * kPx);
         __syncthreads();
-        const uint64_t* mine = reinterpret_cast<const uint64_t*>(stage) + t * (kRun + 2u);
+    }
+    if (!kDepthOnly) {
+        const uint64_t* mine = reinterpret_cast<const uint64_t*>(stage) + t * (kPow2 ? kRun + 2u : kStride);
         vec3 color = make_v3(0.0f, 0.0f, 0.0f);
         auto add = [&](uint64_t val) {
             const uint32_t lo = (uint32_t)val, hi = (uint32_t)(val >> 32);
@@ -1793,17 +1879,17 @@ __global__ void __launch_bounds__(resolve_pixels(kRunLog2)) resolve_staged_kerne
             color.y += channel12(lo >> 12) / 255.0f;
             color.z += channel12(lo) / 255.0f;
         };
-        constexpr uint32_t kPasses = kRun >> (2 * kSsLog2);
 #pragma unroll
         for (int dx = 0; dx < (1 << kSsLog2); ++dx)
 #pragma unroll
             for (int dy = 0; dy < (1 << kSsLog2); ++dy) {
-                const uint64_t* at = mine + morton_encode((uint32_t)dx, (uint32_t)dy) * kPasses;
-                if constexpr (kPasses == 1u) {
-                    add(*at);
+                const uint64_t* at = mine + morton_encode((uint32_t)dx, (uint32_t)dy) * (uint32_t)kPasses;
+                if constexpr (!kPow2 || kPasses == 1) {
+#pragma unroll 8
+                    for (int p = 0; p < kPasses; ++p) add(at[p]);
                 } else {
 #pragma unroll 8
-                    for (uint32_t p = 0; p < kPasses; p += 2u) {
+                    for (int p = 0; p < kPasses; p += 2) {
                         const ulonglong2 q = *reinterpret_cast<const ulonglong2*>(at + p);
                         add(q.x);
                         add(q.y);
@@ -1828,9 +1914,8 @@ __global__ void __launch_bounds__(resolve_pixels(kRunLog2)) resolve_staged_kerne
 // ---------------------------------------------------------------------------------
 // Hi-Z chain (depth_mip_chain.cu:7-67)
 // ---------------------------------------------------------------------------------
-// The whole chain in one launch, for views whose resolve does not write the fine levels (a
-// supersampling factor that is no power of two, runs of 128 samples and more, images of up to
-// four pixels).  A 16x16-thread block covers a 64x64 tile of the depth image:
+// The whole chain in one launch, for views whose resolve does not write the fine levels (128 samples
+// a pixel, images of up to four pixels).  A 16x16-thread block covers a 64x64 tile of the depth image:
 // each thread copies its 4x4 texels into the finest level and reduces them in registers to
 // the next two levels (2x2, then 1), the block reduces its 16x16 results through four more
 // levels in shared memory, and the block that finishes last (a counter, no waiting) reduces
@@ -2482,55 +2567,57 @@ void launch_clear(uint64_t* buf, uint64_t entries, uint64_t value, cudaStream_t 
     if (entries & 1) cudaMemcpyAsync(buf + entries - 1, &buf[0], 8, cudaMemcpyDeviceToDevice, stream);
 }
 
-template <bool kDepthOnly, int kSsLog2, int kRunLog2>
-void launch_resolve_staged(const ResolveArgs& a, const HizView& hiz, dim3 tiles, int ss_log2, int run_log2,
-                           cudaStream_t stream) {
-    if constexpr (kSsLog2 <= 3 && kRunLog2 <= kResolveMaxRunLog2) {
-        if (ss_log2 == kSsLog2 && run_log2 == kRunLog2) {
-            launch_k(resolve_staged_kernel<kDepthOnly, kSsLog2, kRunLog2>,
-                     dim3(tiles.x << resolve_blocks_log2(kSsLog2, kRunLog2), tiles.y), resolve_pixels(kRunLog2), 0, stream, a, hiz);
-        } else if (kRunLog2 < kResolveMaxRunLog2) {
-            launch_resolve_staged<kDepthOnly, kSsLog2, kRunLog2 + 1>(a, hiz, tiles, ss_log2, run_log2, stream);
-        } else {
-            launch_resolve_staged<kDepthOnly, kSsLog2 + 1, (kSsLog2 ? 2 * kSsLog2 + 2 : 2)>(a, hiz, tiles, ss_log2, run_log2, stream);
+// The staged kernel of these sizes, if there is one: kPasses runs through 1..8 and the powers of two.
+template <bool kDepthOnly, int kSsLog2, int kPasses = 1>
+bool launch_resolve_staged(const ResolveArgs& a, const HizView& hiz, dim3 tiles, int ss_log2, cudaStream_t stream) {
+    constexpr int kRun = kPasses << (2 * kSsLog2);
+    if constexpr (kSsLog2 > 3) {
+        return false;
+    } else if constexpr (kRun > kResolveMaxRun) {
+        return launch_resolve_staged<kDepthOnly, kSsLog2 + 1>(a, hiz, tiles, ss_log2, stream);
+    } else {
+        constexpr bool kPow2 = (kRun & (kRun - 1)) == 0;
+        if constexpr (kRun > 1 && (kPow2 || kRun < 64)) {
+            if (ss_log2 == kSsLog2 && a.num_passes == kPasses) {
+                launch_k(resolve_staged_kernel<kDepthOnly, kSsLog2, kPasses>,
+                         dim3(tiles.x << resolve_blocks_log2(kSsLog2, kRun), tiles.y), resolve_pixels(kRun), 0, stream, a, hiz);
+                return true;
+            }
         }
+        return launch_resolve_staged<kDepthOnly, kSsLog2, (kPasses < 8 ? kPasses + 1 : kPasses * 2)>(a, hiz, tiles, ss_log2, stream);
     }
+}
+
+template <bool kDepthOnly>
+void launch_resolve_any(const ResolveArgs& a, const HizView& h, bool monotone, int ss_log2, cudaStream_t stream) {
+    if (ss_log2 >= 0) {
+        const dim3 tiles((unsigned)((a.width * a.ss + kTileSize - 1) >> kTileBits),
+                         (unsigned)((a.height * a.ss + kTileSize - 1) >> kTileBits));
+        if (monotone && launch_resolve_staged<kDepthOnly, 0>(a, h, tiles, ss_log2, stream)) return;
+        const uint64_t threads = ((uint64_t)tiles.x * tiles.y) << (2 * (kTileBits - ss_log2));
+        launch_k(resolve_morton_kernel<kDepthOnly>, (unsigned)((threads + 255) / 256), 256, 0, stream, a, h, ss_log2);
+        return;
+    }
+    const dim3 grid((a.width + 15) / 16, (a.height + 15) / 16);
+    if (monotone && a.ss == 3) launch_k(resolve_kernel<kDepthOnly, 3>, grid, 256, 0, stream, a, h);
+    else launch_k(resolve_kernel<kDepthOnly, 0>, grid, 256, 0, stream, a, h);
 }
 
 int launch_resolve(const ResolveArgs& args, const HizView* hiz, bool depth_only, cudaStream_t stream) {
     ResolveArgs a = args;
-    const HizView none{};
     int ss_log2 = -1;
     for (int l = 0; l <= 3; ++l)
         if (a.ss == (1 << l)) ss_log2 = l;
-    a.hiz_fused = 0;
-    if (ss_log2 >= 0) {
-        const dim3 tiles((unsigned)((a.width * a.ss + kTileSize - 1) >> kTileBits),
-                         (unsigned)((a.height * a.ss + kTileSize - 1) >> kTileBits));
-        const uint32_t run = (uint32_t)(a.ss * a.ss * a.num_passes);
-        int run_log2 = 0;
-        for (int l = 1; l <= kResolveMaxRunLog2; ++l)
-            if (run == (1u << l)) run_log2 = l;
-        // staged: planes for which a key's depth is monotone (through zero or past the float
-        // range it is not); the fine Hi-Z levels need groups of 64 pixels, a chain of four levels
-        const bool staged = run_log2 > 0 && a.near_plane >= 1.0e-6f && a.far_plane <= 1.0e9f;
-        a.hiz_fused = hiz && hiz->levels >= 4 && (!staged || resolve_pixels(run_log2) == 64u) ? 1 : 0;
-        const HizView& h = a.hiz_fused ? *hiz : none;
-        if (staged) {
-            if (depth_only) launch_resolve_staged<true, 0, 1>(a, h, tiles, ss_log2, run_log2, stream);
-            else launch_resolve_staged<false, 0, 1>(a, h, tiles, ss_log2, run_log2, stream);
-        } else {
-            const uint64_t threads = ((uint64_t)tiles.x * tiles.y) << (2 * (kTileBits - ss_log2));
-            const unsigned grid = (unsigned)((threads + 255) / 256);
-            if (depth_only) launch_k(resolve_morton_kernel<true>, grid, 256, 0, stream, a, h, ss_log2);
-            else launch_k(resolve_morton_kernel<false>, grid, 256, 0, stream, a, h, ss_log2);
-        }
-    } else {
-        dim3 block(16, 16);
-        dim3 grid((a.width + 15) / 16, (a.height + 15) / 16);
-        if (depth_only) launch_k(resolve_kernel<true>, grid, block, 0, stream, a);
-        else launch_k(resolve_kernel<false>, grid, block, 0, stream, a);
-    }
+    // planes for which a key's depth is monotone (through zero or past the float range it is not)
+    const bool monotone = a.near_plane >= 1.0e-6f && a.far_plane <= 1.0e9f;
+    // the fine Hi-Z levels need a chain of four levels and groups of 64 pixels, which the blocks of
+    // more than 64 samples a pixel are not
+    const int run = a.ss * a.ss * a.num_passes;
+    const bool small_blocks = ss_log2 >= 0 && monotone && run == kResolveMaxRun;
+    a.hiz_fused = hiz && hiz->levels >= 4 && !small_blocks ? 1 : 0;
+    const HizView h = a.hiz_fused ? *hiz : HizView{};
+    if (depth_only) launch_resolve_any<true>(a, h, monotone, ss_log2, stream);
+    else launch_resolve_any<false>(a, h, monotone, ss_log2, stream);
     return a.hiz_fused;
 }
 

@@ -49,7 +49,9 @@ def _chain(depth, min_levels):
     (8, 8, 2, 4, 0), (9, 7, 2, 4, 2), (65, 33, 2, 4, 5),         # one group of 64 pixels and its edges
     (129, 127, 1, 4, 0), (131, 70, 1, 1, 3), (257, 19, 2, 3, 0),  # 16 x 16-texel blocks; unstaged runs
     (67, 35, 4, 4, 0), (67, 35, 4, 8, 1), (40, 23, 8, 1, 0),     # 64- and 32-pixel blocks, one group a tile
-    (97, 61, 3, 2, 0), (1030, 517, 2, 2, 0),                     # row-major; levels past shared memory
+    (97, 61, 3, 2, 0), (37, 50, 3, 1, 2), (33, 31, 5, 1, 0),     # factors that are no power of two
+    (70, 41, 2, 5, 0), (90, 33, 4, 3, 0), (41, 90, 1, 7, 0), (21, 17, 2, 9, 0),  # runs that are none
+    (1030, 517, 2, 2, 0),                                        # levels past shared memory
 ])
 def test_resolve_and_hiz_against_numpy(width, height, ss, spp, min_levels):
     raw = synth.cube(4000, seed=9)
