@@ -73,6 +73,18 @@ struct FrameConst {
     int width, height;
 };
 
+// The splat buffer's clear, taken along by a frame's first kernel (pairs 0: no clear).
+struct ClearArgs {
+    ulonglong2* buffer;
+    uint64_t pairs;
+    unsigned long long value;
+};
+
+// Scenes of up to this many Gaussians (in blocks of four) have their block cull inside the preprocess:
+// a launch less, where a warp has at most two chunks to test and to work on.
+constexpr uint32_t kSelfCullChunks = 2;
+constexpr uint32_t kSelfCullGaussians = 32u * 4736u * kSelfCullChunks;  // 4736 warps: 4 blocks on 148 SMs
+
 // The block cull of one pass and, in a frame's first launch, the splat buffer's clear.
 struct CullArgs {
     BlockView b;
@@ -83,9 +95,7 @@ struct CullArgs {
     uint32_t* mask_pair[2];      // the culled chunks' words are zeroed in the one *mask_iter selects
     const uint32_t* mask_iter;
     int second_pass;             // same camera as the pass before: b.outside holds
-    ulonglong2* clear;
-    uint64_t clear_pairs;        // 0: no clear
-    unsigned long long clear_value;
+    ClearArgs clear;
     uint32_t cull_blocks;        // set by launch_cull
     uint32_t words_per_block;
 };
@@ -103,6 +113,9 @@ struct PreprocessArgs {
     BlockView blocks;
     const uint32_t* chunk_list;   // 32-Gaussian chunks with a visible block (null: every chunk)
     const uint32_t* chunk_count;
+    int cull_here;                // test the chunks' nodes here (no list; per_block 4, kSelfCullGaussians)
+    ClearArgs clear;              // with the frame's first pass, unless the cull brought it
+    uint32_t blocks_here;         // set by the launch: the blocks after them clear
     int immediate_threshold;      // > 0: splat Gaussians of <= this many points in the preprocess
     uint64_t* buffer;             // splat buffer (immediate splatting only)
     // When mask_iter is set, mask_cur / mask_prev are mask_pair[it & 1] / mask_pair[(it + 1) & 1]

@@ -407,9 +407,17 @@ BlockView block_view(gps_renderer* r) {
     return b;
 }
 
-// The block cull and chunk list of a pass; the frame's first launch, which also clears the splat
-// buffer, when `clear_value` is given.
-void cull_blocks(gps_renderer* r, const FrameConst& fc, const unsigned long long* clear_value, cudaStream_t st) {
+// Where a pass's block cull happens.
+enum CullWhere { kCullNone, kCullInPreprocess, kCullLaunch };
+
+CullWhere cull_where(const gps_renderer* r, const FrameConst& fc) {
+    if (!fc.enable_hier || !r->scene->block_count || r->n == 0) return kCullNone;
+    return r->scene->per_block == 4 && r->n <= kSelfCullGaussians && r->s.immediate_splat_threshold <= 0 ? kCullInPreprocess
+                                                                                                        : kCullLaunch;
+}
+
+// The block cull and chunk list of a pass (the first with the splat buffer's clear).
+void cull_blocks(gps_renderer* r, const FrameConst& fc, const ClearArgs* clear, cudaStream_t st) {
     CullArgs a{};
     a.b = block_view(r);
     a.fc = fc;
@@ -419,12 +427,8 @@ void cull_blocks(gps_renderer* r, const FrameConst& fc, const unsigned long long
     a.mask_pair[0] = r->mask[0].get();
     a.mask_pair[1] = r->mask[1].get();
     a.mask_iter = r->mask_iter.get();
-    a.second_pass = clear_value ? 0 : 1;
-    if (clear_value) {
-        a.clear = reinterpret_cast<ulonglong2*>(r->buffer.get());
-        a.clear_pairs = r->entries / 2;  // a multiple of 4096 entries
-        a.clear_value = *clear_value;
-    }
+    a.second_pass = clear ? 0 : 1;
+    if (clear) a.clear = *clear;
     launch_cull(a, st);
 }
 
@@ -438,10 +442,12 @@ bool screen_binned(const gps_renderer* r) {
     return GPS_SPLAT_BINNED != 0 && r->entries * sizeof(uint64_t) >= kBinMinBufferBytes;
 }
 
-void render_pass(gps_renderer* r, const FrameConst& fc, int frame, bool first, cudaStream_t st) {
+// `clear`: the preprocess clears the splat buffer on the way (null: that is done).
+void render_pass(gps_renderer* r, const FrameConst& fc, int frame, bool first, const ClearArgs* clear, cudaStream_t st) {
     const int frame_seed = 4 * frame + (first ? 0 : 2);
     BlockView blocks = block_view(r);
-    const bool listed = fc.enable_hier && blocks.node_count;
+    const CullWhere cull = cull_where(r, fc);
+    const bool listed = cull == kCullLaunch;
     if (listed && !first) {  // (the first pass's cull came with the clear)
         r->timer.mark(kStCull, st);
         cull_blocks(r, fc, nullptr, st);
@@ -462,6 +468,8 @@ void render_pass(gps_renderer* r, const FrameConst& fc, int frame, bool first, c
     pa.blocks = blocks;
     pa.chunk_list = listed ? r->chunk_list.get() : nullptr;
     pa.chunk_count = listed ? r->chunk_count.get() : nullptr;
+    pa.cull_here = cull == kCullInPreprocess ? 1 : 0;
+    if (clear) pa.clear = *clear;
     pa.immediate_threshold = r->s.immediate_splat_threshold;
     pa.buffer = r->buffer.get();
     pa.loaded = r->loaded.get();
@@ -986,12 +994,18 @@ gps_status render_frame_impl(gps_renderer* r, const gps_camera* cam, float* d_im
     const uint64_t bg = 0xFFFFFFF000000000ull |
                         rgb_to_36bits(make_v3(r->s.background[0], r->s.background[1], r->s.background[2]));
     r->frame_launches = 0;
-    r->timer.mark(kStClear, st);
-    const unsigned long long clear_value = bg;
-    if (fc.enable_hier && r->scene->block_count && r->n > 0) cull_blocks(r, fc, &clear_value, st);
-    else launch_clear(r->buffer.get(), r->entries, bg, st);
-    count_launch(r, kStClear);
-    if (r->n > 0) render_pass(r, fc, cam->frame, true, st);
+    // the clear goes with the frame's first kernel: the block cull's or, without one, the preprocess,
+    // unless that splats into the buffer itself
+    const ClearArgs clear{reinterpret_cast<ulonglong2*>(r->buffer.get()), r->entries / 2, bg};  // (a multiple of 4096 entries)
+    const bool culls = cull_where(r, fc) == kCullLaunch;
+    const bool with_preprocess = !culls && r->n > 0 && r->s.immediate_splat_threshold <= 0;
+    if (!with_preprocess) {
+        r->timer.mark(kStClear, st);
+        if (culls) cull_blocks(r, fc, &clear, st);
+        else launch_clear(r->buffer.get(), r->entries, bg, st);
+        count_launch(r, kStClear);
+    }
+    if (r->n > 0) render_pass(r, fc, cam->frame, true, with_preprocess ? &clear : nullptr, st);
     ResolveArgs ra{};
     ra.buffer = r->buffer.get();
     ra.color = d_image;
@@ -1017,7 +1031,7 @@ gps_status render_frame_impl(gps_renderer* r, const gps_camera* cam, float* d_im
         count_launch(r, kStResolve);
         build_hiz(fine);
         if (r->n > 0) {
-            render_pass(r, fc, cam->frame, false, st);
+            render_pass(r, fc, cam->frame, false, nullptr, st);
             r->second_pass_last = true;
         }
     }
