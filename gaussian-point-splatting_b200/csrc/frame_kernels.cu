@@ -281,9 +281,10 @@ __global__ void super_bounds_kernel(const float4* __restrict__ nodes, uint32_t n
 // Preprocess (gaussian_point_splatting.cu:17-65 + 147-307)
 // ---------------------------------------------------------------------------------
 __device__ __forceinline__ void splat_samples_biased(u32x2& seed, const SplatRecord& rec, const FrameConst& fc,
-                                                     uint64_t* __restrict__ buffer);
+                                                     uint64_t* __restrict__ buffer, int first, int last);
 __device__ __forceinline__ void splat_samples_unbiased(u32x2& seed, const SplatRecord& rec, const FrameConst& fc,
-                                                       uint64_t* __restrict__ buffer);
+                                                       uint64_t* __restrict__ buffer, const uint32_t* spread, int first,
+                                                       int last);
 
 // One Gaussian: true if it splats this pass (record and count written).  kImmediate: a
 // Gaussian of at most a.immediate_threshold points is splatted here instead, its samples
@@ -391,9 +392,10 @@ __device__ __forceinline__ bool preprocess_one(const PreprocessArgs& a, const Sc
                            (uint32_t)key, (uint32_t)(key >> 32));
         if constexpr (kImmediate) {
             if ((int)num_points <= a.immediate_threshold) {
+                const int samples = fc.num_passes * fc.k_points;
                 for (uint32_t pt = 0; pt < num_points; ++pt) {
-                    if (fc.use_unbiased) splat_samples_unbiased(seed, rec, fc, a.buffer);
-                    else splat_samples_biased(seed, rec, fc, a.buffer);
+                    if (fc.use_unbiased) splat_samples_unbiased(seed, rec, fc, a.buffer, nullptr, 0, samples);
+                    else splat_samples_biased(seed, rec, fc, a.buffer, 0, samples);
                 }
                 a.counts[idx] = 0;
                 break;
@@ -976,7 +978,7 @@ __device__ __forceinline__ void atomic_add_color(unsigned long long* address, un
     } while (assumed != old);
 }
 
-// Biased mode (use_unbiased_2d_splatting = false): one point's samples from `seed` onwards (the seed
+// Biased mode (use_unbiased_2d_splatting = false): one point's samples first..last - 1 (the seed
 // advances, as splatGaussianPoint's does), kBiasedBatch at a time: their slots, then their
 // pre-test loads together, then the additions, which start from the loaded values.  A load that
 // missed an addition made since costs a second compare-and-swap, no more: a slot's depth only
@@ -985,7 +987,7 @@ __device__ __forceinline__ void atomic_add_color(unsigned long long* address, un
 constexpr int kBiasedBatch = 4;
 
 __device__ __forceinline__ void splat_samples_biased(u32x2& seed, const SplatRecord& rec, const FrameConst& fc,
-                                                     uint64_t* __restrict__ buffer) {
+                                                     uint64_t* __restrict__ buffer, int first, int last) {
     const vec2 pixel_mean = make_v2(rec.a.x, rec.a.y);
     const float c0 = rec.a.z, c1 = rec.a.w, c2 = rec.b.x;
     const vec3 conic = make_v3(rec.b.y, rec.b.z, rec.b.w);
@@ -995,17 +997,16 @@ __device__ __forceinline__ void splat_samples_biased(u32x2& seed, const SplatRec
     const uint64_t key = (uint64_t)rec.d.z | ((uint64_t)rec.d.w << 32);
     const uint64_t view_depth_bits = key & kDepthMask;
     const int k = fc.k_points;
-    const int samples = fc.num_passes * k;
     unsigned long long* buf = reinterpret_cast<unsigned long long*>(buffer);
-    int pass = 0, j = 0;  // sample s0 + b is draw j of spp pass `pass`
-    for (int s0 = 0; s0 < samples; s0 += kBiasedBatch) {
+    int pass = first / k, j = first - pass * k;  // sample s0 + b is draw j of spp pass `pass`
+    for (int s0 = first; s0 < last; s0 += kBiasedBatch) {
         int slot[kBiasedBatch];
         bool live[kBiasedBatch];
 #pragma unroll
         for (int b = 0; b < kBiasedBatch; ++b) {
             live[b] = false;
             slot[b] = 0;
-            if (s0 + b >= samples) continue;
+            if (s0 + b >= last) continue;
             vec2 u = pcg2d(seed);
             vec2 xy = box_muller(u.x, u.y);
             vec2 pixel = make_v2(pixel_mean.x + c0 * xy.x, pixel_mean.y + c1 * xy.x + c2 * xy.y);
@@ -1031,12 +1032,6 @@ __device__ __forceinline__ void splat_samples_biased(u32x2& seed, const SplatRec
         for (int b = 0; b < kBiasedBatch; ++b)
             if (live[b] && (uint64_t)seen[b] > view_depth_bits) atomic_add_color(buf + slot[b], seen[b], key);
     }
-}
-
-__device__ __forceinline__ void splat_point_biased(uint32_t point, const SplatRecord& rec, const FrameConst& fc,
-                                                   int frame_seed, uint64_t* __restrict__ buffer) {
-    u32x2 seed = make_seed(point, (uint32_t)frame_seed);
-    splat_samples_biased(seed, rec, fc, buffer);
 }
 
 // Unbiased mode (the default).  A sample's slot is loaded before its atomicMin is issued (the
@@ -1267,14 +1262,13 @@ struct DrawStep {
 };
 
 // A point that draw_pair leaves out: one sample after the other, untested.  False for any other.
-__device__ __forceinline__ bool splat_wide_point(u32x2& seed, const SampleConst& c, int k, unsigned long long key,
-                                                 unsigned long long* buf) {
+__device__ __forceinline__ bool splat_wide_point(u32x2& seed, const SampleConst& c, int k, int first, int last,
+                                                 unsigned long long key, unsigned long long* buf) {
     if (!wide_sample(c)) return false;
-    for (int p = 0; p < c.passes; ++p)
-        for (int j = 0; j < k; ++j) {
-            uint32_t tile, code;
-            if (draw_sample(seed, c, tile, code)) atomicMin(buf + sample_slot(c, tile, code, p), key);
-        }
+    for (int i = first; i < last; ++i) {
+        uint32_t tile, code;
+        if (draw_sample(seed, c, tile, code)) atomicMin(buf + sample_slot(c, tile, code, i / k), key);
+    }
     return true;
 }
 
@@ -1282,24 +1276,25 @@ __device__ __forceinline__ unsigned long long pretest_load(const unsigned long l
     return GPS_SPLAT_PRETEST == 1 ? __ldca(at) : GPS_SPLAT_PRETEST == 2 ? __ldcg(at) : ~0ull;
 }
 
-// One point's samples from `seed` onwards, any k (the seed advances, as splatGaussianPoint's does).
+// One point's samples first..last - 1 of its k * num_passes, any k (the seed advances from the first
+// sample's to the one after the last, as splatGaussianPoint's does).
 __device__ __forceinline__ void splat_samples_unbiased(u32x2& seed, const SplatRecord& rec, const FrameConst& fc,
-                                                       uint64_t* __restrict__ buffer) {
-    const SampleConst c = sample_const(rec, fc, nullptr);
+                                                       uint64_t* __restrict__ buffer, const uint32_t* spread, int first, int last) {
+    const SampleConst c = sample_const(rec, fc, spread);
     const unsigned long long key = (unsigned long long)rec.d.z | ((unsigned long long)rec.d.w << 32);
     unsigned long long* buf = reinterpret_cast<unsigned long long*>(buffer);
-    const int k = fc.k_points, samples = fc.num_passes * k;
-    if (splat_wide_point(seed, c, k, key, buf)) return;
-    int p = 0, j = 0;  // sample s0 + b is draw j of spp pass p
-    for (int s0 = 0; s0 < samples; s0 += 4) {
+    const int k = fc.k_points;
+    if (splat_wide_point(seed, c, k, first, last, key, buf)) return;
+    int p = first / k, j = first - p * k;  // sample s0 + b is draw j of spp pass p
+    for (int s0 = first; s0 < last; s0 += 4) {
         uint32_t tile[4], code[4], slot[4];
         bool live[4];
 #pragma unroll
         for (int b = 0; b < 4; b += 2) {
             live[b] = live[b + 1] = false;
             tile[b] = tile[b + 1] = code[b] = code[b + 1] = 0u;
-            if (s0 + b + 1 < samples) draw_pair(seed, c, tile + b, code + b, live + b);
-            else if (s0 + b < samples) live[b] = draw_one(seed, c, tile[b], code[b]);
+            if (s0 + b + 1 < last) draw_pair(seed, c, tile + b, code + b, live + b);
+            else if (s0 + b < last) live[b] = draw_one(seed, c, tile[b], code[b]);
         }
         unsigned long long seen[4];
 #pragma unroll
@@ -1317,10 +1312,11 @@ __device__ __forceinline__ void splat_samples_unbiased(u32x2& seed, const SplatR
     }
 }
 
-__device__ __forceinline__ void splat_point_unbiased(uint32_t point, const SplatRecord& rec, const FrameConst& fc,
-                                                     int frame_seed, uint64_t* __restrict__ buffer) {
+// The seed of a point's sample `first`: every sample is one step of the generator.
+__device__ __forceinline__ u32x2 sample_seed(uint32_t point, int frame_seed, int first) {
     u32x2 seed = make_seed(point, (uint32_t)frame_seed);
-    splat_samples_unbiased(seed, rec, fc, buffer);
+    for (int i = 0; i < first; ++i) seed = pcg2d_step(seed);
+    return seed;
 }
 
 // The same samples with K known at compile time.
@@ -1333,7 +1329,7 @@ __device__ __forceinline__ void splat_point_unbiased_k(uint32_t point, const Spl
     const SampleConst c = sample_const(rec, fc, spread);
     const unsigned long long key = (unsigned long long)rec.d.z | ((unsigned long long)rec.d.w << 32);
     unsigned long long* buf = reinterpret_cast<unsigned long long*>(buffer);
-    if (splat_wide_point(seed, c, K, key, buf)) return;
+    if (splat_wide_point(seed, c, K, 0, c.passes * K, key, buf)) return;
     if (K == 1 && c.passes == 1) {  // nothing to pair or to pipeline
         uint32_t tile, code;
         const bool live = draw_one(seed, c, tile, code);
@@ -1392,7 +1388,7 @@ __device__ __forceinline__ void splat_point_in_tile(uint32_t point, const SplatR
     const uint32_t key_high = rec.d.w;
     const unsigned long long key = (unsigned long long)rec.d.z | ((unsigned long long)rec.d.w << 32);
     unsigned long long* buf = reinterpret_cast<unsigned long long*>(buffer);
-    if (splat_wide_point(seed, c, K, key, buf)) return;
+    if (splat_wide_point(seed, c, K, 0, c.passes * K, key, buf)) return;
     my_tile += c.tile_bias;
     for (int p = 0; p < c.passes; p += Step::kPasses, nearest += Step::kPasses * kNearPlane) {
         Step step;
@@ -1502,16 +1498,32 @@ __device__ __forceinline__ void splat_group(const SplatArgs& a, const PointOrder
 }
 
 // Groups of kRounds positions per thread while there are at least two per block; a small pass keeps
-// one position per thread and barrier so that its points still spread over every block.
-template <uint32_t kThreads, uint32_t kRounds, class Point>
+// one position per thread and barrier so that its points still spread over every block, and one
+// that would leave half the threads idle splits each point's samples into up to four shares: the
+// pass then takes as long as a share's chain of draws (60k town at 320x180, 28k points of 16
+// samples: frame 55.7 -> 53.5 us).  The code for it costs the other passes 1-2%, so only kernels for small
+// views have it (kShares; see launch_splat).  point(p, record, first, last): samples first..last - 1.
+template <uint32_t kThreads, uint32_t kRounds, bool kShares, class Point>
 __device__ __forceinline__ void splat_walk(const SplatArgs& a, const PointOrder& o, uint32_t* starts, Point&& point) {
+    const uint32_t samples = (uint32_t)(a.fc.num_passes * a.fc.k_points);
     auto walk = [&](auto rounds) {
         constexpr uint32_t r = decltype(rounds)::value;
         for (uint32_t group = blockIdx.x; (unsigned long long)group * (kThreads * r) < o.points; group += gridDim.x)
-            splat_group<kThreads, r>(a, o, group, starts, point);
+            splat_group<kThreads, r>(a, o, group, starts, [&](uint32_t p, const SplatRecord& rec) { point(p, rec, 0u, samples); });
     };
-    if ((unsigned long long)o.points >= 2ull * gridDim.x * (kThreads * kRounds)) walk(std::integral_constant<uint32_t, kRounds>{});
-    else walk(std::integral_constant<uint32_t, 1u>{});
+    const unsigned long long threads = (unsigned long long)gridDim.x * kThreads;
+    if (o.points >= 2ull * threads * kRounds) {
+        walk(std::integral_constant<uint32_t, kRounds>{});
+    } else if (!kShares || o.points * 2ull > threads || samples < 4u) {
+        walk(std::integral_constant<uint32_t, 1u>{});
+    } else if constexpr (kShares) {
+        const uint32_t shares = o.points * 4ull > threads || samples < 8u ? 2u : 4u;
+        const uint32_t per = (samples / 2u + shares - 1u) / shares * 2u + (samples & 1u);  // pairs stay together
+        for (uint32_t w = blockIdx.x; (unsigned long long)(w / shares) * kThreads < o.points; w += gridDim.x) {
+            const uint32_t first = min(w % shares * per, samples), last = min(first + per, samples);
+            splat_group<kThreads, 1>(a, o, w / shares, starts, [&](uint32_t p, const SplatRecord& rec) { point(p, rec, first, last); });
+        }
+    }
 }
 
 __device__ __forceinline__ void fill_spread(uint32_t* spread) {
@@ -1519,7 +1531,8 @@ __device__ __forceinline__ void fill_spread(uint32_t* spread) {
 }
 
 // K > 0: unbiased splatting with K points per thread per pass; K = 0: any other setting.
-template <int K>
+// kShares: for views that may leave half the threads without a point (see splat_walk).
+template <int K, bool kShares>
 #ifndef GPS_SPLAT_MIN_BLOCKS
 #define GPS_SPLAT_MIN_BLOCKS 4
 #endif
@@ -1531,12 +1544,17 @@ __global__ void __launch_bounds__(kSplatTile, kSplatRounds > 1 ? (K >= 8 ? 2 : G
     fill_spread(s_spread);
     const PointOrder o = point_order(a);
     clear_for_next_pass(a, o.points);
-    splat_walk<kSplatTile, kSplatRounds>(a, o, s_start, [&](uint32_t p, const SplatRecord& rec) {
+    splat_walk<kSplatTile, kSplatRounds, kShares>(a, o, s_start, [&](uint32_t p, const SplatRecord& rec, uint32_t first, uint32_t last) {
         if constexpr (K > 0) {
-            splat_point_unbiased_k<K>(p, rec, a.fc, a.frame_seed, a.buffer, s_spread);
-        } else {
-            if (a.fc.use_unbiased) splat_point_unbiased(p, rec, a.fc, a.frame_seed, a.buffer);
-            else splat_point_biased(p, rec, a.fc, a.frame_seed, a.buffer);
+            if (!kShares || last - first == (uint32_t)(a.fc.num_passes * K)) {
+                splat_point_unbiased_k<K>(p, rec, a.fc, a.frame_seed, a.buffer, s_spread);
+                return;
+            }
+        }
+        if constexpr (kShares) {
+            u32x2 seed = sample_seed(p, a.frame_seed, (int)first);
+            if (K > 0 || a.fc.use_unbiased) splat_samples_unbiased(seed, rec, a.fc, a.buffer, s_spread, (int)first, (int)last);
+            else splat_samples_biased(seed, rec, a.fc, a.buffer, (int)first, (int)last);
         }
     });
 }
@@ -1572,7 +1590,7 @@ __global__ void __launch_bounds__(kBinnedThreads, kBinnedBlocks) splat_binned_ke
     const PointOrder o = point_order(a);
     clear_for_next_pass(a, o.points);
     if (!o.binned || (unsigned long long)o.points < 2ull * gridDim.x * kBinnedGroup) {
-        splat_walk<kBinnedThreads, kBinnedRounds>(a, o, s_start, [&](uint32_t p, const SplatRecord& rec) {
+        splat_walk<kBinnedThreads, kBinnedRounds, false>(a, o, s_start, [&](uint32_t p, const SplatRecord& rec, uint32_t, uint32_t) {
             splat_point_unbiased_k<K>(p, rec, a.fc, a.frame_seed, a.buffer, s_spread);
         });
         return;
@@ -2619,11 +2637,11 @@ void launch_scan(const ScanArgs& a, uint32_t scan_tiles, cudaStream_t stream) {
     launch_scan_passes(a, stream);
 }
 
-template <int K>
+template <int K, bool kShares>
 int splat_blocks_per_sm() {
     static int per_sm = 0;
     if (per_sm == 0) {
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, splat_kernel<K>, kSplatTile, 0);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, splat_kernel<K, kShares>, kSplatTile, 0);
         if (per_sm < 1) per_sm = 1;
     }
     return per_sm;
@@ -2636,7 +2654,7 @@ int splat_grid_size(int block) {
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&g_num_sms, cudaDevAttrMultiProcessorCount, dev);
     }
-    return g_num_sms * splat_blocks_per_sm<0>();
+    return g_num_sms * splat_blocks_per_sm<0, true>();
 }
 
 // The shared-memory pre-test needs bins of one tile (up to 8192 x 8192 pixels), a buffer that starts
@@ -2659,6 +2677,11 @@ bool launch_splat_binned(const SplatArgs& a, cudaStream_t stream) {
     return true;
 }
 
+template <int K, bool kShares>
+void launch_splat_plain(const SplatArgs& a, cudaStream_t stream) {
+    launch_k(splat_kernel<K, kShares>, g_num_sms * splat_blocks_per_sm<K, kShares>(), kSplatTile, 0, stream, a);
+}
+
 void launch_splat(const SplatArgs& a, int grid, int block, cudaStream_t stream) {
     (void)block;
     if (g_num_sms == 0) splat_grid_size(kSplatTile);
@@ -2669,17 +2692,16 @@ void launch_splat(const SplatArgs& a, int grid, int block, cudaStream_t stream) 
             return;
     }
     // a persistent grid: as many blocks as fit on the device at once
-    if (a.fc.use_unbiased && a.fc.k_points == 4) {
-        launch_k(splat_kernel<4>, g_num_sms * splat_blocks_per_sm<4>(), kSplatTile, 0, stream, a);
-    } else if (a.fc.use_unbiased && a.fc.k_points == 2) {
-        launch_k(splat_kernel<2>, g_num_sms * splat_blocks_per_sm<2>(), kSplatTile, 0, stream, a);
-    } else if (a.fc.use_unbiased && a.fc.k_points == 8) {
-        launch_k(splat_kernel<8>, g_num_sms * splat_blocks_per_sm<8>(), kSplatTile, 0, stream, a);
-    } else if (a.fc.use_unbiased && a.fc.k_points == 1) {
-        launch_k(splat_kernel<1>, g_num_sms * splat_blocks_per_sm<1>(), kSplatTile, 0, stream, a);
-    } else {
-        launch_k(splat_kernel<0>, grid, kSplatTile, 0, stream, a);
-    }
+    const int k = a.fc.use_unbiased ? a.fc.k_points : 0;
+    // Views of up to 2M samples: at the one or two points per 16 of them that scenes have, fewer points
+    // than half the threads (320x180, ss 2, 4 spp: 0.9M samples, 28k points, 152k threads).
+    const bool small = (uint64_t)a.fc.up_width * (uint64_t)a.fc.up_height * (uint64_t)a.fc.num_passes <= (2u << 20) &&
+                       a.fc.num_passes * k >= 4;
+    if (k == 4) small ? launch_splat_plain<4, true>(a, stream) : launch_splat_plain<4, false>(a, stream);
+    else if (k == 2) small ? launch_splat_plain<2, true>(a, stream) : launch_splat_plain<2, false>(a, stream);
+    else if (k == 1) small ? launch_splat_plain<1, true>(a, stream) : launch_splat_plain<1, false>(a, stream);
+    else if (k == 8) launch_splat_plain<8, false>(a, stream);
+    else launch_k(splat_kernel<0, true>, grid, kSplatTile, 0, stream, a);
 }
 
 void launch_clear(uint64_t* buf, uint64_t entries, uint64_t value, cudaStream_t stream) {
