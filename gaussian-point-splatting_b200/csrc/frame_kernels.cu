@@ -1575,12 +1575,17 @@ __global__ void __launch_bounds__(kSplatTile, kSplatRounds > 1 ? (K >= 8 ? 2 : G
 // it keeps the test in L1.
 //
 // A block takes a.work's next run of consecutive groups, so that a tile serves several groups.  Passes
-// with less than two groups per block take the other walk, which spreads them over more blocks.
-constexpr uint32_t kBinnedThreads = 256, kBinnedRounds = 4, kBinnedGroup = kBinnedThreads * kBinnedRounds;
-constexpr int kBinnedBlocks = 4;  // per SM, as far as their shared memory allows
+// with less than one group per block take the other walk, which spreads them over more blocks.
+//
+// Up to 6 samples per pixel: blocks of 256 threads, four per SM as far as their shared memory allows.
+// From 7 to 13 one block has the SM, with 1024 threads (16 views of a 1M town, five of them at 8 samples:
+// 2625 -> 2441 us a batch; with one group per block enough instead of two, 2407).
+constexpr uint32_t kBinnedGroup = 1024;
+constexpr int binned_blocks(uint32_t threads) { return threads <= 256u ? 4 : 1; }
 
-template <int K>
-__global__ void __launch_bounds__(kBinnedThreads, kBinnedBlocks) splat_binned_kernel(SplatArgs a) {
+template <int K, uint32_t kBinnedThreads>
+__global__ void __launch_bounds__(kBinnedThreads, binned_blocks(kBinnedThreads)) splat_binned_kernel(SplatArgs a) {
+    constexpr uint32_t kBinnedRounds = kBinnedGroup / kBinnedThreads;
     previous_kernel_done();
     __shared__ uint32_t s_start[kBinnedGroup];
     __shared__ uint32_t s_spread[kTileSize];
@@ -1589,7 +1594,7 @@ __global__ void __launch_bounds__(kBinnedThreads, kBinnedBlocks) splat_binned_ke
     fill_spread(s_spread);
     const PointOrder o = point_order(a);
     clear_for_next_pass(a, o.points);
-    if (!o.binned || (unsigned long long)o.points < 2ull * gridDim.x * kBinnedGroup) {
+    if (!o.binned || (unsigned long long)o.points < (unsigned long long)gridDim.x * kBinnedGroup) {
         splat_walk<kBinnedThreads, kBinnedRounds, false>(a, o, s_start, [&](uint32_t p, const SplatRecord& rec, uint32_t, uint32_t) {
             splat_point_unbiased_k<K>(p, rec, a.fc, a.frame_seed, a.buffer, s_spread);
         });
@@ -2658,23 +2663,29 @@ int splat_grid_size(int block) {
 }
 
 // The shared-memory pre-test needs bins of one tile (up to 8192 x 8192 pixels), a buffer that starts
-// cleared, and planes that leave room for at least two blocks in an SM's 227 KB: up to 6 samples
-// per pixel.
-constexpr int kBinnedMaxPasses = 6;
+// cleared, and the planes in an SM's 227 KB beside the rest of a block's shared memory.
+constexpr int kBinnedMaxPasses = 13, kBinnedSmallPasses = 6;
 constexpr int kSmemPerSm = 227 * 1024;
+constexpr int kBinnedStatic = (int)(kBinnedGroup + kTileSize + 4u) * 4 + 1024;  // starts, table, the system's 1 KB
 
-template <int K>
-bool launch_splat_binned(const SplatArgs& a, cudaStream_t stream) {
+template <int K, uint32_t kThreads>
+bool launch_splat_binned(const SplatArgs& a, int max_passes, cudaStream_t stream) {
     const int smem = a.fc.num_passes * (int)kNearPlane * 4;
     // (the limit is the device context's, so it is not remembered here; one value for all callers)
-    if (cudaFuncSetAttribute(splat_binned_kernel<K>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             kBinnedMaxPasses * (int)kNearPlane * 4) != cudaSuccess) {
+    if (cudaFuncSetAttribute(splat_binned_kernel<K, kThreads>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             max_passes * (int)kNearPlane * 4) != cudaSuccess) {
         cudaGetLastError();
         return false;
     }
-    const int blocks = std::min(kBinnedBlocks, kSmemPerSm / (smem + (int)(kBinnedGroup + kTileSize + 4u) * 4 + 1024));
-    launch_k(splat_binned_kernel<K>, g_num_sms * blocks, kBinnedThreads, (size_t)smem, stream, a);
+    const int blocks = std::min(kThreads <= 256u ? 4 : 1, kSmemPerSm / (smem + kBinnedStatic));
+    launch_k(splat_binned_kernel<K, kThreads>, g_num_sms * blocks, kThreads, (size_t)smem, stream, a);
     return true;
+}
+
+template <int K>
+bool launch_splat_binned(const SplatArgs& a, cudaStream_t stream) {
+    return a.fc.num_passes <= kBinnedSmallPasses ? launch_splat_binned<K, 256u>(a, kBinnedSmallPasses, stream)
+                                                 : launch_splat_binned<K, 1024u>(a, kBinnedMaxPasses, stream);
 }
 
 template <int K, bool kShares>

@@ -11,7 +11,9 @@ import synth
 
 pytestmark = pytest.mark.gpu
 
-MIN_POINTS = 2 * 592 * 1024  # of a pass that surely takes the shared-memory test (4 blocks on 148 SMs)
+def _min_points(spp):
+    """Of a pass that surely takes the shared-memory test: two groups per block, 4 or 1 blocks on 148 SMs."""
+    return 2 * (592 if spp <= 6 else 148) * 1024
 
 
 def _frames(scene, s, cams, crowded):
@@ -42,7 +44,9 @@ def _frames(scene, s, cams, crowded):
     (1237, 689, 3, 1, 250_000_000, gpsplat.GPS_SCENE_COMPRESSED),   # planes no power of two
     (1300, 1000, 2, 2, 250_000_000, gpsplat.GPS_SCENE_FP32),
     (1100, 900, 6, 1, 250_000_000, gpsplat.GPS_SCENE_HALF),         # the most planes, two blocks per SM
-    (1100, 900, 7, 1, 250_000_000, gpsplat.GPS_SCENE_FP32),         # one more: the other kernel
+    (1100, 900, 7, 1, 250_000_000, gpsplat.GPS_SCENE_FP32),         # one more: a block of 1024 threads per SM
+    (1100, 900, 13, 4, 250_000_000, gpsplat.GPS_SCENE_FP32),        # its most planes
+    (1100, 900, 14, 1, 250_000_000, gpsplat.GPS_SCENE_FP32),        # one more: the test in L1
     (1920, 1080, 4, 1, 1_300_000, gpsplat.GPS_SCENE_FP32),          # truncated: Gaussian order
 ])
 def test_binned_equals_gaussian_order(width, height, spp, k, max_points, fmt):
@@ -56,5 +60,5 @@ def test_binned_equals_gaussian_order(width, height, spp, k, max_points, fmt):
     for (a, points, order, truncated), (b, _, other, _) in zip(binned, plain):
         assert other == 0 and order == (0 if truncated else 1)
         assert truncated == (1 if max_points < 2_000_000 else 0)
-        assert truncated or points >= MIN_POINTS, points
+        assert truncated or points >= _min_points(spp), points
         assert np.array_equal(a, b)
