@@ -78,15 +78,28 @@ __device__ __forceinline__ bool mask_bit(const uint32_t* m, uint32_t g) {
 // ---------------------------------------------------------------------------------
 // Block cull (gaussian_bvh.cu:215-329)
 // ---------------------------------------------------------------------------------
+// The sums of both tests are spelled out in the rounding that the reference's kernel is compiled to.
+// Left to the compiler, which products are fused depends on the kernel they are inlined into, and one
+// to seven of 8.4M boxes a frame were then culled otherwise, with other point indices and hence other
+// samples for all that follow (the forms were told apart by the culled bits of 40 such frames).
 __device__ __forceinline__ bool aabb_outside_frustum(vec3 bmin, vec3 bmax, const vec4* planes) {
 #pragma unroll
     for (int i = 0; i < 6; ++i) {
         const vec3 n = make_v3(planes[i].x, planes[i].y, planes[i].z);
         const float d = planes[i].w;
         vec3 v = make_v3(n.x >= 0.0f ? bmax.x : bmin.x, n.y >= 0.0f ? bmax.y : bmin.y, n.z >= 0.0f ? bmax.z : bmin.z);
-        if (dot(n, v) + d < 0.0f) return true;
+        if (__fadd_rn(__fmaf_rn(n.z, v.z, __fmaf_rn(n.x, v.x, __fmul_rn(n.y, v.y))), d) < 0.0f) return true;
     }
     return false;
+}
+
+// One row of view-projection * (v, 1).
+__device__ __forceinline__ float project_row(float a, float b, float c, float d, vec3 v) {
+    return __fadd_rn(__fmaf_rn(a, v.x, __fmul_rn(b, v.y)), __fmaf_rn(c, v.z, d));
+}
+__device__ __forceinline__ vec4 project_corner(const mat4& m, vec3 v) {
+    return make_v4(project_row(m.c[0].x, m.c[1].x, m.c[2].x, m.c[3].x, v), project_row(m.c[0].y, m.c[1].y, m.c[2].y, m.c[3].y, v),
+                   project_row(m.c[0].z, m.c[1].z, m.c[2].z, m.c[3].z, v), project_row(m.c[0].w, m.c[1].w, m.c[2].w, m.c[3].w, v));
 }
 
 __device__ __forceinline__ bool aabb_project_bounds(vec3 bmin, vec3 bmax, const mat4& vp, int width, int height,
@@ -99,7 +112,7 @@ __device__ __forceinline__ bool aabb_project_bounds(vec3 bmin, vec3 bmax, const 
     bool any_front = false;
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
-        vec4 clip = vp * make_v4(corners[i].x, corners[i].y, corners[i].z, 1.0f);
+        const vec4 clip = project_corner(vp, corners[i]);
         if (clip.w <= 0.0f) continue;
         any_front = true;
         vec3 ndc = make_v3(clip.x / clip.w, clip.y / clip.w, clip.z / clip.w);
