@@ -238,8 +238,8 @@ def stage_rooflines(stages, spec, st, entries, passes, w, h, peak):
         ms, launches = stages.get(k, (0.0, 0))
         if b is None or ms <= 0 or launches <= 0:
             continue
-        if k == "scan":
-            launches = max(1, launches // 2)  # two launches per pass: tile scan, downsweep
+        if k == "scan":  # one to three launches per pass; the splat has one
+            launches = max(1, stages.get("splat", (0.0, 0))[1])
         per = ms / launches
         gbs = b / (per / 1000.0) / 1e9
         out[k] = {"achieved_gbs": gbs, "frac": gbs / peak, "ms_per_launch": per, "algorithmic_bytes": b}

@@ -197,7 +197,10 @@ gps_status gps_renderer_stats(gps_renderer* r, gps_stats* out);
 /* Per-stage GPU timing with CUDA events on the frame's stream (off by default).  Stages:
  * 0 clear, 1 block cull, 2 preprocess, 3 scan, 4 splat, 5 resolve, 6 Hi-Z, 7 post-process;
  * out_ms[8] receives the accumulated milliseconds, out_launches[8] (may be NULL) the kernel
- * launches per stage, since enabling or the last reset. */
+ * launches per stage, since enabling or the last reset.  Work that shares a launch counts with
+ * that launch: the clear goes with the first pass's block cull (stage 0) or, in frames without one
+ * and for small scenes, with its preprocess (stage 2), which then also culls; the fine Hi-Z levels
+ * go with the resolves. */
 gps_status gps_renderer_enable_timing(gps_renderer* r, int32_t enable);
 gps_status gps_renderer_stage_times(gps_renderer* r, float* out_ms, uint64_t* out_launches, int32_t reset);
 /* The current 64-bit splat buffer (depth28 << 36 | rgb36, Morton 64x64 tiles, spp innermost). */
