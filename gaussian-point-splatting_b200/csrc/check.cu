@@ -1,0 +1,49 @@
+// Entry points for the tests: device steps and launchers of the frame path, one at a time, as the
+// library's kernels use them.  Built into a library of its own (libgps_check.so) on top of
+// libgps_b200.so, with the same flags; no part of the renderer calls anything here.
+#include <cstdint>
+#include <vector>
+#include <cuda_runtime.h>
+#include "frame_kernels.h"
+
+namespace {
+
+template <class T>
+struct DeviceArray {
+    T* p = nullptr;
+    explicit DeviceArray(size_t n, int fill = 0) {
+        if (cudaMalloc(&p, n * sizeof(T)) == cudaSuccess) cudaMemset(p, fill, n * sizeof(T));
+        else p = nullptr;
+    }
+    ~DeviceArray() { cudaFree(p); }
+};
+
+}  // namespace
+
+// The block cull of n Gaussians of which no block is culled, its chunk count starting at `stale`:
+// list[0 .. 2 * chunks) (0xFFFFFFFF where nothing was written) and the count after it.
+extern "C" int gps_check_cull_list(uint32_t n, uint32_t stale, uint32_t* list, uint32_t* count) {
+    using namespace gps;
+    const uint32_t nodes = (n + 3u) / 4u, words = (nodes + 31u) / 32u, chunks = (n + 31u) / 32u;
+    DeviceArray<float4> boxes(2 * (size_t)words * 32), supers(2 * (size_t)words);
+    DeviceArray<uint32_t> culled(words + 1), outside(words + 1), mask(chunks + 1), iter(1), number(1), out(2 * (size_t)chunks, 0xFF);
+    if (!boxes.p || !supers.p || !culled.p || !outside.p || !mask.p || !iter.p || !number.p || !out.p) return 1;
+    cudaMemcpy(number.p, &stale, sizeof(stale), cudaMemcpyHostToDevice);
+    CullArgs a{};
+    a.b.nodes = boxes.p;
+    a.b.culled = culled.p;
+    a.b.node_count = nodes;
+    a.b.words = words;
+    a.b.per_block = 4;
+    a.b.chunk_count = number.p;
+    a.b.supers = supers.p;
+    a.b.outside = outside.p;
+    a.n = n;
+    a.list = out.p;
+    a.mask_pair[0] = a.mask_pair[1] = mask.p;
+    a.mask_iter = iter.p;
+    launch_cull(a, 0);
+    cudaMemcpy(list, out.p, 2 * (size_t)chunks * sizeof(uint32_t), cudaMemcpyDeviceToHost);
+    cudaMemcpy(count, number.p, sizeof(uint32_t), cudaMemcpyDeviceToHost);
+    return (int)cudaGetLastError();
+}

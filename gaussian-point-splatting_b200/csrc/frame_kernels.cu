@@ -262,7 +262,8 @@ __global__ void __launch_bounds__(256) cull_kernel(CullArgs a) {
         uint32_t slot = 0;
         if (lane == 0u) slot = atomicAdd(b.chunk_count, (uint32_t)__popc(m));
         slot = __shfl_sync(0xffffffffu, slot, 0);
-        if (vis) a.list[slot + (uint32_t)__popc(m & ((1u << lane) - 1u))] = c;
+        slot += (uint32_t)__popc(m & ((1u << lane) - 1u));
+        if (vis && slot < chunks) a.list[slot] = c;  // (always, if the count started at zero)
     }
 }
 
@@ -511,7 +512,7 @@ __global__ void __launch_bounds__(256) preprocess_kernel(PreprocessArgs a, Scene
         // contiguous ranges of the list (or of all chunks), so that tile totals merge; the next listed
         // chunk's attributes are prefetched into L2 while this one is worked on (256M town: preprocess
         // 1.149 -> 1.130 ms/frame)
-        const uint32_t count = a.chunk_list ? *a.chunk_count : (a.n + 31u) >> 5;
+        const uint32_t chunks = (a.n + 31u) >> 5, count = a.chunk_list ? min(*a.chunk_count, chunks) : chunks;
         const uint32_t per = (count + warps - 1) / warps;
         const uint32_t b = first * per, e = min(count, b + per);
         uint32_t next = b < e && a.chunk_list ? __ldg(a.chunk_list + b) : b;

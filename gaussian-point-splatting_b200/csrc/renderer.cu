@@ -330,6 +330,7 @@ struct gps_renderer {
     dptr<uint32_t> mask_iter;     // device pass counter selecting the survivor mask pair
     int splat_grid = 0;
     PassCounters* host_counters = nullptr;  // pinned [2]
+    bool aborted = false;  // a launch of the last frame failed: see reset_accumulators
     cudaEvent_t done = nullptr;
     bool have_frame = false;
     bool second_pass_last = false;
@@ -989,11 +990,26 @@ gps_status gps_render_frame(gps_renderer* r, const gps_camera* cam, float* d_ima
 }  // extern "C"
 
 namespace {
+// What a pass's kernels add to starts from zero because the pass before zeroed it on its way (the
+// splat, the scan).  After a frame of which a launch failed that may not have happened: zeroed here,
+// as when the renderer was created, before the next one.
+void reset_accumulators(gps_renderer* r, cudaStream_t st) {
+    cudaMemsetAsync(r->chunk_count.get(), 0, sizeof(uint32_t), st);
+    cudaMemsetAsync(r->loaded.get(), 0, sizeof(uint32_t), st);
+    cudaMemsetAsync(r->hiz_done.get(), 0, sizeof(unsigned), st);
+    cudaMemsetAsync(r->bins.get(), 0, sizeof(unsigned long long) * (kMaxBins + 1), st);
+    cudaMemsetAsync(r->tile_state.get(), 0, sizeof(unsigned long long) * std::max<uint32_t>(scan_tile_count(r->cap_n), 1), st);
+    // (a captured reset may never run: the frames up to the first one outside a capture repeat it)
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(st, &capture) == cudaSuccess && capture == cudaStreamCaptureStatusNone) r->aborted = false;
+}
+
 gps_status render_frame_impl(gps_renderer* r, const gps_camera* cam, float* d_image, float* d_depth, cudaStream_t st) {
     const FrameConst fc = make_frame_const(r, cam);
     const uint64_t bg = 0xFFFFFFF000000000ull |
                         rgb_to_36bits(make_v3(r->s.background[0], r->s.background[1], r->s.background[2]));
     r->frame_launches = 0;
+    if (r->aborted) reset_accumulators(r, st);
     // the clear goes with the frame's first kernel: the block cull's or, without one, the preprocess,
     // unless that splats into the buffer itself
     const ClearArgs clear{reinterpret_cast<ulonglong2*>(r->buffer.get()), r->entries / 2, bg};  // (a multiple of 4096 entries)
@@ -1046,7 +1062,10 @@ gps_status render_frame_impl(gps_renderer* r, const gps_camera* cam, float* d_im
     cudaEventRecord(r->done, st);
     r->have_frame = true;
     cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return fail(GPS_ERR_CUDA, std::string("frame launch failed: ") + cudaGetErrorString(e));
+    if (e != cudaSuccess) {
+        r->aborted = true;
+        return fail(GPS_ERR_CUDA, std::string("frame launch failed: ") + cudaGetErrorString(e));
+    }
     return GPS_OK;
 }
 }  // namespace
