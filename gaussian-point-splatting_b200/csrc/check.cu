@@ -47,3 +47,16 @@ extern "C" int gps_check_cull_list(uint32_t n, uint32_t stale, uint32_t* list, u
     cudaMemcpy(count, number.p, sizeof(uint32_t), cudaMemcpyDeviceToHost);
     return (int)cudaGetLastError();
 }
+
+namespace {
+__global__ void no_kernel() {}
+}  // namespace
+
+// allow_dynamic_smem asked for more than a device has, after an earlier error (or none): whether it
+// refused, and whether an error is pending after it.
+extern "C" void gps_check_smem_refusal(int earlier_error, int* refused, int* pending) {
+    cudaGetLastError();
+    if (earlier_error) cudaSetDevice(-1);
+    *refused = gps::allow_dynamic_smem(reinterpret_cast<const void*>(no_kernel), 1 << 20) ? 0 : 1;
+    *pending = cudaGetLastError() != cudaSuccess ? 1 : 0;
+}

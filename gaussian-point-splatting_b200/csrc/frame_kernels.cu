@@ -2686,11 +2686,8 @@ template <int K, uint32_t kThreads>
 bool launch_splat_binned(const SplatArgs& a, int max_passes, cudaStream_t stream) {
     const int smem = a.fc.num_passes * (int)kNearPlane * 4;
     // (the limit is the device context's, so it is not remembered here; one value for all callers)
-    if (cudaFuncSetAttribute(splat_binned_kernel<K, kThreads>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             max_passes * (int)kNearPlane * 4) != cudaSuccess) {
-        cudaGetLastError();
+    if (!allow_dynamic_smem(reinterpret_cast<const void*>(splat_binned_kernel<K, kThreads>), max_passes * (int)kNearPlane * 4))
         return false;
-    }
     const int blocks = std::min(kThreads <= 256u ? 4 : 1, kSmemPerSm / (smem + kBinnedStatic));
     launch_k(splat_binned_kernel<K, kThreads>, g_num_sms * blocks, kThreads, (size_t)smem, stream, a);
     return true;

@@ -253,6 +253,15 @@ struct ResolveArgs {
     int hiz_fused;  // set by launch_resolve: the launch writes the fine Hi-Z levels
 };
 
+// Lets `kernel` be launched with up to `bytes` of dynamic shared memory; false if the device has not
+// that much.  Such a refusal is no error of the caller's; one that an earlier launch left stays pending.
+inline bool allow_dynamic_smem(const void* kernel, int bytes) {
+    const bool clean = cudaPeekAtLastError() == cudaSuccess;
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) == cudaSuccess) return true;
+    if (clean) cudaGetLastError();
+    return false;
+}
+
 // launchers (all asynchronous on `stream`)
 void launch_cull(const CullArgs& a, cudaStream_t stream);
 // The boxes around every 32 block nodes (load time).

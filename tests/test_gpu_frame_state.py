@@ -70,3 +70,11 @@ def test_frames_after_a_failed_one(n):
             assert np.array_equal(a, b)
     r.close()
     scene.close()
+
+
+@pytest.mark.parametrize("earlier", [0, 1])
+def test_refused_shared_memory_keeps_an_earlier_error(earlier):
+    refused, pending = ctypes.c_int(0), ctypes.c_int(0)
+    _check_library().gps_check_smem_refusal(earlier, ctypes.byref(refused), ctypes.byref(pending))
+    assert refused.value == 1
+    assert pending.value == earlier
