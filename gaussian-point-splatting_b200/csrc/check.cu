@@ -60,3 +60,31 @@ extern "C" void gps_check_smem_refusal(int earlier_error, int* refused, int* pen
     *refused = gps::allow_dynamic_smem(reinterpret_cast<const void*>(no_kernel), 1 << 20) ? 0 : 1;
     *pending = cudaGetLastError() != cudaSuccess ? 1 : 0;
 }
+
+namespace {
+__global__ void depths_kernel(const uint32_t* __restrict__ keys, uint32_t n, float near_plane, float far_plane, float* __restrict__ out) {
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+        out[i] = gps::depth_of_key(keys[i] << 4, near_plane, far_plane);
+}
+}  // namespace
+
+// The NDC depths of n 28-bit keys (host arrays).
+extern "C" int gps_check_depths(const uint32_t* keys, uint32_t n, float near_plane, float far_plane, float* out) {
+    DeviceArray<uint32_t> k(n);
+    DeviceArray<float> d(n);
+    if (!k.p || !d.p) return 1;
+    cudaMemcpy(k.p, keys, (size_t)n * 4, cudaMemcpyHostToDevice);
+    depths_kernel<<<148 * 8, 256>>>(k.p, n, near_plane, far_plane, d.p);
+    cudaMemcpy(out, d.p, (size_t)n * 4, cudaMemcpyDeviceToHost);
+    return (int)cudaGetLastError();
+}
+
+// Whether the library's sweep over all keys finds a depth that falls as the key grows (-1: an error).
+extern "C" int gps_check_depth_falls(float near_plane, float far_plane) {
+    DeviceArray<uint32_t> falls(1);
+    if (!falls.p) return -1;
+    gps::launch_depth_monotone(near_plane, far_plane, falls.p, 0);
+    uint32_t n = 0;
+    cudaMemcpy(&n, falls.p, sizeof(n), cudaMemcpyDeviceToHost);
+    return cudaGetLastError() == cudaSuccess ? (n ? 1 : 0) : -1;
+}

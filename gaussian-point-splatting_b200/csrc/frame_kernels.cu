@@ -1690,9 +1690,20 @@ __device__ __forceinline__ float resolve_pixel(const ResolveArgs& a, int x, int 
 // A 12-bit channel as a float by its bits under 2^23 (exact): no conversion instruction.
 __device__ __forceinline__ float channel12(uint32_t c) { return __uint_as_float(0x4B000000u | (c & 0xFFFu)) - 8388608.0f; }
 
-__device__ __forceinline__ float depth_of_key(uint32_t high_word, const ResolveArgs& a) {
-    const float view_depth = view_depth_from_key((uint64_t)(high_word >> 4), a.near_plane, a.far_plane);
-    return gmin(1e9f, view_to_projected_depth(view_depth, a.near_plane, a.far_plane));
+// Counts the keys whose depth is above the next key's.
+constexpr uint32_t kSweepKeys = 256;  // consecutive keys of a thread
+
+__global__ void __launch_bounds__(256) depth_monotone_kernel(float near_plane, float far_plane, uint32_t* falls) {
+    const uint32_t first = (blockIdx.x * blockDim.x + threadIdx.x) * kSweepKeys;
+    const uint32_t last = min(first + kSweepKeys, (uint32_t)kDepthMax);
+    bool fell = false;
+    float before = depth_of_key(first << 4, near_plane, far_plane);
+    for (uint32_t k = first + 1u; k <= last; ++k) {
+        const float depth = depth_of_key(k << 4, near_plane, far_plane);
+        fell |= !(before <= depth);
+        before = depth;
+    }
+    if (__any_sync(0xffffffffu, fell) && (threadIdx.x & 31u) == 0u) atomicAdd(falls, 1u);
 }
 
 // resolve_pixel with the factor known: the kSs x kSs samples of a pass are in flight together, and the
@@ -1737,7 +1748,7 @@ __device__ __forceinline__ float resolve_pixel_ss(const ResolveArgs& a, int x, i
         a.color[3 * idx + 1] = color.y * inv_passes;
         a.color[3 * idx + 2] = color.z * inv_passes;
     }
-    return depth_of_key(nearest, a);
+    return depth_of_key(nearest, a.near_plane, a.far_plane);
 }
 
 // The frame's counters written to pinned host memory by the first block of the final resolve: a
@@ -1800,7 +1811,7 @@ __device__ __forceinline__ uint32_t morton_compact(uint32_t a) {
 
 // Any supersampling factor: 16 x 16 pixels per block, in Morton order so that groups of 64 threads
 // are 8 x 8 pixels (hiz_fine_levels).  kSs: the factor at compile time, whose samples of a pass are then
-// loaded together (0: any), for planes that launch_resolve calls monotone.
+// loaded together (0: any), for monotone planes (a.monotone).
 template <bool kDepthOnly, int kSs>
 __global__ void __launch_bounds__(256) resolve_kernel(ResolveArgs a, HizView hiz) {
     previous_kernel_done();
@@ -1853,10 +1864,11 @@ __global__ void __launch_bounds__(256) resolve_morton_kernel(ResolveArgs a, HizV
 // block reads with coalesced 16-byte loads.  Used for SS 1, 2, 4, 8 with 1 to 8 or a power of two of
 // samples per pixel and 2 to 128 samples in all.
 //   depth only: of every entry pair the smaller high word goes to shared memory; a pixel's depth
-//     is that of its smallest key.  The conversion to NDC does not decrease with the key (every
-//     step of it rounds monotonically for 0 < near < far; checked over all 2^28 keys for 40 pairs
-//     of planes between 1e-6 and 1e9, and launch_resolve keeps to that range), so the smallest
-//     key's depth is the smallest depth, bit for bit.
+//     is that of its smallest key.  That is the smallest depth bit for bit where the conversion to NDC
+//     does not fall anywhere as the key grows.  It ends in an approximate division, of which only an
+//     error bound is promised, so a renderer sweeps all 2^28 keys of its planes once, when it is
+//     created (a.monotone; 0.4 ms); for planes that fail (a near plane at or below zero: the
+//     view depth passes through zero) every sample is converted, as in resolve_pixel.
 //   final: the run itself goes to shared memory, two pad words after each pixel's samples to keep
 //     a warp's 16-byte reads on different banks (an odd number of words per pixel where the run is no
 //     power of two and read word by word); the 12-bit channels become floats by their bits
@@ -1975,7 +1987,7 @@ __global__ void __launch_bounds__(resolve_pixels(kPasses << (2 * kSsLog2))) reso
             a.color[3 * idx + 2] = color.z * inv_passes;
         }
     }
-    const float depth = depth_of_key(nearest, a);
+    const float depth = depth_of_key(nearest, a.near_plane, a.far_plane);
     if (inside && !(kDepthOnly && a.hiz_fused)) a.depth[(uint32_t)(y * a.width + x)] = depth;
     if constexpr (kPx == 64u) {
         if (a.hiz_fused) hiz_fine_levels(hiz, depth, x, y, a.hiz_min_levels, exchange);
@@ -2757,18 +2769,22 @@ bool launch_resolve_staged(const ResolveArgs& a, const HizView& hiz, dim3 tiles,
 }
 
 template <bool kDepthOnly>
-void launch_resolve_any(const ResolveArgs& a, const HizView& h, bool monotone, int ss_log2, cudaStream_t stream) {
+void launch_resolve_any(const ResolveArgs& a, const HizView& h, int ss_log2, cudaStream_t stream) {
     if (ss_log2 >= 0) {
         const dim3 tiles((unsigned)((a.width * a.ss + kTileSize - 1) >> kTileBits),
                          (unsigned)((a.height * a.ss + kTileSize - 1) >> kTileBits));
-        if (monotone && launch_resolve_staged<kDepthOnly, 0>(a, h, tiles, ss_log2, stream)) return;
+        if (a.monotone && launch_resolve_staged<kDepthOnly, 0>(a, h, tiles, ss_log2, stream)) return;
         const uint64_t threads = ((uint64_t)tiles.x * tiles.y) << (2 * (kTileBits - ss_log2));
         launch_k(resolve_morton_kernel<kDepthOnly>, (unsigned)((threads + 255) / 256), 256, 0, stream, a, h, ss_log2);
         return;
     }
     const dim3 grid((a.width + 15) / 16, (a.height + 15) / 16);
-    if (monotone && a.ss == 3) launch_k(resolve_kernel<kDepthOnly, 3>, grid, 256, 0, stream, a, h);
+    if (a.monotone && a.ss == 3) launch_k(resolve_kernel<kDepthOnly, 3>, grid, 256, 0, stream, a, h);
     else launch_k(resolve_kernel<kDepthOnly, 0>, grid, 256, 0, stream, a, h);
+}
+
+void launch_depth_monotone(float near_plane, float far_plane, uint32_t* falls, cudaStream_t stream) {
+    depth_monotone_kernel<<<(unsigned)((kDepthMax + 1u) / kSweepKeys / 256u), 256, 0, stream>>>(near_plane, far_plane, falls);
 }
 
 int launch_resolve(const ResolveArgs& args, const HizView* hiz, bool depth_only, cudaStream_t stream) {
@@ -2776,16 +2792,14 @@ int launch_resolve(const ResolveArgs& args, const HizView* hiz, bool depth_only,
     int ss_log2 = -1;
     for (int l = 0; l <= 3; ++l)
         if (a.ss == (1 << l)) ss_log2 = l;
-    // planes for which a key's depth is monotone (through zero or past the float range it is not)
-    const bool monotone = a.near_plane >= 1.0e-6f && a.far_plane <= 1.0e9f;
     // the fine Hi-Z levels need a chain of four levels and groups of 64 pixels, which the blocks of
     // more than 64 samples a pixel are not
     const int run = a.ss * a.ss * a.num_passes;
-    const bool small_blocks = ss_log2 >= 0 && monotone && run == kResolveMaxRun;
+    const bool small_blocks = ss_log2 >= 0 && a.monotone && run == kResolveMaxRun;
     a.hiz_fused = hiz && hiz->levels >= 4 && !small_blocks ? 1 : 0;
     const HizView h = a.hiz_fused ? *hiz : HizView{};
-    if (depth_only) launch_resolve_any<true>(a, h, monotone, ss_log2, stream);
-    else launch_resolve_any<false>(a, h, monotone, ss_log2, stream);
+    if (depth_only) launch_resolve_any<true>(a, h, ss_log2, stream);
+    else launch_resolve_any<false>(a, h, ss_log2, stream);
     return a.hiz_fused;
 }
 

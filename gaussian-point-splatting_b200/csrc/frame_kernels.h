@@ -243,6 +243,7 @@ struct ResolveArgs {
     int width, height, num_passes, ss;
     uint64_t entries;
     float near_plane, far_plane;
+    int monotone;  // a key's depth falls nowhere as the key grows (launch_depth_monotone)
     uint64_t initial_value;
     // The final resolve also hands the frame's counters to the host: those of its first
     // `report_passes` passes, zeros for the others (null report_to: not this launch).
@@ -285,6 +286,8 @@ uint32_t scan_tile_count(uint32_t n);
 constexpr uint32_t kScanTileGaussians = 16384;  // Gaussians per scan tile (counts are padded to it)
 void launch_splat(const SplatArgs& a, int grid, int block, cudaStream_t stream);
 void launch_clear(uint64_t* buf, uint64_t entries, uint64_t value, cudaStream_t stream);
+// Adds to *falls if a depth key's NDC depth between these planes is above a larger key's.
+void launch_depth_monotone(float near_plane, float far_plane, uint32_t* falls, cudaStream_t stream);
 // hiz: also write its four finest levels where this view's resolve can (the result says so; a
 // depth-only launch then does not write a.depth).
 int launch_resolve(const ResolveArgs& a, const HizView* hiz, bool depth_only, cudaStream_t stream);

@@ -284,6 +284,16 @@ GPS_HD float view_to_projected_depth(float z_view, float near_plane, float far_p
     return a + b / z_view;
 }
 
+#if defined(__CUDACC__)
+// NDC depth of a key's high word, no more than 1e9 (the resolves' start value; so is a NaN).  A function
+// of its own, not inlined: which of its products are fused depends on the kernel it is inlined into,
+// and the sweep for planes where it is monotone has to run the very code that the resolves run.
+static __device__ __noinline__ float depth_of_key(uint32_t high_word, float near_plane, float far_plane) {
+    const float view_depth = view_depth_from_key((uint64_t)(high_word >> 4), near_plane, far_plane);
+    return gmin(1e9f, view_to_projected_depth(view_depth, near_plane, far_plane));
+}
+#endif
+
 // post_processing_kernels.cuh:71-104: 64x64 Morton tiles, samples-per-pixel innermost.
 GPS_HD uint32_t morton_spread(uint32_t a) {
     a = (a | (a << 8)) & 0x00FF00FFu;

@@ -330,6 +330,7 @@ struct gps_renderer {
     dptr<uint32_t> mask_iter;     // device pass counter selecting the survivor mask pair
     int splat_grid = 0;
     PassCounters* host_counters = nullptr;  // pinned [2]
+    bool depth_monotone = false;  // see launch_depth_monotone
     bool aborted = false;  // a launch of the last frame failed: see reset_accumulators
     cudaEvent_t done = nullptr;
     bool have_frame = false;
@@ -941,6 +942,13 @@ gps_status create_renderer(gps_scene* scene, const gps_settings* settings, const
         // means "nothing occluded" for frame 1
         fill_f32<<<148 * 4, 256>>>(r->mip.get(), r->cap_mip, INFINITY);
         GPS_CUDA(cudaGetLastError());
+        // (`loaded` is a zero word until the first frame)
+        launch_depth_monotone(s.near_view_plane, s.far_view_plane, r->loaded.get(), 0);
+        GPS_CUDA(cudaGetLastError());
+        uint32_t falls = 0;
+        GPS_CUDA(cudaMemcpy(&falls, r->loaded.get(), sizeof(falls), cudaMemcpyDeviceToHost));
+        GPS_CUDA(cudaMemset(r->loaded.get(), 0, sizeof(uint32_t)));
+        r->depth_monotone = falls == 0;
         GPS_CUDA(cudaMallocHost(&r->host_counters, sizeof(PassCounters) * 2));
         std::memset(r->host_counters, 0, sizeof(PassCounters) * 2);
         GPS_CUDA(cudaEventCreateWithFlags(&r->done, cudaEventDisableTiming));
@@ -1033,6 +1041,7 @@ gps_status render_frame_impl(gps_renderer* r, const gps_camera* cam, float* d_im
     ra.entries = r->entries;
     ra.near_plane = r->s.near_view_plane;
     ra.far_plane = r->s.far_view_plane;
+    ra.monotone = r->depth_monotone ? 1 : 0;
     ra.initial_value = bg;
     ra.hiz_min_levels = r->s.occlusion_culling_min_reduce_count;
     auto build_hiz = [&](bool fine_done) {
