@@ -1452,6 +1452,11 @@ __device__ __forceinline__ PointOrder point_order(const SplatArgs& a) {
     return o;
 }
 
+// Whether this pass is splat_binned_kernel's: in screen-bin order, with enough points.
+__device__ __forceinline__ bool takes_tile_test(const SplatArgs& a, const PointOrder& o) {
+    return o.binned && o.points >= a.tile_test_from;
+}
+
 // What the next pass's kernels accumulate into is cleared here; nothing in the splat reads it.
 __device__ __forceinline__ void clear_for_next_pass(const SplatArgs& a, uint32_t points) {
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < a.clear_a_words; i += gridDim.x * blockDim.x)
@@ -1555,8 +1560,9 @@ __global__ void __launch_bounds__(kSplatTile, kSplatRounds > 1 ? (K >= 8 ? 2 : G
     previous_kernel_done();
     __shared__ uint32_t s_start[kSplatWindow];
     __shared__ uint32_t s_spread[kTileSize];
-    fill_spread(s_spread);
     const PointOrder o = point_order(a);
+    if (takes_tile_test(a, o)) return;
+    fill_spread(s_spread);
     clear_for_next_pass(a, o.points);
     splat_walk<kSplatTile, kSplatRounds, kShares>(a, o, s_start, [&](uint32_t p, const SplatRecord& rec, uint32_t first, uint32_t last) {
         if constexpr (K > 0) {
@@ -1588,8 +1594,13 @@ __global__ void __launch_bounds__(kSplatTile, kSplatRounds > 1 ? (K >= 8 ? 2 : G
 // The second pass would have to read its tiles, 128 KB each at 4 spp: 160 -> 209 us on the 4M town, so
 // it keeps the test in L1.
 //
-// A block takes a.work's next run of consecutive groups, so that a tile serves several groups.  Passes
-// with less than one group per block take the other walk, which spreads them over more blocks.
+// A block takes a.work's next run of consecutive groups, so that a tile serves several groups.
+//
+// Whether a pass is in screen-bin order, and how many points it has, is known on the device only: the
+// plain kernel is launched too, and each of them returns at once where the other takes the pass (4M town
+// at 1080p: 875 us a frame with and without the second launch).  The plain walk inside this kernel would run beside the planes' shared memory, with
+// fewer blocks and next to no L1 for its pre-test: a crowded pass of the 1M town at 1080p, 4 spp, took
+// 595 us that way against 331, a sparse one (60k town) 76 against 52.
 //
 // Up to 6 samples per pixel: blocks of 256 threads, four per SM as far as their shared memory allows.
 // From 7 to 13 one block has the SM, with 1024 threads (16 views of a 1M town, five of them at 8 samples:
@@ -1605,15 +1616,10 @@ __global__ void __launch_bounds__(kBinnedThreads, binned_blocks(kBinnedThreads))
     __shared__ uint32_t s_spread[kTileSize];
     __shared__ uint32_t s_next;
     extern __shared__ __align__(16) uint32_t s_nearest[];  // num_passes planes of kNearPlane words
-    fill_spread(s_spread);
     const PointOrder o = point_order(a);
+    if (!takes_tile_test(a, o)) return;
+    fill_spread(s_spread);
     clear_for_next_pass(a, o.points);
-    if (!o.binned || (unsigned long long)o.points < (unsigned long long)gridDim.x * kBinnedGroup) {
-        splat_walk<kBinnedThreads, kBinnedRounds, false>(a, o, s_start, [&](uint32_t p, const SplatRecord& rec, uint32_t, uint32_t) {
-            splat_point_unbiased_k<K>(p, rec, a.fc, a.frame_seed, a.buffer, s_spread);
-        });
-        return;
-    }
     const uint32_t quads = (uint32_t)a.fc.num_passes * (kNearPlane / 4u);
     const uint32_t tiles_per_row = (uint32_t)(a.fc.up_width + kTileSize - 1) >> kTileBits;
     const uint32_t groups = (o.points + kBinnedGroup - 1u) / kBinnedGroup;
@@ -2694,19 +2700,25 @@ constexpr int kBinnedMaxPasses = 13, kBinnedSmallPasses = 6;
 constexpr int kSmemPerSm = 227 * 1024;
 constexpr int kBinnedStatic = (int)(kBinnedGroup + kTileSize + 4u) * 4 + 1024;  // starts, table, the system's 1 KB
 
+// Groups per block from which the shared-memory test takes a pass.  In blocks of 256 threads, two: with
+// one (777k points at 1080p, 4 spp) it takes 111 us against 105, with more it wins (3.4M points: 271 against 333).
+// In blocks of 1024, one (182k points at 8 spp: 100 us either way, 773k: 199 against 229).
+constexpr uint32_t tile_test_groups(uint32_t threads) { return threads <= 256u ? 2u : 1u; }
+
 template <int K, uint32_t kThreads>
-bool launch_splat_binned(const SplatArgs& a, int max_passes, cudaStream_t stream) {
+bool launch_splat_binned(SplatArgs& a, int max_passes, cudaStream_t stream) {
     const int smem = a.fc.num_passes * (int)kNearPlane * 4;
     // (the limit is the device context's, so it is not remembered here; one value for all callers)
     if (!allow_dynamic_smem(reinterpret_cast<const void*>(splat_binned_kernel<K, kThreads>), max_passes * (int)kNearPlane * 4))
         return false;
     const int blocks = std::min(kThreads <= 256u ? 4 : 1, kSmemPerSm / (smem + kBinnedStatic));
+    a.tile_test_from = (uint32_t)(g_num_sms * blocks) * kBinnedGroup * tile_test_groups(kThreads);
     launch_k(splat_binned_kernel<K, kThreads>, g_num_sms * blocks, kThreads, (size_t)smem, stream, a);
     return true;
 }
 
 template <int K>
-bool launch_splat_binned(const SplatArgs& a, cudaStream_t stream) {
+bool launch_splat_binned(SplatArgs& a, cudaStream_t stream) {
     return a.fc.num_passes <= kBinnedSmallPasses ? launch_splat_binned<K, 256u>(a, kBinnedSmallPasses, stream)
                                                  : launch_splat_binned<K, 1024u>(a, kBinnedMaxPasses, stream);
 }
@@ -2716,14 +2728,17 @@ void launch_splat_plain(const SplatArgs& a, cudaStream_t stream) {
     launch_k(splat_kernel<K, kShares>, g_num_sms * splat_blocks_per_sm<K, kShares>(), kSplatTile, 0, stream, a);
 }
 
-void launch_splat(const SplatArgs& a, int grid, int block, cudaStream_t stream) {
+int launch_splat(const SplatArgs& args, int grid, int block, cudaStream_t stream) {
     (void)block;
+    SplatArgs a = args;
+    a.tile_test_from = kNoTileTest;
+    int launches = 1;
     if (g_num_sms == 0) splat_grid_size(kSplatTile);
     if (a.sorted_gid && a.bin_is_tile && a.fresh && a.fc.use_unbiased && a.fc.num_passes <= kBinnedMaxPasses) {
         const int k = a.fc.k_points;
         if (k == 4 ? launch_splat_binned<4>(a, stream) : k == 2 ? launch_splat_binned<2>(a, stream)
             : k == 1 ? launch_splat_binned<1>(a, stream) : false)
-            return;
+            ++launches;
     }
     // a persistent grid: as many blocks as fit on the device at once
     const int k = a.fc.use_unbiased ? a.fc.k_points : 0;
@@ -2736,6 +2751,7 @@ void launch_splat(const SplatArgs& a, int grid, int block, cudaStream_t stream) 
     else if (k == 1) small ? launch_splat_plain<1, true>(a, stream) : launch_splat_plain<1, false>(a, stream);
     else if (k == 8) launch_splat_plain<8, false>(a, stream);
     else launch_k(splat_kernel<0, true>, grid, kSplatTile, 0, stream, a);
+    return launches;
 }
 
 void launch_clear(uint64_t* buf, uint64_t entries, uint64_t value, cudaStream_t stream) {

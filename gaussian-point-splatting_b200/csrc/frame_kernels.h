@@ -191,7 +191,12 @@ struct SplatArgs {
     uint32_t* work;                  // next group of a screen-binned pass; zero before the splat
     int bin_is_tile;                 // a screen bin is one tile of the splat buffer
     int fresh;                       // the buffer starts cleared (a frame's first pass)
+    // set by launch_splat: points from which splat_binned_kernel takes a screen-binned pass; it is
+    // launched beside the plain kernel, and one of them has nothing to do (kNoTileTest: not launched)
+    uint32_t tile_test_from;
 };
+
+constexpr uint32_t kNoTileTest = 0xFFFFFFFFu;
 
 // Screen bins: the splat walks a pass's survivors grouped by the 64x64 splat-buffer tile (or
 // block of tiles, for very large views) that holds their pixel mean, so that blocks running at
@@ -284,7 +289,7 @@ int launch_scan_fused(const ScanArgs& a, cudaStream_t stream);
 int scan_tile_shift(uint32_t n);
 uint32_t scan_tile_count(uint32_t n);
 constexpr uint32_t kScanTileGaussians = 16384;  // Gaussians per scan tile (counts are padded to it)
-void launch_splat(const SplatArgs& a, int grid, int block, cudaStream_t stream);
+int launch_splat(const SplatArgs& a, int grid, int block, cudaStream_t stream);  // returns the launches
 void launch_clear(uint64_t* buf, uint64_t entries, uint64_t value, cudaStream_t stream);
 // Adds to *falls if a depth key's NDC depth between these planes is above a larger key's.
 void launch_depth_monotone(float near_plane, float far_plane, uint32_t* falls, cudaStream_t stream);

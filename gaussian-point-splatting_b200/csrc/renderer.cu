@@ -566,8 +566,7 @@ void render_pass(gps_renderer* r, const FrameConst& fc, int frame, bool first, c
     sp.bin_is_tile = bin_shift == kTileBits ? 1 : 0;
     sp.fresh = first ? 1 : 0;
     sp.chunk_count = listed ? r->chunk_count.get() : nullptr;
-    launch_splat(sp, r->splat_grid, 256, st);
-    count_launch(r, kStSplat);
+    count_launch(r, kStSplat, (uint64_t)launch_splat(sp, r->splat_grid, 256, st));
 }
 
 }  // namespace
