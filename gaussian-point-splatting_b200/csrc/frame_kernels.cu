@@ -1817,21 +1817,27 @@ __device__ __forceinline__ uint32_t morton_compact(uint32_t a) {
 
 // Any supersampling factor: 16 x 16 pixels per block, in Morton order so that groups of 64 threads
 // are 8 x 8 pixels (hiz_fine_levels).  kSs: the factor at compile time, whose samples of a pass are then
-// loaded together (0: any), for monotone planes (a.monotone).
-template <bool kDepthOnly, int kSs>
-__global__ void __launch_bounds__(256) resolve_kernel(ResolveArgs a, HizView hiz) {
+// loaded together (0: any), for monotone planes (a.monotone).  kHiz: with the fine Hi-Z levels.
+// Every thread reads runs of its own, so what bounds it is how many are resident and whether their
+// lines stay in L1: the run-time factor is held to 32 registers (8 blocks per SM), the compiled one has
+// up to 72 for its loads in flight.  With 40 and 48 instead, both resolves at 640x360 took 296 us for
+// ss 5, 5 spp (now 260) and 512 for ss 3, 16 spp (now 296).
+template <bool kDepthOnly, int kSs, bool kHiz>
+__global__ void __launch_bounds__(256, kSs == 0 ? 8 : 1) resolve_kernel(ResolveArgs a, HizView hiz) {
     previous_kernel_done();
     report_counters(a);
-    __shared__ float exchange[8];
     const int x = (int)(blockIdx.x * 16u + morton_compact(threadIdx.x)), y = (int)(blockIdx.y * 16u + morton_compact(threadIdx.x >> 1));
     const bool inside = x < a.width && y < a.height;
     float depth = 0.0f;
     if (inside) {
         if constexpr (kSs > 0) depth = resolve_pixel_ss<kDepthOnly, kSs>(a, x, y);
         else depth = resolve_pixel<kDepthOnly>(a, x, y);
-        if (!(kDepthOnly && a.hiz_fused)) a.depth[y * a.width + x] = depth;
+        if (!(kDepthOnly && kHiz)) a.depth[y * a.width + x] = depth;
     }
-    if (a.hiz_fused) hiz_fine_levels(hiz, depth, x, y, a.hiz_min_levels, exchange);
+    if constexpr (kHiz) {
+        __shared__ float exchange[8];
+        hiz_fine_levels(hiz, depth, x, y, a.hiz_min_levels, exchange);
+    }
 }
 
 // Power-of-two supersampling: the pixels of each 64x64 splat tile in Morton order.  An
@@ -1849,20 +1855,26 @@ __device__ __forceinline__ void morton_pixel(const ResolveArgs& a, uint32_t g, i
     y = (int)((tile / tiles_per_row) * tile_px + morton_compact(m >> 1));
 }
 
-// With `hiz` (a.hiz_levels) the fine Hi-Z levels come with it, and a depth-only launch then
-// leaves the depth image itself to the final resolve.
-template <bool kDepthOnly>
-__global__ void __launch_bounds__(256) resolve_morton_kernel(ResolveArgs a, HizView hiz, int ss_log2) {
+// kHiz: the fine Hi-Z levels come with it, and a depth-only launch then leaves the depth image itself
+// to the final resolve.  Where the image fills the SMs (2048 threads each), the lines that its threads
+// are reading are 256 KB an SM, all of L1, and the few bytes of shared memory and the wait for the block's
+// other pixels cost more than the launch they save: 1080p, ss 2, 15 spp, both resolves and the chain
+// 810 us with, 709 without, and 708 before there were fine levels here; ss 1, 24 spp 372 / 359 / 361, ss 1,
+// 9 spp 119 / 123 / 130.  launch_resolve_any draws the line.
+template <bool kDepthOnly, bool kHiz>
+__global__ void __launch_bounds__(256, 8) resolve_morton_kernel(ResolveArgs a, HizView hiz, int ss_log2) {
     previous_kernel_done();
     report_counters(a);
-    __shared__ float exchange[8];
     int x, y;
     morton_pixel(a, blockIdx.x * blockDim.x + threadIdx.x, ss_log2, x, y);
     const bool inside = x < a.width && y < a.height;
     float depth = 0.0f;
     if (inside) depth = resolve_pixel<kDepthOnly>(a, x, y);
-    if (inside && !(kDepthOnly && a.hiz_fused)) a.depth[y * a.width + x] = depth;
-    if (a.hiz_fused) hiz_fine_levels(hiz, depth, x, y, a.hiz_min_levels, exchange);
+    if (inside && !(kDepthOnly && kHiz)) a.depth[y * a.width + x] = depth;
+    if constexpr (kHiz) {
+        __shared__ float exchange[8];
+        hiz_fine_levels(hiz, depth, x, y, a.hiz_min_levels, exchange);
+    }
 }
 
 // Staged variant: a block's pixels are consecutive in Morton-tile order, so their samples are
@@ -2784,39 +2796,46 @@ bool launch_resolve_staged(const ResolveArgs& a, const HizView& hiz, dim3 tiles,
     }
 }
 
-template <bool kDepthOnly>
-void launch_resolve_any(const ResolveArgs& a, const HizView& h, int ss_log2, cudaStream_t stream) {
+template <bool kDepthOnly, bool kHiz>
+void launch_resolve_plain(const ResolveArgs& a, const HizView& h, dim3 tiles, int ss_log2, cudaStream_t stream) {
     if (ss_log2 >= 0) {
-        const dim3 tiles((unsigned)((a.width * a.ss + kTileSize - 1) >> kTileBits),
-                         (unsigned)((a.height * a.ss + kTileSize - 1) >> kTileBits));
-        if (a.monotone && launch_resolve_staged<kDepthOnly, 0>(a, h, tiles, ss_log2, stream)) return;
         const uint64_t threads = ((uint64_t)tiles.x * tiles.y) << (2 * (kTileBits - ss_log2));
-        launch_k(resolve_morton_kernel<kDepthOnly>, (unsigned)((threads + 255) / 256), 256, 0, stream, a, h, ss_log2);
+        launch_k(resolve_morton_kernel<kDepthOnly, kHiz>, (unsigned)((threads + 255) / 256), 256, 0, stream, a, h, ss_log2);
         return;
     }
     const dim3 grid((a.width + 15) / 16, (a.height + 15) / 16);
-    if (a.monotone && a.ss == 3) launch_k(resolve_kernel<kDepthOnly, 3>, grid, 256, 0, stream, a, h);
-    else launch_k(resolve_kernel<kDepthOnly, 0>, grid, 256, 0, stream, a, h);
+    if (a.monotone && a.ss == 3) launch_k(resolve_kernel<kDepthOnly, 3, kHiz>, grid, 256, 0, stream, a, h);
+    else launch_k(resolve_kernel<kDepthOnly, 0, kHiz>, grid, 256, 0, stream, a, h);
 }
 
 void launch_depth_monotone(float near_plane, float far_plane, uint32_t* falls, cudaStream_t stream) {
     depth_monotone_kernel<<<(unsigned)((kDepthMax + 1u) / kSweepKeys / 256u), 256, 0, stream>>>(near_plane, far_plane, falls);
 }
 
-int launch_resolve(const ResolveArgs& args, const HizView* hiz, bool depth_only, cudaStream_t stream) {
-    ResolveArgs a = args;
+template <bool kDepthOnly>
+int launch_resolve_any(ResolveArgs a, const HizView* hiz, cudaStream_t stream) {
     int ss_log2 = -1;
     for (int l = 0; l <= 3; ++l)
         if (a.ss == (1 << l)) ss_log2 = l;
-    // the fine Hi-Z levels need a chain of four levels and groups of 64 pixels, which the blocks of
-    // more than 64 samples a pixel are not
+    const dim3 tiles((unsigned)((a.width * a.ss + kTileSize - 1) >> kTileBits), (unsigned)((a.height * a.ss + kTileSize - 1) >> kTileBits));
+    // the fine Hi-Z levels need a chain of four levels and groups of 64 pixels, which the staged blocks
+    // of more than 64 samples a pixel are not
     const int run = a.ss * a.ss * a.num_passes;
-    const bool small_blocks = ss_log2 >= 0 && a.monotone && run == kResolveMaxRun;
-    a.hiz_fused = hiz && hiz->levels >= 4 && !small_blocks ? 1 : 0;
-    const HizView h = a.hiz_fused ? *hiz : HizView{};
-    if (depth_only) launch_resolve_any<true>(a, h, ss_log2, stream);
-    else launch_resolve_any<false>(a, h, ss_log2, stream);
+    const bool chain = hiz && hiz->levels >= 4;
+    a.hiz_fused = chain && run != kResolveMaxRun ? 1 : 0;
+    if (ss_log2 >= 0 && a.monotone && launch_resolve_staged<kDepthOnly, 0>(a, a.hiz_fused ? *hiz : HizView{}, tiles, ss_log2, stream))
+        return a.hiz_fused;
+    // unstaged runs: see resolve_morton_kernel (ss 8: a group of 64 pixels is a tile; 640x360, 3 spp, 580 us
+    // with the levels, 560 without)
+    const bool morton_fused = a.ss < 8 && (run <= 16 || (uint64_t)a.width * (uint64_t)a.height <= 148u * 2048u);
+    a.hiz_fused = chain && (ss_log2 < 0 || morton_fused) ? 1 : 0;
+    if (a.hiz_fused) launch_resolve_plain<kDepthOnly, true>(a, *hiz, tiles, ss_log2, stream);
+    else launch_resolve_plain<kDepthOnly, false>(a, HizView{}, tiles, ss_log2, stream);
     return a.hiz_fused;
+}
+
+int launch_resolve(const ResolveArgs& a, const HizView* hiz, bool depth_only, cudaStream_t stream) {
+    return depth_only ? launch_resolve_any<true>(a, hiz, stream) : launch_resolve_any<false>(a, hiz, stream);
 }
 
 void launch_hiz_build(const HizView& h, const float* depth, int min_levels, bool fine_done, cudaStream_t stream) {
