@@ -768,6 +768,7 @@ __global__ void __launch_bounds__(kTileScanThreads) scan_tiles_kernel(ScanArgs a
 // [first, first + count): one or none for most, but a Gaussian right in front of the camera owns
 // thousands, which its whole warp then writes.  All lanes call it; count 0: nothing to do.
 // (tiles starting at or past P are never walked, and the array holds max_points / 256 + 2)
+template <bool kWide>
 __device__ __forceinline__ void own_tiles(uint32_t* __restrict__ tile_first_rank, uint32_t first, uint32_t count,
                                           uint32_t rank, uint32_t P) {
     const uint64_t end = min((uint64_t)first + count, (uint64_t)P);
@@ -778,8 +779,20 @@ __device__ __forceinline__ void own_tiles(uint32_t* __restrict__ tile_first_rank
     const uint32_t lane = threadIdx.x & 31u;
     for (unsigned big = __ballot_sync(0xffffffffu, n > 4u); big; big &= big - 1u) {
         const int src = __ffs(big) - 1;
-        const uint32_t t = __shfl_sync(0xffffffffu, t0, src), m = __shfl_sync(0xffffffffu, n, src),
-                       r = __shfl_sync(0xffffffffu, rank, src);
+        uint32_t t = __shfl_sync(0xffffffffu, t0, src), m = __shfl_sync(0xffffffffu, n, src);
+        const uint32_t r = __shfl_sync(0xffffffffu, rank, src);
+        // kWide: four at a time where there are many (a survivor of 100M points, in a scan of 2M counts, holds
+        // up its warp for 26 us, one by one for 63).  A frame's Gaussians have at most half a point per
+        // pixel, and the code for it costs its binning 5 us of 33.6M Gaussians.
+        if (kWide && m > 128u) {
+            const uint32_t head = (0u - (uint32_t)(reinterpret_cast<uintptr_t>(tile_first_rank + t) >> 2)) & 3u, quads = (m - head) / 4u;
+            uint4* to = reinterpret_cast<uint4*>(tile_first_rank + t + head);
+            if (lane < head) tile_first_rank[t + lane] = r;
+#pragma unroll 4
+            for (uint32_t i = lane; i < quads; i += 32u) to[i] = make_uint4(r, r, r, r);
+            t += head + 4u * quads;
+            m -= head + 4u * quads;
+        }
         for (uint32_t i = lane; i < m; i += 32u) tile_first_rank[t + i] = r;
     }
 }
@@ -888,7 +901,7 @@ __global__ void __launch_bounds__(kScanThreads, kBinned ? 4 : 5) scan_write_kern
                 a.surv_gid[r0 + k] = g;
                 a.surv_start[r0 + k] = pt;
             }
-            if (!kBinned) own_tiles(a.tile_first_rank, pt, pt < P ? cnt : 0u, r0 + k, P);
+            if (!kBinned) own_tiles<true>(a.tile_first_rank, pt, pt < P ? cnt : 0u, r0 + k, P);
         }
         r0 += tot_s;
         p0 += tot_p;
@@ -922,7 +935,7 @@ __global__ void __launch_bounds__(256) bin_survivors_kernel(ScanArgs a) {
             cnt = a.counts[g];
         }
         if (!binned) {
-            own_tiles(a.tile_first_rank, pt, pt < P ? cnt : 0u, k, P);
+            own_tiles<false>(a.tile_first_rank, pt, pt < P ? cnt : 0u, k, P);
             continue;
         }
         if (live) {
@@ -966,7 +979,7 @@ __global__ void __launch_bounds__(256) bin_survivors_kernel(ScanArgs a) {
             a.sorted_pstart[slot] = pt;
             a.sorted_qstart[slot] = first;
         }
-        own_tiles(a.tile_first_rank, first, cnt, slot, P);
+        own_tiles<false>(a.tile_first_rank, first, cnt, slot, P);
     }
 }
 
