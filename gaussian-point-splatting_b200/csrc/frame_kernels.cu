@@ -809,6 +809,13 @@ __device__ __forceinline__ void own_tiles(uint32_t* __restrict__ tile_first_rank
 // takes less time than a launch that scans them (up to kDirectTiles words, 32 KB from L2).
 constexpr uint32_t kDirectTiles = 4096;
 
+// A 16384-Gaussian tile whose warps need no more than kSparseSteps steps for their 2048 Gaussians is taken
+// at once, not in four rounds with their barriers and lists.  200M counts, 1% of them marked: 273 -> 155 us
+// (206 when a thread took its Gaussians twice and there were no lists), 64 neighbours in each
+// tile 214 -> 99 (144); 70M, 10%, 12 steps (rounds) 162, 18 steps 182.  Not in the render path, where
+// the survivors of a tile are many or none: 33.6M town 1167 -> 1177 us a frame with it.
+constexpr uint32_t kSparseTile = 2560, kSparseSteps = 12;
+
 template <int kScanRounds, bool kDirect, bool kBinned>
 __global__ void __launch_bounds__(kScanThreads, kBinned ? 4 : 5) scan_write_kernel(ScanArgs a, uint32_t tiles) {
     previous_kernel_done();
@@ -826,10 +833,11 @@ __global__ void __launch_bounds__(kScanThreads, kBinned ? 4 : 5) scan_write_kern
         return;
     }
     const uint32_t tile = blockIdx.x - (kBinned ? 1u : 0u);
-    uint32_t r0, p0, P;
+    uint32_t r0, p0, P, in_tile;  // in_tile: its survivors
     if (kDirect) {
         // a tile without survivors has nothing to write (the first one writes the counters)
-        if (tile != 0u && (a.tile_state[tile] >> 32) == 0ull) return;
+        in_tile = (uint32_t)(a.tile_state[tile] >> 32);
+        if (tile != 0u && in_tile == 0u) return;
         uint32_t s_pre = 0, p_pre = 0, s_all = 0, p_all = 0;
         for (uint32_t i = threadIdx.x; i < tiles; i += kScanThreads) {
             const unsigned long long v = a.tile_state[i];
@@ -867,30 +875,15 @@ __global__ void __launch_bounds__(kScanThreads, kBinned ? 4 : 5) scan_write_kern
         p0 = (uint32_t)pre;
         // culled regions of the scene cost two loads, not a pass over their masks
         // (256M town: scan 0.586 -> 0.548 ms/frame)
-        if (r0 == (tile + 1u < tiles ? (uint32_t)(a.tile_state[tile + 1u] >> 32) : a.counters->survivors)) return;
+        in_tile = (tile + 1u < tiles ? (uint32_t)(a.tile_state[tile + 1u] >> 32) : a.counters->survivors) - r0;
+        if (in_tile == 0u) return;
         P = a.counters->points;
     }
     const uint32_t* mask = a.mask;  // (a select, not a runtime index into the parameter array)
     if (a.mask_iter) mask = (*a.mask_iter & 1u) ? a.mask_pair[1] : a.mask_pair[0];
-    for (int q = 0; q < kScanRounds; ++q) {
-        const uint32_t base = (tile * kScanRounds + (uint32_t)q) * kScanTileSmall;
-        if (base >= a.n) break;
-        uint32_t tot_s, tot_p;
-        {
-            uint32_t cnt[kScanItems], pts = 0, at, pt;
-            uint32_t bits = scan_load(a, mask, base + threadIdx.x * kScanItems, cnt);
-#pragma unroll
-            for (int i = 0; i < kScanItems; ++i) pts += cnt[i];
-            block_scan_pair<kScanThreads>((uint32_t)__popc(bits), pts, at, pt, tot_s, tot_p);
-#pragma unroll
-            for (int i = 0; i < kScanItems; ++i)
-                if ((bits >> i) & 1u) {
-                    list_g[at] = (uint16_t)(threadIdx.x * kScanItems + i);
-                    list_p[at++] = pt;
-                    pt += cnt[i];
-                }
-            if (threadIdx.x == 0u) list_p[tot_s] = tot_p;
-        }
+    // The listed survivors of the Gaussians from `base` on, whose totals are tot_s and tot_p.
+    auto write_out = [&](uint32_t base, uint32_t tot_s, uint32_t tot_p) {
+        if (threadIdx.x == 0u) list_p[tot_s] = tot_p;
         __syncthreads();
         for (uint32_t k0 = threadIdx.x & ~31u; k0 < tot_s; k0 += kScanThreads) {
             const uint32_t k = k0 + lane;
@@ -906,6 +899,122 @@ __global__ void __launch_bounds__(kScanThreads, kBinned ? 4 : 5) scan_write_kern
         r0 += tot_s;
         p0 += tot_p;
         __syncthreads();
+    };
+    // 16 Gaussians per thread from `base` on.
+    auto take = [&](uint32_t base) {
+        uint32_t cnt[kScanItems], pts = 0, at, pt, tot_s, tot_p;
+        const uint32_t bits = scan_load(a, mask, base + threadIdx.x * kScanItems, cnt);
+#pragma unroll
+        for (int i = 0; i < kScanItems; ++i) pts += cnt[i];
+        block_scan_pair<kScanThreads>((uint32_t)__popc(bits), pts, at, pt, tot_s, tot_p);
+#pragma unroll
+        for (int i = 0; i < kScanItems; ++i)
+            if ((bits >> i) & 1u) {
+                list_g[at] = (uint16_t)(threadIdx.x * kScanItems + i);
+                list_p[at++] = pt;
+                pt += cnt[i];
+            }
+        write_out(base, tot_s, tot_p);
+    };
+    const uint32_t first = tile * (kScanRounds * kScanTileSmall);
+    if constexpr (kScanRounds > 1 && !kBinned) {
+        // few survivors: a warp has 64 mask words, a lane two of them.  The warp goes from bit to bit in every
+        // lane's words together, or, where the survivors are neighbours, from word to word with a lane per
+        // Gaussian, whichever takes fewer steps.
+        static_assert(kScanRounds * kScanTileSmall == 64u * kScanThreads, "two mask words per thread");
+        if (in_tile <= kSparseTile) {
+            const uint32_t mine = first + 64u * threadIdx.x;
+            const uint32_t lo = mine < a.n ? __ldg(&mask[mine >> 5]) : 0u, hi = mine + 32u < a.n ? __ldg(&mask[(mine >> 5) + 1u]) : 0u;
+            uint64_t bits = ((uint64_t)hi << 32) | lo;
+            if (mine < a.n && a.n - mine < 64u) bits &= (1ull << (a.n - mine)) - 1ull;
+            const uint32_t words = __ballot_sync(0xffffffffu, bits != 0ull);  // (pairs of words)
+            const uint32_t most = __reduce_max_sync(0xffffffffu, (uint32_t)__popcll(bits));
+            const bool by_bit = most <= 2u * (uint32_t)__popc(words);
+            if (!__syncthreads_or((by_bit ? most : 2u * (uint32_t)__popc(words)) > kSparseSteps)) {
+                uint32_t pts = 0;
+                const uint32_t warp = threadIdx.x >> 5, warp_first = first + 2048u * warp;
+                if (by_bit) {
+                    for (uint64_t m = bits; m; m &= m - 1ull) pts += __ldg(a.counts + mine + (uint32_t)(__ffsll((long long)m) - 1));
+                } else {
+                    for (uint32_t m = words; m; m &= m - 1u) {
+                        const int src = __ffs(m) - 1;
+                        const uint64_t both = __shfl_sync(0xffffffffu, bits, src);
+                        const uint32_t* c = a.counts + warp_first + 64u * (uint32_t)src + lane;
+                        if ((both >> lane) & 1ull) pts += __ldg(c);
+                        if ((both >> (lane + 32u)) & 1ull) pts += __ldg(c + 32);
+                    }
+                }
+                // the warps before this one and, going by bit, the lanes before this one
+                const uint32_t survivors = (uint32_t)__popcll(bits);
+                uint32_t s_in = survivors, p_in = pts;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const uint32_t vs = __shfl_up_sync(0xffffffffu, s_in, o), vp = __shfl_up_sync(0xffffffffu, p_in, o);
+                    if (lane >= (uint32_t)o) {
+                        s_in += vs;
+                        p_in += vp;
+                    }
+                }
+                if (lane == 31u) {
+                    sums[0][warp] = s_in;
+                    sums[1][warp] = p_in;
+                }
+                __syncthreads();
+                for (uint32_t v = 0; v < warp; ++v) {
+                    r0 += sums[0][v];
+                    p0 += sums[1][v];
+                }
+                if (by_bit) {
+                    uint32_t r = r0 + s_in - survivors, pt = p0 + p_in - pts;
+                    uint64_t m = bits;
+                    for (uint32_t k = 0; k < most; ++k) {
+                        const bool live = m != 0ull;
+                        const uint32_t g = mine + (live ? (uint32_t)(__ffsll((long long)m) - 1) : 0u);
+                        const uint32_t cnt = live ? __ldg(a.counts + g) : 0u;  // (again, from L1)
+                        if (live) {
+                            a.surv_gid[r] = g;
+                            a.surv_start[r] = pt;
+                        }
+                        own_tiles<true>(a.tile_first_rank, pt, pt < P ? cnt : 0u, r, P);
+                        r += live ? 1u : 0u;
+                        pt += cnt;
+                        m &= m - 1ull;
+                    }
+                } else {
+                    for (uint32_t m = words; m; m &= m - 1u) {
+                        const int src = __ffs(m) - 1;
+                        const uint64_t both = __shfl_sync(0xffffffffu, bits, src);
+#pragma unroll
+                        for (int h = 0; h < 2; ++h) {
+                            const uint32_t w = (uint32_t)(both >> (32 * h));
+                            if (!w) continue;
+                            const uint32_t g = warp_first + 64u * (uint32_t)src + 32u * (uint32_t)h + lane;
+                            const uint32_t cnt = (w >> lane) & 1u ? __ldg(a.counts + g) : 0u;
+                            uint32_t sum = cnt;
+#pragma unroll
+                            for (int o = 1; o < 32; o <<= 1) {
+                                const uint32_t v = __shfl_up_sync(0xffffffffu, sum, o);
+                                if (lane >= (uint32_t)o) sum += v;
+                            }
+                            const uint32_t r = r0 + (uint32_t)__popc(w & ((1u << lane) - 1u)), pt = p0 + sum - cnt;
+                            if ((w >> lane) & 1u) {
+                                a.surv_gid[r] = g;
+                                a.surv_start[r] = pt;
+                            }
+                            own_tiles<true>(a.tile_first_rank, pt, pt < P ? cnt : 0u, r, P);
+                            r0 += (uint32_t)__popc(w);
+                            p0 += __shfl_sync(0xffffffffu, sum, 31);
+                        }
+                    }
+                }
+                return;
+            }
+        }
+    }
+    for (int q = 0; q < kScanRounds; ++q) {
+        const uint32_t base = first + (uint32_t)q * kScanTileSmall;
+        if (base >= a.n) break;
+        take(base);
     }
 }
 
