@@ -2514,8 +2514,7 @@ constexpr int kTaaTile = 32, kTaaRows = 2, kTaaHeight = 8 * kTaaRows, kTaaSpan =
 __global__ void __launch_bounds__(256, 6) taa_kernel(uint8_t* __restrict__ image, float* __restrict__ out_color,
                            const float* __restrict__ cur_color,
                            const float* __restrict__ prev_color, const float* __restrict__ cur_depth,
-                           const float* __restrict__ prev_depth, mat4 reproj, float blend, int width, int height,
-                           int frame_number) {
+                           const float* __restrict__ prev_depth, mat4 reproj, float blend, int width, int height) {
     previous_kernel_done();
     __shared__ float tile[(kTaaHeight + 2) * kTaaSpan];
     __shared__ float put[8][kTaaTile * 3];
@@ -2563,7 +2562,7 @@ __global__ void __launch_bounds__(256, 6) taa_kernel(uint8_t* __restrict__ image
         vec3 color = mid1;
         const bool inside = x < width && y < height;
         const int idx = y * width + x;
-        if (inside && frame_number > 0) {
+        if (inside) {
             const float depth = depths[r];
             vec4 clip = make_v4((x + 0.5f) / width * 2.0f - 1.0f, (y + 0.5f) / height * 2.0f - 1.0f, depth, 1.0f);
             vec4 prev = reproj * clip;
@@ -2636,6 +2635,25 @@ __global__ void __launch_bounds__(256, 6) taa_kernel(uint8_t* __restrict__ image
         lo1 = lo2;
         hi1 = hi2;
         mid1 = mid2;
+    }
+}
+
+// A frame without history: the colours as they are.  Four values per thread where the buffers are aligned
+// for it; in taa_kernel, whose tile nobody needs then, 4K took 67.7 us (41.8 before it had one).
+__global__ void __launch_bounds__(256) taa_first_kernel(uint8_t* __restrict__ image, float* __restrict__ out_color,
+                                                        const float* __restrict__ cur_color, uint32_t values, int aligned) {
+    previous_kernel_done();
+    auto byte_of = [](float v) { return (uint8_t)roundf(gclamp(v, 0.0f, 1.0f) * 255.0f); };
+    const uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) * 4u;
+    if (aligned && i + 4u <= values) {
+        const float4 c = *reinterpret_cast<const float4*>(cur_color + i);
+        *reinterpret_cast<float4*>(out_color + i) = c;
+        *reinterpret_cast<uchar4*>(image + i) = make_uchar4(byte_of(c.x), byte_of(c.y), byte_of(c.z), byte_of(c.w));
+        return;
+    }
+    for (uint32_t k = i; k < min(i + 4u, values); ++k) {
+        out_color[k] = cur_color[k];
+        image[k] = byte_of(cur_color[k]);
     }
 }
 
@@ -2999,9 +3017,16 @@ void launch_block_bounds(const float4* pos_op, const float4* rot, const float4* 
 void launch_taa(uint8_t* image, float* out_color, const float* cur_color, const float* prev_color,
                 const float* cur_depth, const float* prev_depth, const mat4& reproj, float blend, int width, int height,
                 int frame_number, cudaStream_t stream) {
+    if (frame_number <= 0) {
+        const uint32_t values = 3u * (uint32_t)width * (uint32_t)height;
+        const uintptr_t at = reinterpret_cast<uintptr_t>(out_color) | reinterpret_cast<uintptr_t>(cur_color);
+        const int aligned = (at & 15u) == 0 && (reinterpret_cast<uintptr_t>(image) & 3u) == 0;
+        launch_k(taa_first_kernel, (values + 1023u) / 1024u, 256, 0, stream, image, out_color, cur_color, values, aligned);
+        return;
+    }
     const dim3 grid((unsigned)((width + kTaaTile - 1) / kTaaTile), (unsigned)((height + kTaaHeight - 1) / kTaaHeight));
     launch_k(taa_kernel, grid, 256, 0, stream, image, out_color, cur_color, prev_color, cur_depth, prev_depth, reproj,
-             blend, width, height, frame_number);
+             blend, width, height);
 }
 
 void launch_progressive(uint8_t* image, float* cur_color, float* accum, int width, int height, int frames,
