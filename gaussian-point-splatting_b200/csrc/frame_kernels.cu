@@ -190,9 +190,8 @@ __device__ __forceinline__ uint32_t cull_word(const CullArgs& a, uint32_t word, 
 // tests the box around a word's 32 nodes (first pass) or looks whether all 32 were outside in the
 // first pass (second pass, same camera), the words that are left go to a list in shared memory,
 // and the warps take those.  A block has a.words_per_block words (8 to 64: enough blocks to fill the
-// GPU where the scene is small) and lists the chunks whose first node is among them; where the
-// chunk size is no multiple of the node size, the last chunk also needs up to eight nodes of the
-// next word, tested here too.
+// GPU where the scene is small) and lists their chunks: a word's 32 nodes of per_block Gaussians are exactly
+// per_block chunks, so a chunk's nodes are all in one word.
 // One launch instead of three; cull and clear 225 -> 133 us a frame with 8.4M nodes (33.6M town, of
 // which the boxes are 42 us at the copy rate), the frame 1530 -> 1434; 1M nodes 1009 -> 999; taking 256
 // nodes a block one group after the other instead, 253.
@@ -204,13 +203,11 @@ __global__ void __launch_bounds__(256) cull_kernel(CullArgs a) {
         clear_beside(a.clear, blockIdx.x - a.cull_blocks, gridDim.x - a.cull_blocks);
         return;
     }
-    __shared__ uint32_t culled[kCullWords + 1], outside[kCullWords + 1], todo[kCullWords + 1], todo_count;
+    __shared__ uint32_t culled[kCullWords], outside[kCullWords], todo[kCullWords], todo_count;
     const BlockView& b = a.b;
     const uint32_t t = threadIdx.x, lane = t & 31u, warp = t >> 5;
     const uint32_t w0 = blockIdx.x * a.words_per_block, n0 = w0 << 5, pb = b.per_block;
-    const uint32_t own = min(a.words_per_block, b.words - w0), n1 = n0 + (own << 5);
-    // the next word too if this block's last chunk reaches into it
-    const uint32_t words = own + (w0 + own < b.words && (n1 * pb & 31u) != 0u ? 1u : 0u);
+    const uint32_t words = min(a.words_per_block, b.words - w0);
     if (t == 0u) todo_count = 0u;
     __syncthreads();
     if (t < words) {
@@ -237,24 +234,20 @@ __global__ void __launch_bounds__(256) cull_kernel(CullArgs a) {
         }
     }
     __syncthreads();
-    if (t < own) {
+    if (t < words) {
         b.culled[w0 + t] = culled[t];
         if (!a.second_pass) b.outside[w0 + t] = outside[t];
     }
     uint32_t* mask = (*a.mask_iter & 1u) ? a.mask_pair[1] : a.mask_pair[0];
     const uint32_t chunks = (a.n + 31u) >> 5;
-    const uint32_t c0 = (n0 * pb + 31u) >> 5, c1 = min((n1 * pb + 31u) >> 5, chunks);
+    const uint32_t c0 = w0 * pb, c1 = min((w0 + words) * pb, chunks);
     for (uint32_t base = c0 + (warp << 5); base < c1; base += 256u) {
         const uint32_t c = base + lane;
         bool vis = false;
         if (c < c1) {
             const uint32_t first = (c << 5) / pb - n0, last = min((c << 5) + 31u, a.n - 1u) / pb - n0;
-            for (uint32_t w = first >> 5; w <= last >> 5; ++w) {
-                uint32_t of = 0xffffffffu;  // the chunk's nodes in word w
-                if (w == first >> 5) of &= 0xffffffffu << (first & 31u);
-                if (w == last >> 5) of &= 0xffffffffu >> (31u - (last & 31u));
-                vis |= (~culled[w] & of) != 0u;
-            }
+            const uint32_t nodes = 0xffffffffu << (first & 31u) & 0xffffffffu >> (31u - (last & 31u));
+            vis = (~culled[first >> 5] & nodes) != 0u;
             if (!vis) mask[c] = 0u;
         }
         const uint32_t m = __ballot_sync(0xffffffffu, vis);
