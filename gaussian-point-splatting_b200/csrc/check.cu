@@ -5,6 +5,7 @@
 #include <vector>
 #include <cuda_runtime.h>
 #include "frame_kernels.h"
+#include "gps_draw.cuh"
 
 namespace {
 
@@ -170,5 +171,99 @@ extern "C" int gps_check_cull(const float* nodes, uint32_t count, uint32_t per_b
         download(list[pass], out.p, (size_t)chunks * 4);
         download(mask[pass], masks.p, (size_t)chunks * 4);
     }
+    return (int)cudaGetLastError();
+}
+
+namespace {
+
+using Tally = unsigned long long;
+
+// Over all floats: where the draw's steps differ from CUDA's functions.
+__global__ void draw_steps_kernel(Tally* differ) {
+    using namespace gps;
+    const uint64_t threads = (uint64_t)gridDim.x * blockDim.x;
+    uint32_t d[6] = {0, 0, 0, 0, 0, 0};
+    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < (1ull << 32); i += threads) {
+        const float v = __uint_as_float((uint32_t)i);
+        if (v >= 1.e-37f && v <= 1.0f) {
+            const float l = __logf(v);
+            d[0] += l > 0.0f;
+            d[1] += -neg_root(2.0f * l) != __fsqrt_rn(fmaxf(-2.0f * l, 0.0f));
+        }
+        if (v >= 1.e-7f && v <= 171.0f) {
+            const float2 r = neg_root2(make_float2(-v, -v));
+            d[2] += -r.x != __fsqrt_rn(v) || -r.y != __fsqrt_rn(v) || -neg_root(-v) != __fsqrt_rn(v);
+        }
+        const float2 f = floor_bits2(make_float2(v, v));
+        const uint32_t b = __float_as_uint(floor_bits(v)) - kFloorBits;
+        if (fabsf(v) < 4194304.0f) d[3] += (int)b != (int)floorf(v) || __float_as_uint(f.x) - kFloorBits != b || __float_as_uint(f.y) - kFloorBits != b;
+        else d[4] += b < 200000u || __float_as_uint(f.x) - kFloorBits < 200000u || __float_as_uint(f.y) - kFloorBits < 200000u;
+        if (v >= 0.0f && v <= 2.0f) {
+            const float2 p = by_li2_max2(make_float2(v, v));
+            d[5] += p.x != v / kLi2Max || p.y != v / kLi2Max;
+        }
+    }
+    for (int k = 0; k < 6; ++k)
+        if (d[k]) atomicAdd(differ + k, (Tally)d[k]);
+}
+
+// Samples of random Gaussians: those that draw_pair and draw_one draw otherwise than draw_sample; live ones.
+__global__ void draws_kernel(uint32_t gaussians, uint32_t draws, uint32_t salt, Tally* out) {
+    using namespace gps;
+    uint32_t differ = 0, live = 0;
+    FrameConst fc{};
+    fc.num_passes = 4;
+    fc.up_width = 3840;
+    fc.up_height = 2160;
+    for (uint32_t g = blockIdx.x * blockDim.x + threadIdx.x; g < gaussians; g += gridDim.x * blockDim.x) {
+        u32x2 r = make_seed(g, salt);
+        const vec2 a = pcg2d(r), b = pcg2d(r), c = pcg2d(r);
+        const float mx = a.x * 3900.0f - 30.0f, my = a.y * 2220.0f - 30.0f;
+        const float sx = exp2f(b.x * 12.0f - 2.0f), sy = exp2f(b.y * 12.0f - 2.0f), rho = (c.x - 0.5f) * 1.99f;
+        const float xx = sx * sx + 0.3f, yy = sy * sy + 0.3f, xy = rho * sx * sy, inv = 1.0f / (xx * yy - xy * xy);
+        SplatRecord rec;
+        rec.a = make_float4(mx, my, sqrtf(xx), xy / sqrtf(xx));
+        rec.b = make_float4(sqrtf(yy - rec.a.w * rec.a.w), yy * inv, -xy * inv, xx * inv);
+        rec.c = make_float4(g & 7u ? c.y * 0.996f + 0.004f : 1.0f, 0.0f, 0.0f, 0.0f);
+        ivec2 lo, hi;
+        if (!gaussian_tile_bounds(lo, hi, {fc.up_width, fc.up_height}, make_v3(xx, xy, yy), make_v2(mx, my))) continue;
+        rec.d = make_uint4((uint32_t)lo.x | ((uint32_t)lo.y << 16), (uint32_t)hi.x | ((uint32_t)hi.y << 16), 0u, 0u);
+        const SampleConst k = sample_const(rec, fc, nullptr);
+        u32x2 one = make_seed(g, salt + 1u), two = one, single = one;
+        for (uint32_t s = 0; s < draws; s += 2u) {
+            uint32_t tile[2], code[2];
+            bool on[2];
+            draw_pair(two, k, tile, code, on);
+            for (int j = 0; j < 2; ++j) {
+                uint32_t t0, c0, t1, c1;
+                const bool l0 = draw_sample(one, k, t0, c0), l1 = draw_one(single, k, t1, c1);
+                live += l0;
+                differ += l0 != on[j] || l0 != l1 || (l0 && (t0 != tile[j] || c0 != code[j] || t1 != tile[j] || c1 != code[j]));
+            }
+        }
+        differ += one.x != two.x || one.y != two.y || one.x != single.x;
+    }
+    if (differ) atomicAdd(out, (Tally)differ);
+    atomicAdd(out + 1, (Tally)live);
+}
+
+}  // namespace
+
+// differ[6]: logarithms above zero, neg_root of one, neg_root of any radicand, floor_bits, floor_bits out
+// of range, by_li2_max2.
+extern "C" int gps_check_draw_steps(unsigned long long* differ) {
+    DeviceArray<Tally> d(6);
+    if (!d.p) return 1;
+    draw_steps_kernel<<<148 * 8, 256>>>(d.p);
+    download(differ, d.p, 6 * sizeof(Tally));
+    return (int)cudaGetLastError();
+}
+
+// out[2]: samples drawn otherwise, live samples.
+extern "C" int gps_check_draws(uint32_t gaussians, uint32_t draws, uint32_t salt, unsigned long long* out) {
+    DeviceArray<Tally> d(2);
+    if (!d.p) return 1;
+    draws_kernel<<<148 * 8, 128>>>(gaussians, draws, salt, d.p);
+    download(out, d.p, 2 * sizeof(Tally));
     return (int)cudaGetLastError();
 }
