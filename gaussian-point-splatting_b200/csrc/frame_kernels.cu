@@ -1586,9 +1586,7 @@ __global__ void clear_kernel(ulonglong2* __restrict__ buf, uint64_t pairs, unsig
 }
 
 // One output pixel: the mean colour of its SS x SS x spp samples and their nearest NDC depth,
-// in the reference's loop order.  The depth arithmetic is kept in exactly this form (and
-// loop shape) because the reference's result depends on how the compiler evaluates it under
-// fast math; the parity tests check it bit for bit.
+// in the reference's loop order, with the depth steps in the rounding that gps_math.cuh spells out.
 template <bool kDepthOnly>
 __device__ __forceinline__ float resolve_pixel(const ResolveArgs& a, int x, int y) {
     const uint32_t idx = (uint32_t)(y * a.width + x);
@@ -1811,7 +1809,7 @@ __global__ void __launch_bounds__(256, 8) resolve_morton_kernel(ResolveArgs a, H
 //     is that of its smallest key.  That is the smallest depth bit for bit where the conversion to NDC
 //     does not fall anywhere as the key grows.  It ends in an approximate division, of which only an
 //     error bound is promised, so a renderer sweeps all 2^28 keys of its planes once, when it is
-//     created (a.monotone; 0.4 ms); for planes that fail (a near plane at or below zero: the
+//     created (a.monotone; under half a millisecond); for planes that fail (a near plane at or below zero: the
 //     view depth passes through zero) every sample is converted, as in resolve_pixel.
 //   final: the run itself goes to shared memory, two pad words after each pixel's samples to keep
 //     a warp's 16-byte reads on different banks (an odd number of words per pixel where the run is no

@@ -270,8 +270,15 @@ GPS_HD vec3 conic_of(vec3 cov2d, float inv_det) {
 }
 
 // linalg.cuh:406-411: 28-bit linear view-depth key
+// The two steps back to an NDC depth are spelled out on the device in the rounding that the resolves
+// were compiled to (equal for all keys of ten pairs of planes): left to the compiler it depends on
+// the kernel, and the sweep for planes where they are monotone has to run what the resolves run.
 GPS_HD float view_depth_from_key(uint64_t depth, float near_plane, float far_plane) {
+#if defined(__CUDA_ARCH__)
+    return -__fmaf_rn((float)depth / (float)kDepthMax, far_plane - near_plane, near_plane);
+#else
     return -(((float)depth / (float)kDepthMax) * (far_plane - near_plane) + near_plane);
+#endif
 }
 GPS_HD uint64_t depth_key(float depth, float near_plane, float far_plane) {
     float t = gclamp((fabsf(depth) - near_plane) / (far_plane - near_plane), 0.0f, 1.0f);
@@ -279,16 +286,20 @@ GPS_HD uint64_t depth_key(float depth, float near_plane, float far_plane) {
 }
 // linalg.cuh:413-420
 GPS_HD float view_to_projected_depth(float z_view, float near_plane, float far_plane) {
+#if !defined(__CUDA_ARCH__)
     float a = (far_plane + near_plane) / (far_plane - near_plane);
+#endif
     float b = (2.0f * far_plane * near_plane) / (far_plane - near_plane);
+#if defined(__CUDA_ARCH__)
+    return __fmaf_rn(far_plane + near_plane, 1.0f / (far_plane - near_plane), b / z_view);
+#else
     return a + b / z_view;
+#endif
 }
 
 #if defined(__CUDACC__)
-// NDC depth of a key's high word, no more than 1e9 (the resolves' start value; so is a NaN).  A function
-// of its own, not inlined: which of its products are fused depends on the kernel it is inlined into,
-// and the sweep for planes where it is monotone has to run the very code that the resolves run.
-static __device__ __noinline__ float depth_of_key(uint32_t high_word, float near_plane, float far_plane) {
+// NDC depth of a key's high word, no more than 1e9 (the resolves' start value; so is a NaN).
+GPS_D float depth_of_key(uint32_t high_word, float near_plane, float far_plane) {
     const float view_depth = view_depth_from_key((uint64_t)(high_word >> 4), near_plane, far_plane);
     return gmin(1e9f, view_to_projected_depth(view_depth, near_plane, far_plane));
 }
