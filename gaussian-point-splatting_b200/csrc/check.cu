@@ -267,3 +267,73 @@ extern "C" int gps_check_draws(uint32_t gaussians, uint32_t draws, uint32_t salt
     download(out, d.p, 2 * sizeof(Tally));
     return (int)cudaGetLastError();
 }
+
+namespace {
+
+struct SplatCase {
+    const gps::SplatRecord* records;
+    const uint32_t *gid, *start;
+    uint32_t survivors, points;
+    int frame_seed, width, height, passes, k, unbiased;
+};
+
+// One thread per point, one sample after the other in the reference's form, no pre-test.
+__global__ void plain_splat_kernel(SplatCase a, unsigned long long* buffer) {
+    using namespace gps;
+    FrameConst fc{};
+    fc.num_passes = a.passes;
+    fc.up_width = a.width;
+    fc.up_height = a.height;
+    for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < a.points; p += gridDim.x * blockDim.x) {
+        uint32_t r = 0;  // the last survivor that starts at or before p
+        for (uint32_t n = a.survivors; n > 1u;) {
+            const uint32_t half = n / 2u;
+            if (a.start[r + half] <= p) {
+                r += half;
+                n -= half;
+            } else {
+                n = half;
+            }
+        }
+        const SplatRecord rec = a.records[a.gid[r]];
+        const SampleConst c = sample_const(rec, fc, nullptr);
+        const uint64_t key = (uint64_t)rec.d.z | ((uint64_t)rec.d.w << 32);
+        u32x2 seed = make_seed(p, (uint32_t)a.frame_seed);
+        for (int i = 0; i < a.passes * a.k; ++i) {
+            if (a.unbiased) {
+                uint32_t tile, code;
+                if (draw_sample(seed, c, tile, code)) atomicMin(buffer + sample_slot(c, tile, code, i / a.k), (unsigned long long)key);
+                continue;
+            }
+            const vec2 u = pcg2d(seed), xy = box_muller(u.x, u.y);
+            const float px = floorf(c.pixel_mean.x + c.c0 * xy.x), py = floorf(c.pixel_mean.y + c.c1 * xy.x + c.c2 * xy.y);
+            const int x = (int)px, y = (int)py;
+            if (x < c.minx || x >= c.maxx || y < c.miny || y >= c.maxy) continue;
+            if (c.opacity * gaussian_value(c.conic, make_v2(c.pixel_mean.x - px, c.pixel_mean.y - py)) < 1.0f / 255.0f) continue;
+            unsigned long long* at = buffer + splat_index(x, y, i / a.k, a.passes, a.width, a.height);
+            for (unsigned long long old = *at;;) {
+                if ((key & kDepthMask) > (old & kDepthMask)) break;
+                const unsigned long long now = (key & kDepthMask) < (old & kDepthMask)
+                                                   ? key : (old & kDepthMask) | (((old & kColorMask) + (key & kColorMask)) & kColorMask);
+                const unsigned long long was = atomicCAS(at, old, now);
+                if (was == old) break;
+                old = was;
+            }
+        }
+    }
+}
+
+}  // namespace
+
+// The splat of a pass from its records and survivors (device arrays) into a buffer of `entries` that starts at `initial`.
+extern "C" int gps_check_splat(const float* d_records, const uint32_t* d_gid, const uint32_t* d_start, uint32_t survivors,
+                               uint32_t points, int frame_seed, int width, int height, int passes, int k, int unbiased,
+                               uint64_t initial, uint64_t entries, uint64_t* out) {
+    DeviceArray<unsigned long long> buffer(entries);
+    if (!buffer.p) return 1;
+    gps::launch_clear(reinterpret_cast<uint64_t*>(buffer.p), entries, initial, 0);
+    const SplatCase a{reinterpret_cast<const gps::SplatRecord*>(d_records), d_gid, d_start, survivors, points, frame_seed, width, height, passes, k, unbiased};
+    plain_splat_kernel<<<148 * 4, 128>>>(a, buffer.p);
+    download(out, buffer.p, entries * 8);
+    return (int)cudaGetLastError();
+}
