@@ -1802,9 +1802,9 @@ __global__ void __launch_bounds__(256, 8) resolve_morton_kernel(ResolveArgs a, H
 }
 
 // Staged variant: a block's pixels are consecutive in Morton-tile order, so their samples are
-// one contiguous run of the buffer (px_per_block x SS*SS*spp entries, at most 48 KB), which the
+// one contiguous run of the buffer (px_per_block x SS*SS*spp entries, at most 32 KB), which the
 // block reads with coalesced 16-byte loads.  Used for SS 1, 2, 4, 8 with 1 to 8 or a power of two of
-// samples per pixel and 2 to 128 samples in all.
+// samples per pixel and, in all, a power of two from 2 to 128 or any number below 64.
 //   depth only: of every entry pair the smaller high word goes to shared memory; a pixel's depth
 //     is that of its smallest key.  That is the smallest depth bit for bit where the conversion to NDC
 //     does not fall anywhere as the key grows.  It ends in an approximate division, of which only an
@@ -2492,7 +2492,7 @@ namespace {
 // that kernel has left the GPU instead of after its completion has been reported back.  No kernel
 // signals earlier (griddepcontrol.launch_dependents): blocks of the next kernel that wait beside
 // a persistent grid's tail land unevenly on the SMs, and frames got slower (16M town: 2.79
-// against 2.38 ms).  A frame is 6 to 18 launches, most of them a few microseconds long on small
+// against 2.38 ms).  A frame is 4 to 18 launches, most of them a few microseconds long on small
 // views.  Measured with the frame's counters handed over by the final resolve, against plain
 // launches and a copy: 20k cube at 160x90 45.5 -> 22.0 us a frame, 60k town at 320x180 130 -> 89,
 // 1M cube at 640x360 177 -> 154, 4M town at 1080p 1121 -> 1076.
@@ -2697,7 +2697,9 @@ int launch_splat(const SplatArgs& args, int grid, int block, cudaStream_t stream
     // a persistent grid: as many blocks as fit on the device at once
     const int k = a.fc.use_unbiased ? a.fc.k_points : 0;
     // Views of up to 2M samples: at the one or two points per 16 of them that scenes have, fewer points
-    // than half the threads (320x180, ss 2, 4 spp: 0.9M samples, 28k points, 152k threads).
+    // than half the threads (320x180, ss 2, 4 spp: 0.9M samples, 28k points, 152k threads).  60k town, split /
+    // not: 320x180 at 8 spp (1.8M) 63.9 / 72.1 us a frame, 640x360 at 1 spp (0.9M, four samples a point) 54.4 /
+    // 53.1; 1280x720 at 2 spp (7.4M) 82.0 / 80.3, 960x540 at 4 spp (8.3M) 84.5 / 85.1.
     const bool small = (uint64_t)a.fc.up_width * (uint64_t)a.fc.up_height * (uint64_t)a.fc.num_passes <= (2u << 20) &&
                        a.fc.num_passes * k >= 4;
     if (k == 4) small ? launch_splat_plain<4, true>(a, stream) : launch_splat_plain<4, false>(a, stream);

@@ -81,7 +81,9 @@ struct ClearArgs {
 };
 
 // Scenes of up to this many Gaussians (in blocks of four) have their block cull inside the preprocess:
-// a launch less, where a warp has at most two chunks to test and to work on.
+// a launch less, where a warp has at most two chunks to test and to work on.  Town at 320x180 and 1280x720 in
+// us a frame, with one, two and four chunks a warp: 152k Gaussians 59.6, 57.2, 60.3 and 82.5, 78.6, 82.0;
+// 300k 61.2, 59.7, 61.7 and 92.9, 89.8, 92.8; 305k (a launch, but for four) 60.9, 60.9, 62.1 and 94.0, 93.9, 94.1.
 constexpr uint32_t kSelfCullChunks = 2;
 constexpr uint32_t kSelfCullGaussians = 32u * 4736u * kSelfCullChunks;  // 4736 warps: 4 blocks on 148 SMs
 
