@@ -1109,13 +1109,12 @@ __device__ __forceinline__ void atomic_add_color(unsigned long long* address, un
 }
 
 // Biased mode (use_unbiased_2d_splatting = false): one point's samples first..last - 1 (the seed
-// advances, as splatGaussianPoint's does), kBiasedBatch at a time: their slots, then their
-// pre-test loads together, then the additions, which start from the loaded values.  A load that
-// missed an addition made since costs a second compare-and-swap, no more: a slot's depth only
-// decreases.  (Before, one sample waited for the last one's two loads: 300k town,
-// 999x571, 4 spp: frame 110.3 -> 109.5 us)
-constexpr int kBiasedBatch = 4;
-
+// advances, as splatGaussianPoint's does), in order: a slot's pre-test load, then the addition, which
+// starts from the loaded value.  A load that missed an addition made since costs a second
+// compare-and-swap, no more: a slot's depth only decreases.  What bounds it is those chains and the
+// instructions around them, not the loads' latency, which the other warps cover: four samples at a time,
+// with their loads together, took 340 us for 225 (700k town, 1280x720, 4 spp; with a load of its own for the
+// addition 253), and no setting was faster that way.
 __device__ __forceinline__ void splat_samples_biased(u32x2& seed, const SplatRecord& rec, const FrameConst& fc,
                                                      uint64_t* __restrict__ buffer, int first, int last) {
     const vec2 pixel_mean = make_v2(rec.a.x, rec.a.y);
@@ -1128,39 +1127,28 @@ __device__ __forceinline__ void splat_samples_biased(u32x2& seed, const SplatRec
     const uint64_t view_depth_bits = key & kDepthMask;
     const int k = fc.k_points;
     unsigned long long* buf = reinterpret_cast<unsigned long long*>(buffer);
-    int pass = first / k, j = first - pass * k;  // sample s0 + b is draw j of spp pass `pass`
-    for (int s0 = first; s0 < last; s0 += kBiasedBatch) {
-        int slot[kBiasedBatch];
-        bool live[kBiasedBatch];
-#pragma unroll
-        for (int b = 0; b < kBiasedBatch; ++b) {
-            live[b] = false;
-            slot[b] = 0;
-            if (s0 + b >= last) continue;
-            vec2 u = pcg2d(seed);
-            vec2 xy = box_muller(u.x, u.y);
-            vec2 pixel = make_v2(pixel_mean.x + c0 * xy.x, pixel_mean.y + c1 * xy.x + c2 * xy.y);
-            pixel = make_v2(floorf(pixel.x), floorf(pixel.y));
-            int x = (int)pixel.x;
-            int y = (int)pixel.y;
-            vec2 delta = make_v2(pixel_mean.x - pixel.x, pixel_mean.y - pixel.y);
-            if (x >= minx && x < maxx && y >= miny && y < maxy) {
-                float gw = gaussian_value(conic, delta);
-                float alpha = opacity * gw;
-                live[b] = !(alpha < 1.0f / 255.0f);
-                slot[b] = splat_index(x, y, pass, fc.num_passes, fc.up_width, fc.up_height);
-            }
-            if (++j == k) {
-                j = 0;
-                ++pass;
+    int pass = first / k, j = first - pass * k;  // sample s is draw j of spp pass `pass`
+    for (int s = first; s < last; ++s) {
+        vec2 u = pcg2d(seed);
+        vec2 xy = box_muller(u.x, u.y);
+        vec2 pixel = make_v2(pixel_mean.x + c0 * xy.x, pixel_mean.y + c1 * xy.x + c2 * xy.y);
+        pixel = make_v2(floorf(pixel.x), floorf(pixel.y));
+        int x = (int)pixel.x;
+        int y = (int)pixel.y;
+        vec2 delta = make_v2(pixel_mean.x - pixel.x, pixel_mean.y - pixel.y);
+        if (x >= minx && x < maxx && y >= miny && y < maxy) {
+            float gw = gaussian_value(conic, delta);
+            float alpha = opacity * gw;
+            if (!(alpha < 1.0f / 255.0f)) {
+                unsigned long long* slot = buf + splat_index(x, y, pass, fc.num_passes, fc.up_width, fc.up_height);
+                const unsigned long long seen = __ldcg(slot);
+                if ((uint64_t)seen > view_depth_bits) atomic_add_color(slot, seen, key);
             }
         }
-        unsigned long long seen[kBiasedBatch];
-#pragma unroll
-        for (int b = 0; b < kBiasedBatch; ++b) seen[b] = live[b] ? __ldcg(buf + slot[b]) : 0ull;
-#pragma unroll
-        for (int b = 0; b < kBiasedBatch; ++b)
-            if (live[b] && (uint64_t)seen[b] > view_depth_bits) atomic_add_color(buf + slot[b], seen[b], key);
+        if (++j == k) {
+            j = 0;
+            ++pass;
+        }
     }
 }
 
