@@ -428,8 +428,12 @@ __device__ __forceinline__ bool preprocess_one(const PreprocessArgs& a, const Sc
 // has up to two chunks, half the scene apart so that a visible region's neighbours go to different
 // warps, and its lanes test those chunks' nodes first.  Frames of the 60k town
 // at 320x180 62.7 -> 56.3 us, 300k at 999x571 109.5 -> 106.0, with the clear here too a 20k cube 18.5 -> 17.7.
+//
+// kImmediate: the compiler takes 80 registers for the splat in it, three blocks per SM; held to 64 (and a few
+// spills outside the sample loop), four: 150k town, compressed, 411x191, all Gaussians of up to 20 points
+// splatted here, 8 spp: 917 -> 544 us (FP32 918 -> 544).
 template <class Scene, bool kImmediate, bool kCull>
-__global__ void __launch_bounds__(256) preprocess_kernel(PreprocessArgs a, Scene scene) {
+__global__ void __launch_bounds__(256, kImmediate ? 4 : 0) preprocess_kernel(PreprocessArgs a, Scene scene) {
     previous_kernel_done();
     if (blockIdx.x >= a.blocks_here) {
         clear_beside(a.clear, blockIdx.x - a.blocks_here, gridDim.x - a.blocks_here);
